@@ -84,7 +84,7 @@ void free_contact_buffers(rg_system* s) {
   cudaFree(N.xrow);
   cudaFree(N.dx); cudaFree(N.prow); cudaFree(N.pactive);
   cudaFree(N.pmax); cudaFree(N.cmask); cudaFree(N.owner); cudaFree(N.cursor); cudaFree(N.remaining);
-  cudaFree(N.blk); cudaFree(N.slot_of); cudaFree(N.bar); cudaFree(N.view_dev); cudaFree(N.team_dev);
+  cudaFree(N.blk); cudaFree(N.bar); cudaFree(N.view_dev); cudaFree(N.team_dev);
   N = Nsc();
   cudaFree(s->d_cf);
   s->d_cf = nullptr;
@@ -140,10 +140,8 @@ cudaError_t alloc_contact_buffers(rg_system* s, int ccap, int hcap) {
   if ((e = cudaMalloc(&N.cursor, sizeof(int) * (kMaxColors + 2)))) return e;
   if ((e = cudaMalloc(&N.remaining, sizeof(int) * 1024))) return e;
   if ((e = cudaMalloc(&N.blk, sizeof(int) * (s->coop_blocks + 32)))) return e;
-  if ((e = cudaMalloc(&N.slot_of, sizeof(int) * (size_t)n))) return e;
-  if ((e = cudaMemset(N.slot_of, 0xff, sizeof(int) * (size_t)n))) return e;
-  if ((e = cudaMalloc(&N.bar, sizeof(unsigned int) * 8))) return e;
-  if ((e = cudaMemset(N.bar, 0, sizeof(unsigned int) * 8))) return e;
+  if ((e = cudaMalloc(&N.bar, kTeamBarBytes))) return e;
+  if ((e = cudaMemset(N.bar, 0, kTeamBarBytes))) return e;
   if ((e = cudaMalloc(&N.view_dev, nsc_view_bytes()))) return e;
   if ((e = cudaMalloc(&N.team_dev, nsc_team_bytes()))) return e;
   if ((e = cudaMalloc(&s->d_cf, sizeof(double) * (13 * (size_t)ccap + 64)))) return e;

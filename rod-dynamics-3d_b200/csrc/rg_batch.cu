@@ -365,7 +365,7 @@ cudaError_t ensure_dev(rg_batch* b, size_t nteams, size_t nmembers) {
     cudaFree(b->d_bars);
     b->cap_teams = (int)std::max<size_t>(nteams, (size_t)b->coop_blocks);
     if ((e = cudaMalloc(&b->d_teams, sizeof(TeamDesc) * b->cap_teams))) return e;
-    if ((e = cudaMalloc(&b->d_bars, sizeof(unsigned int) * 4 * b->cap_teams))) return e;
+    if ((e = cudaMalloc(&b->d_bars, kTeamBarBytes * b->cap_teams))) return e;
     cudaFree(b->d_team_ns);
     if ((e = cudaMalloc(&b->d_team_ns, sizeof(long long) * b->cap_teams))) return e;
   }
@@ -385,7 +385,7 @@ cudaError_t upload(rg_batch* b, std::vector<TeamDesc>& teams, const std::vector<
     if (b->sys[k]->cfg.model == RG_MODEL_NSC) views[k] = make_view(b->sys[k]);
   }
   for (size_t t = 0; t < teams.size(); ++t) {
-    teams[t].bar = b->d_bars + 4 * t;
+    teams[t].bar = b->d_bars + kTeamBarBytes / sizeof(unsigned int) * t;
     teams[t].t_ns = b->d_team_ns + t;
   }
   bool any = false;
@@ -417,7 +417,7 @@ void drop_graph(rg_batch* b) {
 cudaError_t launch_nsc(rg_batch* b, int nteams, int grid, int nsteps, bool graph_ok) {
   if (grid <= 0 || nsteps <= 0) return cudaSuccess;
   if (!(graph_ok && b->use_graph)) {
-    cudaMemsetAsync(b->d_bars, 0, sizeof(unsigned int) * 4 * nteams, b->stream);
+    cudaMemsetAsync(b->d_bars, 0, kTeamBarBytes * nteams, b->stream);
     nsc_batch_launch(b->d_views, b->d_teams, nteams, b->d_members, grid, nsteps, b->stream);
     return cudaGetLastError();
   }
@@ -426,7 +426,7 @@ cudaError_t launch_nsc(rg_batch* b, int nteams, int grid, int nsteps, bool graph
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (e) return e;
-    cudaMemsetAsync(b->d_bars, 0, sizeof(unsigned int) * 4 * nteams, b->stream);
+    cudaMemsetAsync(b->d_bars, 0, kTeamBarBytes * nteams, b->stream);
     nsc_batch_launch(b->d_views, b->d_teams, nteams, b->d_members, grid, nsteps, b->stream);
     e = cudaStreamEndCapture(b->stream, &g);
     if (e) return e;

@@ -165,11 +165,13 @@ struct Nsc {
   int* cursor = nullptr;                // kMaxColors+1
   int* remaining = nullptr;             // colouring rounds
   int* blk = nullptr;                   // per-block scan scratch
-  int* slot_of = nullptr;               // n per-body local slots (-1)
   unsigned int* bar = nullptr;          // team barrier words
   void* view_dev = nullptr;             // device copy of the step view
   void* team_dev = nullptr;             // device team descriptor
 };
+// bytes behind a team's barrier words (zeroed before every launch): 4 words
+// and the residual ring of the split solve (rg_nsc.cu)
+constexpr size_t kTeamBarBytes = 1024;
 constexpr int kRowComps = 42;
 constexpr int kExportComps = 11;
 constexpr int kPosComps = 12;

@@ -40,15 +40,20 @@ MlpDev mlp_dev(rg_system* s);
 // ---------------------------------------------------------------------------
 // Teams and team barriers.
 // ---------------------------------------------------------------------------
+constexpr int kChunk = 32;  // most sweeps of a chunk of the split solve
+static_assert(kTeamBarBytes >= 16 + sizeof(double) * 3 * kChunk, "barrier words and residual ring of a team");
 struct Team {
   int b0, nb;
-  unsigned int* bar;
+  unsigned int* bar;      // 4 barrier words, then the residual ring
   int* err;
   long long spin_limit;   // polls per barrier wait before ERR_TIMEOUT
   unsigned int absent;    // test hook: blocks the barriers wait for in vain
   __device__ int rank() const { return (int)blockIdx.x - b0; }
   __device__ int tid() const { return rank() * (int)blockDim.x + (int)threadIdx.x; }
   __device__ int size() const { return nb * (int)blockDim.x; }
+  // residuals of the split solve's chunks: three buffers of kChunk, zero at
+  // the start of a launch
+  __device__ double* ring() const { return reinterpret_cast<double*>(bar + 4); }
 };
 
 __device__ inline bool team_sync(const Team& T) {
@@ -103,6 +108,10 @@ struct PhaseClock {
 // Dynamic shared memory of the persistent step: the small-solve arrays, or
 // the list-build tiles while a rebuild runs (phases never overlap).
 extern __shared__ __align__(16) unsigned char nsc_dyn_smem[];
+struct SmallSmem;
+// The small-solve arrays, by their symbol: a function that takes them as a
+// reference would reach them through generic loads and stores.
+__device__ __forceinline__ SmallSmem& small_smem() { return *reinterpret_cast<SmallSmem*>(nsc_dyn_smem); }
 // list-build candidate queues, after the tiles
 constexpr int kBuildQ = 4096;
 constexpr size_t kBuildQOff = (sizeof(BuildSmem) + 15) & ~(size_t)15;
@@ -783,58 +792,90 @@ __device__ __noinline__ bool project_phase(const Team& T, const NscView& V, int 
 
 
 // ---------------------------------------------------------------------------
-// Small contact sets (C <= kSmallC): one block solves everything in shared
-// memory.  Contact c is owned by thread c; its bodies get compact local slots
-// (a per-body slot map in global memory, reset afterwards), so colouring
-// scratch, body velocities, manifold rows and impulses all live on chip and
-// phases synchronise with __syncthreads.  Same arithmetic, same order as the
-// team path and the oracle.
+// Contact sets of up to kSmallC contacts: solved on chip, island by island.
+//
+// Every block of the team colours the whole contact graph in its own shared
+// memory (no barrier, the same colours everywhere) and finds its connected
+// components.  Components share no dynamic body, so Gauss-Seidel on one never
+// reads what another writes: block r takes the r-th share of them and keeps
+// their body velocities in shared memory.  The sweeps stop when the largest
+// change of any contact falls below the tolerance, so the blocks run a chunk
+// of sweeps, keep the state after each, publish the chunk's residuals, and
+// after one team barrier all put back the state of the sweep at which the
+// whole set stopped: the same sweeps as one sequential solver makes, bit for
+// bit.  A component that a sweep left unchanged stays unchanged and is not
+// swept again.
+//
+// A contact is owned by two adjacent lanes, one per body: a lane holds its
+// side of the manifold row, updates its body, and gets the three numbers it
+// needs of the other side by shuffle.  That halves the chain of dependent
+// FP64 operations, and the row of one contact per lane pair stays in
+// registers; up to 16 contacts need a single warp and no block barrier.
+//
+// Sets of at most kPairs contacts stay on the team's first block (solo): a
+// chunk's barrier and its surplus sweeps cost more there than the split saves.
+//
+// Bound: latency of a row update (about 1,200 cycles: some 50 dependent FP64
+// operations, two square roots, three exchanges) times colours times sweeps.
+// Measured per sweep: N = 20,000, 200 contacts 10 -> 2.9 us (one block; rows
+// in shared memory and one lane per contact before), N = 50,000, 450 contacts
+// 23 -> 2.4 us (rows and velocities in global memory before); whole steps
+// 274 -> 180 us and 2,020 -> 385 us.  Above kSmallC contacts the shared
+// memory for velocities ends and the team path takes over.
 // ---------------------------------------------------------------------------
-#ifndef RG_SMALL_C
-#define RG_SMALL_C kTile
+#ifndef RG_NSC_BLOCK
+#define RG_NSC_BLOCK (2 * kTile)
 #endif
-constexpr int kSmallC = RG_SMALL_C;      // one contact per thread
-constexpr int kSmallB = 2 * kSmallC;     // local body slots
+constexpr int kBlock = RG_NSC_BLOCK;     // threads per block of the persistent step
+constexpr int kPairs = kBlock / 2;       // lane pairs of a block
+constexpr int kSmallC = 4 * kPairs;      // contacts of the on-chip solve
+constexpr int kSmallB = 2 * kSmallC;     // body slots
+constexpr int kHash = 2 * kSmallB;       // body -> slot table (power of two)
+constexpr int kSplit = 512;              // most blocks the components are split over
+constexpr int kVel = 6 * kSmallB;        // doubles of the velocity space
+static_assert((kHash & (kHash - 1)) == 0 && kSmallB <= 65536, "hash table and 16-bit slots");
 
 struct SmallSmem {
-  double row[kRowComps * kSmallC];   // manifold rows (or projection rows)
-  double lam[3 * kSmallC];
-  double vel[6 * kSmallB];           // v, w (or dx, dθ) per local slot
-  unsigned long long pmax[2 * kSmallB];
-  unsigned long long cmask[kSmallB];
-  int body[kSmallB];                 // body of a slot (-1: unused)
-  int dyn[kSmallB];                  // 1: dynamic body
-  int la[kSmallC], lb[kSmallC];      // local slots of contact c
-  int color[kSmallC], order[kSmallC];
-  int cnt[kMaxColors + 1], coff[kMaxColors + 1], cur[kMaxColors + 1];
-  int nloc, rem, ncol, act;
-  double red[32];
-  float feat[kMlpIn * kSmallC];      // learned warm start features [8][kSmallC]
-  float pred[kMlpOut * kSmallC];     // predicted impulse changes [3][kSmallC]
-  int mtile[kSmallC / 16];           // 16-contact tiles that need the network
+  // v, w (or dx, dθ) per local body slot, 6 doubles each, then the states
+  // after the sweeps of a chunk.  Before the velocities are loaded the space
+  // serves the colouring and the split (SmallScratch), then the warm-cache
+  // keys, then the network's third layer.
+  alignas(16) double vel[kVel];
+  // the network's W1, W4 and small parameters; before that the degrees
+  alignas(16) unsigned char stage[(kStageSmallBytes + 15) / 16 * 16];
+  alignas(16) __nv_bfloat16 wh[kStageWh];  // the network's second layer
+  double locs[kChunk * 32];          // residuals of a chunk's sweeps, per lane or warp
+  double res[kChunk];                // residuals of the chunk over the team
+  int body[kSmallB];                 // body of a local slot
+  unsigned char dyn[kSmallB];        // 1: dynamic body
+  // this block's contacts in colour-major slots: contact, colour, body slots
+  unsigned short order[kSmallC], pa[kSmallC], pb[kSmallC];
+  unsigned char pcol[kSmallC];
   unsigned char cached[kSmallC];     // 1: the slot's contact is in the warm cache
-  // one hidden layer of the network (the rest is staged in pmax/cmask)
-#ifndef RG_NO_MLP_STAGE
-  alignas(16) __nv_bfloat16 wh[kStageWh];
-#else
-  alignas(16) __nv_bfloat16 wh[8];  // build without in-step inference staging
-#endif
+  int cnt[kMaxColors + 1], coff[kMaxColors + 1], cur[kMaxColors + 1];
+  int nloc, ncol, nbody;
+  int scan_w[32];
+  int mtile[kSmallC / 16];           // 16-contact tiles that need the network
 };
-#ifndef RG_NO_MLP_STAGE
-static_assert(sizeof(unsigned long long) * 3 * kSmallB >= kStageSmallBytes, "MLP staging space");
-#endif
+struct SmallScratch {  // whole contact set: slots of all bodies, colours
+  union {
+    unsigned long long pmax[2 * kSmallB];
+    struct {  // after the colouring
+      int lab[kSmallC], blab[kSmallB], irank[kSmallC], hist[kSplit], bl[kSmallB];
+    };
+  };
+  unsigned long long cmask[kSmallB];
+  int hkey[kHash];
+  unsigned short hslot[kHash];
+  int body[kSmallB];
+  unsigned char dyn[kSmallB];
+  unsigned short la[kSmallC], lb[kSmallC], color[kSmallC];  // by contact
+};
+static_assert(sizeof(SmallScratch) <= sizeof(double) * kVel, "colouring scratch");
+static_assert(sizeof(SmallSmem::stage) >= sizeof(int) * kSmallB, "degrees");
+static_assert(sizeof(__nv_bfloat16) * kStageWh <= sizeof(double) * kVel, "third network layer");
 static_assert(sizeof(SmallSmem) >= kBuildQOff + 2 * sizeof(unsigned) * kBuildQ,
               "list-build tiles and queues share the small-solve memory");
-
-__device__ inline double small_block_max(double v, SmallSmem& S) {
-  v = warp_max(v);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) S.red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  // every warp combines the per-warp maxima itself (one load per lane)
-  const int lane = threadIdx.x & 31;
-  return warp_max(lane < (int)(blockDim.x >> 5) ? S.red[lane] : 0.0);  // every thread
-}
 
 // True when contact c has an entry in the warm cache of the previous step
 // (W entries): the learned start by default serves only the others.
@@ -845,66 +886,87 @@ __device__ inline bool warm_cached(const NscView& V, int c, int W) {
   return q < W && V.wkey[q] == k;
 }
 
-// Local slots for the bodies of contacts 0..C-1 (C <= blockDim).
-__device__ __noinline__ void small_map(const NscView& V, int C, SmallSmem& S) {
+// Slots for the bodies of contacts 0..C-1 (C <= kSmallC), through a hash
+// table of body numbers in shared memory.
+__device__ __noinline__ void small_map(const NscView& V, int C) {
+  SmallSmem& S = small_smem();
   const int t = threadIdx.x;
+  SmallScratch& X = *reinterpret_cast<SmallScratch*>(S.vel);
+  const int size = C <= 64 ? 256 : (C <= kPairs ? 4 * kPairs : kHash);  // at least 4 C, a power of two
   if (t == 0) S.nloc = 0;
+  for (int k = t; k < size; k += blockDim.x) X.hkey[k] = -1;
   __syncthreads();
-  if (t < C) {
-    int x[2] = {V.con.a[t], V.con.b[t]};
-    int sl[2];
-    for (int k = 0; k < 2; ++k) {
-      int idx = atomicAdd(&S.nloc, 1);
-      int old = atomicCAS(&V.slot_of[x[k]], -1, idx);
-      S.body[idx] = old == -1 ? x[k] : -1;
-      sl[k] = old == -1 ? idx : old;
+  for (int e = t; e < 2 * C; e += blockDim.x) {
+    const int c = e >> 1;
+    const int x = (e & 1) ? V.con.b[c] : V.con.a[c];
+    unsigned pos = ((unsigned)x * 0x9E3779B1u) >> 7;
+    for (;;) {  // at most 2 C of the entries are ever taken
+      pos &= size - 1;
+      const int old = atomicCAS(&X.hkey[pos], -1, x);
+      if (old == -1) {
+        const int idx = atomicAdd(&S.nloc, 1);
+        X.hslot[pos] = (unsigned short)idx;
+        X.body[idx] = x;
+        X.dyn[idx] = V.st.inv_mass[x] > 0.0 ? 1 : 0;
+      }
+      if (old == -1 || old == x) break;
+      ++pos;
     }
-    S.la[t] = sl[0];
-    S.lb[t] = sl[1];
+    if (e & 1) X.lb[c] = (unsigned short)pos;
+    else X.la[c] = (unsigned short)pos;
   }
   __syncthreads();
-  for (int s = t; s < S.nloc; s += blockDim.x) {
-    int x = S.body[s];
-    S.dyn[s] = (x >= 0 && V.st.inv_mass[x] > 0.0) ? 1 : 0;
+  for (int c = t; c < C; c += blockDim.x) {
+    X.la[c] = X.hslot[X.la[c]];
+    X.lb[c] = X.hslot[X.lb[c]];
   }
   __syncthreads();
-}
-__device__ void small_unmap(const NscView& V, SmallSmem& S) {
-  for (int s = threadIdx.x; s < S.nloc; s += blockDim.x)
-    if (S.body[s] >= 0) V.slot_of[S.body[s]] = -1;
 }
 
-// Jones-Plassmann first fit on local slots; fills S.color / S.order /
-// S.coff and the global colour arrays.  Returns the colour count or -1.
-__device__ __noinline__ int small_color(const NscView& V, int C, SmallSmem& S) {
+// Jones-Plassmann first fit on the slots: X.color per contact.  Returns the
+// colour count or -1.
+__device__ __noinline__ int small_color(const NscView& V, int C, bool lead) {
+  SmallSmem& S = small_smem();
   const int t = threadIdx.x;
-  for (int s = t; s < S.nloc; s += blockDim.x) {
-    S.pmax[s] = 0; S.pmax[kSmallB + s] = 0; S.cmask[s] = 0;
+  SmallScratch& X = *reinterpret_cast<SmallScratch*>(S.vel);
+  constexpr unsigned short kNone = 0xffff;
+  if (S.nloc == 2 * C) {  // no body twice: one colour
+    for (int c = t; c < C; c += blockDim.x) X.color[c] = 0;
+    if (t == 0) S.ncol = C > 0;
+    if (t == 0 && lead) V.ctl->colors = C > 0;
+    __syncthreads();
+    return C > 0;
   }
-  for (int k = t; k <= kMaxColors; k += blockDim.x) { S.cnt[k] = 0; S.cur[k] = 0; }
-  if (t < C) S.color[t] = -1;
+  for (int s = t; s < S.nloc; s += blockDim.x) {
+    X.pmax[s] = 0; X.pmax[kSmallB + s] = 0; X.cmask[s] = 0;
+  }
+  for (int c = t; c < C; c += blockDim.x) X.color[c] = kNone;
   if (t == 0) S.ncol = 0;
   __syncthreads();
   int round = 0;
   for (; round < kMaxRounds; ++round) {
-    unsigned long long* pm = S.pmax + (round & 1) * kSmallB;
-    unsigned long long* pn = S.pmax + ((round + 1) & 1) * kSmallB;
-    if (t == 0) S.rem = 0;
-    if (t < C && S.color[t] < 0) {
-      unsigned long long p = jp_priority((unsigned)t);
-      if (S.dyn[S.la[t]]) atomicMax(&pm[S.la[t]], p);
-      if (S.dyn[S.lb[t]]) atomicMax(&pm[S.lb[t]], p);
+    unsigned long long* pm = X.pmax + (round & 1) * kSmallB;
+    unsigned long long* pn = X.pmax + ((round + 1) & 1) * kSmallB;
+    for (int c = t; c < C; c += blockDim.x) {
+      if (X.color[c] != kNone) continue;
+      const unsigned long long p = jp_priority((unsigned)c);
+      if (X.dyn[X.la[c]]) atomicMax(&pm[X.la[c]], p);
+      if (X.dyn[X.lb[c]]) atomicMax(&pm[X.lb[c]], p);
     }
     __syncthreads();
-    if (t < C && S.color[t] < 0) {
-      unsigned long long p = jp_priority((unsigned)t);
-      int sl[2] = {S.la[t], S.lb[t]};
+    int rem = 0;
+    for (int c = t; c < C; c += blockDim.x) {
+      if (X.color[c] != kNone) continue;
+      const unsigned long long p = jp_priority((unsigned)c);
+      const int sl[2] = {X.la[c], X.lb[c]};
       bool win = true;
       unsigned long long used = 0;
       for (int k = 0; k < 2; ++k) {
-        if (!S.dyn[sl[k]]) continue;
+        if (!X.dyn[sl[k]]) continue;
         if (pm[sl[k]] != p) win = false;
-        used |= S.cmask[sl[k]];
+        // two winners of a round never share a dynamic body, so a mask that
+        // changes in this round is only read by losers
+        used |= *(volatile unsigned long long*)&X.cmask[sl[k]];
         pn[sl[k]] = 0;
       }
       if (win) {
@@ -913,199 +975,770 @@ __device__ __noinline__ int small_color(const NscView& V, int C, SmallSmem& S) {
           atomicOr(&V.ctl->err, ERR_COLOR);
           col = kMaxColors - 1;
         }
-        S.color[t] = col;
+        X.color[c] = (unsigned short)col;
         for (int k = 0; k < 2; ++k)
-          if (S.dyn[sl[k]]) atomicOr(&S.cmask[sl[k]], 1ull << col);
-        atomicAdd(&S.cnt[col], 1);
+          if (X.dyn[sl[k]]) atomicOr(&X.cmask[sl[k]], 1ull << col);
         atomicMax(&S.ncol, col + 1);
       } else {
-        atomicAdd(&S.rem, 1);
+        rem = 1;
       }
     }
-    __syncthreads();
-    int rem = S.rem;
-    __syncthreads();
-    if (rem == 0) break;
+    if (!__syncthreads_or(rem)) break;
   }
   if (round >= kMaxRounds) {
     if (t == 0) atomicOr(&V.ctl->err, ERR_COLOR);
     return -1;
   }
-  if (t == 0) {
-    int acc = 0;
-    for (int k = 0; k <= kMaxColors; ++k) {
-      S.coff[k] = acc;
-      if (k < kMaxColors) acc += S.cnt[k];
-    }
-    V.ctl->colors = S.ncol;
-  }
-  __syncthreads();
-  if (t < C) {
-    int k = S.color[t];
-    int p = S.coff[k] + atomicAdd(&S.cur[k], 1);
-    S.order[p] = t;
-    V.order[p] = t;
-    V.color[t] = k;
-  }
-  for (int k = t; k <= kMaxColors; k += blockDim.x) V.color_off[k] = S.coff[k];
-  __syncthreads();
-  return S.ncol;
+  const int ncol = S.ncol;
+  if (t == 0 && lead) V.ctl->colors = ncol;
+  __syncthreads();  // every thread has its copy before ncol is used again
+  return ncol;
 }
 
+// This block's share of a contact set: its contacts in colour-major slots
+// 0..count-1 of the on-chip arrays, and slots [base, base + count) of the
+// global row, impulse and feature arrays; most: the largest share.
+struct Share {
+  int count, base, most, colors;
+};
+// A team's blocks get the connected components in the order of their lowest
+// contacts.
+__device__ __noinline__ Share small_split(const Team& T, int C, int ncol) {
+  SmallSmem& S = small_smem();
+  const int t = threadIdx.x, rank = T.rank();
+  SmallScratch& X = *reinterpret_cast<SmallScratch*>(S.vel);
+  const bool split = T.nb > 1;
+  const int nbu = T.nb < kSplit ? T.nb : kSplit;
+  if (!split && ncol <= 1) {  // one block, one colour: the contacts as they are
+    for (int s = t; s < S.nloc; s += blockDim.x) {
+      S.body[s] = X.body[s];
+      S.dyn[s] = X.dyn[s];
+    }
+    for (int c = t; c < C; c += blockDim.x) {
+      S.order[c] = (unsigned short)c;
+      S.pcol[c] = 0;
+      S.pa[c] = X.la[c];
+      S.pb[c] = X.lb[c];
+    }
+    if (t == 0) {
+      S.nbody = S.nloc;
+      S.coff[0] = 0;
+      S.cnt[0] = C;
+    }
+    __syncthreads();
+    return Share{C, 0, C, ncol};
+  }
+  for (int k = t; k <= kMaxColors; k += blockDim.x) { S.cnt[k] = 0; S.cur[k] = 0; }
+  if (t == 0) { S.nbody = 0; S.ncol = 0; }
+  __syncthreads();  // (also: the colouring's maxima are done with)
+  if (split) {
+    for (int c = t; c < C; c += blockDim.x) X.lab[c] = c;
+    for (int s = t; s < S.nloc; s += blockDim.x) X.blab[s] = 0x7fffffff;
+    for (int r = t; r < kSplit; r += blockDim.x) X.hist[r] = 0;
+    // labels fall to the lowest contact of the component
+    int changed = 1;
+    while (__syncthreads_or(changed)) {
+      for (int c = t; c < C; c += blockDim.x) {
+        const int l = X.lab[c];
+        if (X.dyn[X.la[c]]) atomicMin(&X.blab[X.la[c]], l);
+        if (X.dyn[X.lb[c]]) atomicMin(&X.blab[X.lb[c]], l);
+      }
+      __syncthreads();
+      changed = 0;
+      for (int c = t; c < C; c += blockDim.x) {
+        const int l = X.lab[c];
+        int m = l;
+        if (X.dyn[X.la[c]]) m = min(m, X.blab[X.la[c]]);
+        if (X.dyn[X.lb[c]]) m = min(m, X.blab[X.lb[c]]);
+        m = min(m, *(volatile int*)&X.lab[m]);
+        if (m < l) {
+          *(volatile int*)&X.lab[c] = m;
+          changed = 1;
+        }
+      }
+    }
+    // component numbers
+    int total = 0;
+    for (int base = 0; base < C; base += blockDim.x) {
+      const int c = base + t;
+      const int root = c < C && X.lab[c] == c;
+      int tot;
+      const int ex = block_excl_scan(root, S.scan_w, tot);
+      if (root) X.irank[c] = total + ex;
+      total += tot;
+    }
+    __syncthreads();
+    for (int c = t; c < C; c += blockDim.x) {
+      const int blk = X.irank[X.lab[c]] * nbu / total;
+      X.blab[c] = blk;  // (the labels of the bodies are done with; C <= kSmallB)
+      atomicAdd(&X.hist[blk], 1);
+    }
+  }
+  for (int s = t; s < S.nloc; s += blockDim.x) X.bl[s] = -1;
+  __syncthreads();
+  // colours and bodies of the own contacts
+  int maxc = 0;
+  for (int c = t; c < C; c += blockDim.x) {
+    if (split && X.blab[c] != rank) continue;
+    atomicAdd(&S.cnt[X.color[c]], 1);
+    maxc = max(maxc, X.color[c] + 1);
+    for (int k = 0; k < 2; ++k) {
+      const int s = k ? X.lb[c] : X.la[c];
+      if (atomicCAS(&X.bl[s], -1, -2) == -1) {
+        const int idx = atomicAdd(&S.nbody, 1);
+        S.body[idx] = X.body[s];
+        S.dyn[idx] = X.dyn[s];
+        X.bl[s] = idx;
+      }
+    }
+  }
+  if (maxc) atomicMax(&S.ncol, maxc);
+  int low = 0, most = 0;
+  if (split)
+    for (int r = t; r < nbu; r += blockDim.x) {
+      if (r < rank) low += X.hist[r];
+      most = max(most, X.hist[r]);
+    }
+  low = warp_sum_i(low);
+  most = (int)__reduce_max_sync(0xffffffffu, (unsigned)most);
+  if ((t & 31) == 0) {
+    S.scan_w[t >> 5] = low;
+    S.mtile[t >> 5] = most;
+  }
+  __syncthreads();
+  Share sh{0, 0, split ? 0 : C, S.ncol};
+  if (split)
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+      sh.base += S.scan_w[w];
+      sh.most = max(sh.most, S.mtile[w]);
+    }
+  for (int k = 0; k < S.ncol; ++k) sh.count += S.cnt[k];
+  if (t == 0) {
+    int acc = 0;
+    for (int k = 0; k < S.ncol; ++k) {
+      S.coff[k] = acc;
+      acc += S.cnt[k];
+    }
+  }
+  __syncthreads();
+  for (int c = t; c < C; c += blockDim.x) {
+    if (split && X.blab[c] != rank) continue;
+    const int k = X.color[c];
+    const int p = S.coff[k] + atomicAdd(&S.cur[k], 1);
+    S.order[p] = (unsigned short)c;
+    S.pcol[p] = (unsigned char)k;
+    S.pa[p] = (unsigned short)X.bl[X.la[c]];
+    S.pb[p] = (unsigned short)X.bl[X.lb[c]];
+  }
+  __syncthreads();
+  return sh;
+}
+
+// One side of a manifold row: directions, this side's arm, inertia-applied
+// arms and inverse mass, omega / g per direction, bias terms, impulses.
+struct HalfRow {
+  d3 n, t1, t2, r, In, It1, It2;
+  double im, gn, gt1, gt2, bn, brest;
+  double ln, l1, l2;
+};
+
+__device__ inline d3 shfl_pair(unsigned mask, d3 a) {
+  return {__shfl_xor_sync(mask, a.x, 1), __shfl_xor_sync(mask, a.y, 1), __shfl_xor_sync(mask, a.z, 1)};
+}
+
+// build_row of contact c for one side (lane pairs of whole warps call it);
+// with feat, side 0 writes the learned start's features 0-6 of slot p.
+// Returns bit 0: impact, bit 1: in the warm cache (or a wall row).
+__device__ __noinline__ int build_half(const NscView& V, int c, int side, int W, const unsigned long long* keys,
+                                       HalfRow& h, float* feat, int p, double& phi_out, double& vnp_out) {
+  const State& st = V.st;
+  const Contacts& con = V.con;
+  const rg_config& cfg = V.cfg;
+  const unsigned all = 0xffffffffu;
+  const double beta = cfg.nsc_position_stabilization ? cfg.nsc_beta * 0.01 : cfg.nsc_beta;
+  const int a = con.a[c], b = con.b[c];
+  const int bd = side ? b : a;
+  const bool wall = a == b, live = !(wall && side);
+  const d3 n{con.comp(6)[c], con.comp(7)[c], con.comp(8)[c]};
+  const double phi = con.comp(12)[c] - con.comp(13)[c];
+  const int pk = side ? 3 : 0;
+  const d3 pt{con.comp(pk)[c], con.comp(pk + 1)[c], con.comp(pk + 2)[c]};
+  const d3 x = st.x.ld(bd), v = st.v.ld(bd), w = st.w.ld(bd), Iinv = st.Iinv.ld(bd);
+  const dq q = st.q.ld(bd);
+  const double im = live ? st.inv_mass[bd] : 0.0, rest = st.rest[bd];
+  const d3 sh{con.comp(9)[c], con.comp(10)[c], con.comp(11)[c]};
+  const d3 ref = fabs(n.x) < 0.9 ? mk3(1, 0, 0) : mk3(0, 1, 0);
+  const d3 cr = cross(n, ref);
+  const d3 t1 = cr / len(cr);
+  const d3 t2 = cross(n, t1);
+  d3 r = side ? pt - (x + sh) : pt - x;
+  if (!live) r = mk3(0, 0, 0);
+  // iinv_apply of the three arms (the columns of the rotation once)
+  d3 c0, c1, c2;
+  rot_cols(q, c0, c1, c2);
+  auto iinv = [&](d3 m) {
+    if (im <= 0.0) return mk3(0, 0, 0);
+    const double b0 = dot(c0, m) * Iinv.x, b1 = dot(c1, m) * Iinv.y, b2 = dot(c2, m) * Iinv.z;
+    return c0 * b0 + c1 * b1 + c2 * b2;
+  };
+  const d3 rn = cross(r, n), rt1 = cross(r, t1), rt2 = cross(r, t2);
+  h.n = n; h.t1 = t1; h.t2 = t2; h.r = r; h.im = im;
+  h.In = iinv(rn); h.It1 = iinv(rt1); h.It2 = iinv(rt2);
+  // diag_of: both sides' terms in the order 1/ma + 1/mb + A + B + cfm
+  const double imo = __shfl_xor_sync(all, im, 1);
+  const double ima = side ? imo : im, imb = side ? im : imo;
+  auto diag = [&](double mine) {
+    const double other = __shfl_xor_sync(all, mine, 1);
+    const double A = side ? other : mine, B = side ? mine : other;
+    const double g = ima + imb + A + B + cfg.nsc_cfm;
+    return cfg.nsc_omega / smax(g, 1e-12);
+  };
+  h.gn = diag(dot(rn, h.In));
+  h.gt1 = diag(dot(rt1, h.It1));
+  h.gt2 = diag(dot(rt2, h.It2));
+  d3 u = v + cross(w, r);
+  if (!live) u = mk3(0, 0, 0);
+  const d3 uo = shfl_pair(all, u);
+  const d3 uA = side ? uo : u, uB = side ? u : uo;
+  const d3 vrel = wall ? -uA : uB - uA;
+  const double vnp = dot(n, vrel);
+  const double ro = __shfl_xor_sync(all, rest, 1);
+  const double e = wall ? rest : (side ? smin(ro, rest) : smin(rest, ro));
+  h.bn = phi < 0.0 ? beta * phi / cfg.dt : 0.0;
+  h.brest = vnp < 0.0 ? e * vnp : 0.0;
+  int cached = wall ? 2 : 0;  // walls start cold and are left alone by the learned start
+  h.ln = h.l1 = h.l2 = 0.0;
+  if (!wall && cfg.nsc_warm_start != RG_WARM_NONE && W > 0) {
+    const unsigned long long k = ((unsigned long long)(unsigned)a << 32) | (unsigned)b;
+    const int f = lower_bound_key(keys, W, k);
+    if (f < W && keys[f] == k) {
+      cached = 2;
+      h.ln = smax(0.0, V.wlam[f]);
+      h.l1 = V.wlam[V.wcap + f];
+      h.l2 = V.wlam[2 * V.wcap + f];
+    }
+  }
+  if (feat && side == 0) {
+    const size_t fld = (size_t)V.ccap;
+    feat[p] = (float)phi;
+    feat[fld + p] = (float)vnp;
+    feat[2 * fld + p] = (float)dot(t1, vrel);
+    feat[3 * fld + p] = (float)dot(t2, vrel);
+    feat[4 * fld + p] = (float)h.ln;
+    feat[5 * fld + p] = (float)h.l1;
+    feat[6 * fld + p] = (float)h.l2;
+  }
+  phi_out = phi;
+  vnp_out = vnp;
+  return (vnp < -1e-6 ? 1 : 0) | cached;
+}
+
+// Half rows of slots beyond the registers: the global row arrays (RowIO).
+__device__ inline void half_store(const RowIO& R, int p, int side, const HalfRow& h) {
+  if (side == 0) {
+    R.w3(R_N, p, h.n); R.w3(R_T1, p, h.t1); R.w3(R_T2, p, h.t2);
+    R.r(R_GN, p) = h.gn; R.r(R_GT1, p) = h.gt1; R.r(R_GT2, p) = h.gt2;
+    R.r(R_BN, p) = h.bn; R.r(R_BREST, p) = h.brest;
+    R.lam[p] = h.ln; R.lam[R.ccap + p] = h.l1; R.lam[2 * (size_t)R.ccap + p] = h.l2;
+  }
+  R.w3(side ? R_RB : R_RA, p, h.r);
+  R.w3(side ? R_IBN : R_IAN, p, h.In);
+  R.w3(side ? R_IBT1 : R_IAT1, p, h.It1);
+  R.w3(side ? R_IBT2 : R_IAT2, p, h.It2);
+  R.r(side ? R_IMB : R_IMA, p) = h.im;
+}
+__device__ inline void half_load(const RowIO& R, int p, int side, HalfRow& h) {
+  h.n = R.r3(R_N, p); h.t1 = R.r3(R_T1, p); h.t2 = R.r3(R_T2, p);
+  h.gn = R.r(R_GN, p); h.gt1 = R.r(R_GT1, p); h.gt2 = R.r(R_GT2, p);
+  h.bn = R.r(R_BN, p); h.brest = R.r(R_BREST, p);
+  h.ln = R.lam[p]; h.l1 = R.lam[R.ccap + p]; h.l2 = R.lam[2 * (size_t)R.ccap + p];
+  h.r = R.r3(side ? R_RB : R_RA, p);
+  h.In = R.r3(side ? R_IBN : R_IAN, p);
+  h.It1 = R.r3(side ? R_IBT1 : R_IAT1, p);
+  h.It2 = R.r3(side ? R_IBT2 : R_IAT2, p);
+  h.im = R.r(side ? R_IMB : R_IMA, p);
+}
+
+// The six numbers of a body slot (three 16-byte words).
+__device__ inline void slot_ld(const double* vs, d3& v, d3& w) {
+  const double2 p = *reinterpret_cast<const double2*>(vs), q = *reinterpret_cast<const double2*>(vs + 2),
+                r = *reinterpret_cast<const double2*>(vs + 4);
+  v = mk3(p.x, p.y, q.x);
+  w = mk3(q.y, r.x, r.y);
+}
+__device__ inline void slot_st(double* vs, d3 v, d3 w) {
+  *reinterpret_cast<double2*>(vs) = make_double2(v.x, v.y);
+  *reinterpret_cast<double2*>(vs + 2) = make_double2(v.z, w.x);
+  *reinterpret_cast<double2*>(vs + 4) = make_double2(w.y, w.z);
+}
+
+// Warm-start impulses of one side (warm_apply).
+__device__ inline void warm_half(const HalfRow& h, double* vs, int side) {
+  d3 v, w;
+  slot_ld(vs, v, w);
+  auto imp = [&](d3 d, d3 I, double l) {
+    if (l == 0.0) return;
+    const d3 dv = d * (l * h.im), dw = I * l;
+    v = side ? v + dv : v - dv;
+    w = side ? w + dw : w - dw;
+  };
+  imp(h.n, h.In, h.ln);
+  imp(h.t1, h.It1, h.l1);
+  imp(h.t2, h.It2, h.l2);
+  slot_st(vs, v, w);
+}
+
+// sqrt(max(0, a)), without the square root's special-value path for the
+// a <= 0 of contacts at or inside their friction limit's end.
+__device__ inline double cone_limit(double a) { return a > 0.0 ? sqrt(a) : 0.0; }
+
+// One Gauss-Seidel row update by a lane pair (psor_row); act: the lanes of
+// the warp that call it.  Both lanes form the same relative velocity and
+// impulses; each updates its own body.  Straight-line: an impulse change of
+// zero adds zero instead of branching around the update (a branch per
+// direction and the reconvergence after it took a fifth of the 1,450 cycles
+// of the branching form; 1,160 now, two square roots among them).  Returns
+// |dλn| + |dλt1| + |dλt2|.
+__device__ __forceinline__ double psor_half(HalfRow& h, double* vs, int side, bool wall, unsigned act, double cfm,
+                                            double mu) {
+  const bool live = !(wall && side);  // a wall takes no impulse and stays at rest
+  d3 v{0, 0, 0}, w{0, 0, 0};
+  if (live) slot_ld(vs, v, w);
+  const d3 u = v + cross(w, h.r);
+  const d3 uo = shfl_pair(act, u);
+  const d3 uA = side ? uo : u, uB = side ? u : uo;
+  d3 vrel = wall ? -uA : uB - uA;
+  // impulse change d along dir: this side's velocities, and the change of
+  // the relative velocity it makes (side A's first, then side B's)
+  auto kick = [&](d3 dir, d3 I, double d, bool last) {
+    const d3 dv = dir * (d * h.im), dw = I * d;
+    v = side ? v + dv : v - dv;
+    w = side ? w + dw : w - dw;
+    if (last) return;
+    const d3 X = dv + cross(dw, h.r);
+    const d3 Xo = shfl_pair(act, X);
+    vrel = vrel + (side ? Xo : X);
+    vrel = vrel + (side ? X : Xo);
+  };
+  const double wn = dot(h.n, vrel) + h.bn + h.brest + cfm * h.ln;
+  const double ln = smax(0.0, h.ln + -h.gn * wn);
+  const double dn = ln - h.ln;
+  kick(h.n, h.In, dn, false);
+  const double mf = mu * ln;
+  const double lim1 = cone_limit(mf * mf - h.l2 * h.l2);
+  const double w1 = dot(h.t1, vrel) + cfm * h.l1;
+  const double l1 = smin(smax(h.l1 + -h.gt1 * w1, -lim1), lim1);
+  const double d1 = l1 - h.l1;
+  kick(h.t1, h.It1, d1, false);
+  const double lim2 = cone_limit(mf * mf - l1 * l1);
+  const double w2 = dot(h.t2, vrel) + cfm * h.l2;
+  const double l2 = smin(smax(h.l2 + -h.gt2 * w2, -lim2), lim2);
+  const double d2 = l2 - h.l2;
+  kick(h.t2, h.It2, d2, true);
+  if (live) slot_st(vs, v, w);
+  h.ln = ln; h.l1 = l1; h.l2 = l2;
+  return fabs(dn) + fabs(d1) + fabs(d2);
+}
+
+// ---- sweeps of a block's share ----------------------------------------------
+// Up to n sweeps; with stop >= 0 the block alone decides and leaves after the
+// first sweep whose every change is below `stop`.  S.locs gets each sweep's
+// residuals (per lane of the one warp, else per warp).  Returns the sweeps
+// made; fewer than n with stop < 0 only when the last one changed nothing
+// (so further ones would not either).  The state after sweep i < keep goes to
+// S.vel[snap + i stride]: 6 nbody velocities, then the impulses per slot.
+struct Sweep {
+  int colors, n;
+  double stop;
+  int keep, snap, stride;
+};
+template <bool ONE>
+__device__ __forceinline__ void sweep_sync() {
+  if (ONE) __syncwarp();
+  else __syncthreads();
+}
+// ONE: at most 16 contacts, the first warp only and no block barrier.
+template <bool ONE, class Row, class Update>
+__device__ __forceinline__ int sweep_share(const Sweep w, int C, Row& h, Update update) {
+  SmallSmem& S = small_smem();
+  const int t = threadIdx.x, pair = t >> 1, side = t & 1;
+  if (ONE && t >= 32) return 0;
+  const int col = pair < C ? (int)S.pcol[pair] : -1;
+  const int q0 = pair < C ? pair : 0;
+  const bool wall = S.pa[q0] == S.pb[q0];
+  double* vs = &S.vel[6 * (side ? S.pb[q0] : S.pa[q0])];
+  const int nv = 6 * S.nbody;
+  int i = 0;
+  while (i < w.n) {
+    double loc = 0.0;
+    for (int k = 0; k < w.colors; ++k) {
+      const bool mine = col == k;
+      const unsigned act = __ballot_sync(0xffffffffu, mine);
+      if (mine) loc = update(h, vs, side, wall, act);
+      if (k + 1 < w.colors) sweep_sync<ONE>();
+    }
+    double* ls = &S.locs[(i & (kChunk - 1)) * 32];
+    if (ONE) {
+      ls[t] = loc;
+    } else {
+      const double m = warp_max(loc);
+      if ((t & 31) == 0) ls[t >> 5] = m;
+    }
+    ++i;
+    if (ONE) __syncwarp();  // (the vote below orders nothing)
+    // one vote: goes on while a change reaches the limit (or, in a chunk,
+    // while anything changes)
+    const int more = w.stop >= 0.0 ? loc >= w.stop : loc != 0.0;
+    if (!(ONE ? __any_sync(0xffffffffu, more) : __syncthreads_or(more))) break;
+    if (i <= w.keep) {  // state after sweep i - 1
+      double* sn = &S.vel[w.snap + (i - 1) * w.stride];
+      for (int k = t; k < nv; k += ONE ? 32 : blockDim.x) sn[k] = S.vel[k];
+      if (pair < C && side == 0) h.keep(sn + nv, pair);
+      sweep_sync<ONE>();
+    }
+  }
+  return i;
+}
+// The same over more contacts than lane pairs: rows from the global arrays.
+template <class Row, class Update>
+__device__ __forceinline__ int sweep_rows(const Sweep w, int C, const RowIO R, Update update) {
+  SmallSmem& S = small_smem();
+  const int t = threadIdx.x, pair = t >> 1, side = t & 1;
+  int i = 0;
+  while (i < w.n) {
+    double loc = 0.0;
+    for (int k = 0; k < w.colors; ++k) {
+      for (int p0 = S.coff[k] & ~(kPairs - 1); p0 < S.coff[k] + S.cnt[k]; p0 += kPairs) {
+        const int p = p0 + pair;
+        const bool mine = p >= S.coff[k] && p < S.coff[k] + S.cnt[k];
+        const unsigned act = __ballot_sync(0xffffffffu, mine);
+        if (!mine) continue;
+        Row g;
+        g.load(R, p, side);
+        const int sa = S.pa[p], sb = S.pb[p];
+        loc = fmax(loc, update(g, &S.vel[6 * (size_t)(side ? sb : sa)], side, sa == sb, act));
+        __syncwarp(act);  // both lanes have read the impulses
+        if (side == 0) g.put(R, p);
+      }
+      if (k + 1 < w.colors) __syncthreads();
+    }
+    const double m = warp_max(loc);
+    if ((t & 31) == 0) S.locs[(i & (kChunk - 1)) * 32 + (t >> 5)] = m;
+    ++i;
+    const int more = w.stop >= 0.0 ? loc >= w.stop : loc != 0.0;
+    if (!__syncthreads_or(more)) break;
+  }
+  return i;
+}
+
+// Sweeps until the residual over the whole team is below tol, or max_it.
+// run(w) makes sweeps, back(state) puts a kept state's impulses (nl a slot)
+// back.  Returns false on a team error; res and sweeps as a single solver's.
+template <class Run, class Back>
+__device__ __forceinline__ bool sweep_until(const Team& T, const Share& sh, int nl, int max_it, double tol, int first,
+                                            unsigned& chunk, Run run, Back back, double& res, int& sweeps) {
+  SmallSmem& S = small_smem();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarp = (int)(blockDim.x >> 5);
+  const int width = sh.count <= 16 ? 32 : nwarp;
+  auto residual = [&](int i) {  // of sweep i, by every warp that calls it
+    return warp_max(lane < width ? S.locs[(i & (kChunk - 1)) * 32 + lane] : 0.0);
+  };
+  res = 0.0;
+  sweeps = 0;
+  if (T.nb == 1) {
+    const int made = sh.count ? run(Sweep{sh.colors, max_it, tol, 0, 0, 0}) : 0;
+    if (t == 0) S.nloc = made;  // (the one-warp form returns 0 in the other warps)
+    __syncthreads();
+    sweeps = S.nloc;
+    if (sweeps) res = residual(sweeps - 1);
+    __syncthreads();
+    return true;
+  }
+  if (max_it <= 0) return team_sync(T);  // every block has read what the others now write
+  const int nv = 6 * S.nbody, stride = nv + nl * sh.count;
+  // states that fit the velocity space of every block (two bodies a contact
+  // at most); none where the impulses live in the global arrays
+  const int room = sh.most > kPairs ? 0 : (kVel - 12 * sh.most) / ((12 + nl) * sh.most);
+  int size = first;
+  bool still = sh.count == 0;
+  while (sweeps < max_it) {
+    const int n = min(min(size, room + 1), max_it - sweeps);
+    size = kChunk;
+    int made = 0;
+    if (!still) {
+      made = run(Sweep{sh.colors, n, -1.0, n - 1, nv, stride});
+      if (t == 0) S.nloc = made;
+      __syncthreads();
+      made = S.nloc;
+    }
+    // publish; the buffer after this one is cleared for the next chunk (every
+    // block has read its last use: it arrived at the barrier after that)
+    double* ring = T.ring() + (chunk % 3) * kChunk;
+    for (int i = warp; i < made; i += nwarp) {
+      const double v = residual(i);
+      if (lane == 0 && v > 0.0) atomic_max_nonneg(&ring[i], v);
+    }
+    if (T.rank() == 0 && t < kChunk) T.ring()[((chunk + 1) % 3) * kChunk + t] = 0.0;
+    ++chunk;
+    if (!team_sync(T)) return false;
+    if (t < n) S.res[t] = __ldcg(&ring[t]);
+    __syncthreads();
+    int m = 0;
+    while (m < n && !(S.res[m] < tol)) ++m;
+    const bool done = m < n;
+    if (!done) m = n - 1;
+    res = S.res[m];
+    sweeps += m + 1;
+    if (!still && m < made - 1) {  // back to the state after sweep m
+      const double* sn = &S.vel[nv + m * stride];
+      for (int k = t; k < nv; k += blockDim.x) S.vel[k] = sn[k];
+      back(sn + nv);
+    }
+    // a share that a sweep left unchanged is done
+    if (!done && made < n) still = true;
+    __syncthreads();
+    if (done) break;
+  }
+  return true;
+}
+
+// The impulse part of a velocity row, and its place in the global arrays.
+struct VelRow : HalfRow {
+  __device__ void keep(double* o, int p) const { o[3 * p] = ln; o[3 * p + 1] = l1; o[3 * p + 2] = l2; }
+  __device__ void back(const double* o, int p) { ln = o[3 * p]; l1 = o[3 * p + 1]; l2 = o[3 * p + 2]; }
+  __device__ void load(const RowIO& R, int p, int side) { half_load(R, p, side, *this); }
+  __device__ void put(const RowIO& R, int p) const {
+    R.lam[p] = ln; R.lam[R.ccap + p] = l1; R.lam[2 * (size_t)R.ccap + p] = l2;
+  }
+};
+template <bool ONE>
+__device__ __noinline__ int vel_sweep(const Sweep w, int C, VelRow& row, double cfm, double mu) {
+  VelRow h = row;
+  const int made = sweep_share<ONE>(w, C, h, [&](VelRow& r, double* vs, int side, bool wall, unsigned act) {
+    return psor_half(r, vs, side, wall, act, cfm, mu);
+  });
+  row.ln = h.ln; row.l1 = h.l1; row.l2 = h.l2;
+  return made;
+}
+__device__ __noinline__ int vel_sweep_rows(const Sweep w, int C, const RowIO R, double cfm, double mu) {
+  return sweep_rows<VelRow>(w, C, R, [&](VelRow& r, double* vs, int side, bool wall, unsigned act) {
+    return psor_half(r, vs, side, wall, act, cfm, mu);
+  });
+}
+
+// Contact sets that the team's first block solves alone: those that fit its
+// registers (a chunk's barrier costs more than the sweeps it saves), and
+// recorded ones, whose records keep one block's slot order.
+__device__ inline bool solo(int C, bool recording) { return C <= kPairs || recording; }
+
 // Colouring, manifold rows, PSOR and the warm cache for C <= kSmallC.
-__device__ __noinline__ bool small_solve(const NscView& V, int C, int Cp, SmallSmem& S, PhaseClock& pc) {
+__device__ __noinline__ bool small_solve(const Team& team, const NscView& V, int C, int Cp, unsigned& chunk,
+                                         PhaseClock& pc) {
+  SmallSmem& S = small_smem();
+  if (solo(C, V.rec_cap > 0) && team.rank() != 0) return true;
+  Team T = team;
+  if (solo(C, V.rec_cap > 0)) T.nb = 1;
   Ctl* ctl = V.ctl;
   const rg_config& cfg = V.cfg;
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, pair = t >> 1, side = t & 1;
+  if (C == 0) {
+    if (t == 0) {
+      *V.wn = 0;
+      ctl->colors = 0;
+      ctl->vel_contacts = 0;
+      ctl->residual = 0.0;
+      ctl->sweeps_last = 0;
+    }
+    return true;
+  }
   // the learned start's gate is known now: its first hidden layer travels to
   // shared memory while the colouring and the rows are built
   const bool mlp_gate = V.use_mlp && (*(volatile int*)V.wn == 0 ||
                                       *(volatile int*)&ctl->sweeps_last > V.mlp_min_sweeps);
+  const int W = *(volatile int*)V.wn;
+  const int rec_base = V.rec_cap > 0 ? *(volatile int*)&ctl->rec_n : 0;
   if (mlp_gate) stage_bf16(S.wh, kWhLd, V.mlp.w2, kMlpH, kMlpH);
-  small_map(V, C, S);
+  small_map(V, C);
   pc.mark(10);
-  int K = small_color(V, C, S);
+  const int K = small_color(V, C, T.rank() == 0);
   if (K < 0) {
     if (mlp_gate) stage_wait();
     return false;
   }
+  const Share sh = small_split(T, C, K);
+  const int Cl = sh.count;
   pc.mark(2);
-  // body velocities on chip
-  for (int s = t; s < S.nloc; s += blockDim.x) {
-    int x = S.body[s];
-    if (x < 0) continue;
-    d3 v = V.st.v.ld(x), w = V.st.w.ld(x);
-    S.vel[s] = v.x; S.vel[kSmallB + s] = v.y; S.vel[2 * kSmallB + s] = v.z;
-    S.vel[3 * kSmallB + s] = w.x; S.vel[4 * kSmallB + s] = w.y; S.vel[5 * kSmallB + s] = w.z;
+  // ---- manifold rows: slot j kPairs + pair of a lane pair, j = 0, 1, .. ----
+  const unsigned long long* keys = V.wkey;
+  if (cfg.nsc_warm_start != RG_WARM_NONE && W <= kVel && Cl > 0) {
+    unsigned long long* ks = reinterpret_cast<unsigned long long*>(S.vel);
+    for (int k = t; k < W; k += blockDim.x) ks[k] = V.wkey[k];
+    keys = ks;
   }
-  RowIO R{S.row, S.lam, kSmallC};
-  const int W = *(volatile int*)V.wn;
-  int* deg = reinterpret_cast<int*>(S.pmax);  // free after colouring
-  if (V.feat_on) {
-    for (int s = t; s < S.nloc; s += blockDim.x) deg[s] = 0;
-    __syncthreads();
-  }
+  int* deg = reinterpret_cast<int*>(S.stage);
+  if (V.feat_on)
+    for (int s = t; s < S.nbody; s += blockDim.x) deg[s] = 0;
+  __syncthreads();
+  const size_t cc = (size_t)V.ccap;
+  const RowIO R{V.row + sh.base, V.lam + sh.base, V.ccap};  // this block's slots
+  float* feat = V.feat + sh.base;
+  const int nt = (Cl + kPairs - 1) / kPairs;
+  VelRow row = {};
   int coll = 0;
-  if (t < C) {
-    const int c = S.order[t];
-    const int br = build_row(V.st, V.con, cfg, c, t, R, V.wkey, V.wlam, W, V.wcap, V.feat_on ? S.feat : nullptr,
-                             kSmallC);
-    coll = br & 1;
-    S.cached[t] = (unsigned char)(br >> 1);
-    if (V.feat_on && c < Cp) {  // wall rows (after the pairs) have no graph degree
-      if (S.dyn[S.la[c]]) atomicAdd(&deg[S.la[c]], 1);
-      if (S.dyn[S.lb[c]]) atomicAdd(&deg[S.lb[c]], 1);
+#pragma unroll 1
+  for (int j = 0; j < nt; ++j) {
+    const int p = j * kPairs + pair;
+    if (j * kPairs + (t >> 5) * 16 >= Cl) continue;  // no contact in this warp
+    const bool valid = p < Cl;
+    const int c = S.order[valid ? p : Cl - 1];
+    double phi, vnp;
+    const int br = build_half(V, c, side, W, keys, row, V.feat_on && valid ? feat : nullptr, p, phi, vnp);
+    if (!valid) continue;
+    if (nt > 1) half_store(R, p, side, row);
+    if (side == 0) {
+      coll += br & 1;
+      S.cached[p] = (unsigned char)(br >> 1);
+    }
+    if (c < Cp) {  // wall rows (after the pairs) have no graph degree and no export
+      const int sl = side ? S.pb[p] : S.pa[p];
+      if (V.feat_on && S.dyn[sl]) atomicAdd(&deg[sl], 1);
+      if (V.xrow) {  // contact-network export, warm-cache order
+        const size_t wc = (size_t)V.wcap;
+        double* xr = V.xrow + c;
+        const int k0 = side ? 6 : 3;
+        xr[k0 * wc] = row.r.x; xr[(k0 + 1) * wc] = row.r.y; xr[(k0 + 2) * wc] = row.r.z;
+        if (side == 0) {
+          xr[0] = row.n.x; xr[wc] = row.n.y; xr[2 * wc] = row.n.z;
+          xr[9 * wc] = phi; xr[10 * wc] = vnp;
+        }
+      }
     }
   }
-  int bcoll = __syncthreads_count(coll);
-  if (t == 0 && bcoll) atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->collisions), (unsigned long long)bcoll);
+  coll = warp_sum_i(coll);
+  if ((t & 31) == 0 && coll) atomicAdd(reinterpret_cast<unsigned long long*>(&ctl->collisions), (unsigned long long)coll);
+  __syncthreads();
   if (V.feat_on) {
-    if (t < C) {
-      const int c = S.order[t], sa = S.la[c], sb = S.lb[c];
-      S.feat[7 * kSmallC + t] = (float)((S.dyn[sa] ? deg[sa] - 1 : 0) + (S.dyn[sb] ? deg[sb] - 1 : 0));
+    for (int p = t; p < Cl; p += blockDim.x) {
+      const int sa = S.pa[p], sb = S.pb[p];
+      feat[7 * cc + p] = (float)((S.dyn[sa] ? deg[sa] - 1 : 0) + (S.dyn[sb] ? deg[sb] - 1 : 0));
     }
-    __syncthreads();
     if (mlp_gate) {
       // the contacts the learned start is for (every contact, or those new
       // since the last step); the network runs only on tiles that hold one
-      const bool want = t < C && S.order[t] < Cp && (V.mlp_all || !S.cached[t]);  // never a wall row
-      if (t < kSmallC / 16) S.mtile[t] = 0;
+      for (int k = t; k < kSmallC / 16; k += blockDim.x) S.mtile[k] = 0;
       __syncthreads();
-      if (want) S.mtile[t >> 4] = 1;
-      if (__syncthreads_or(want)) {
+      unsigned want = 0;
+      for (int j = 0; j < nt; ++j) {
+        const int p = j * kPairs + pair;
+        if (p < Cl && S.order[p] < Cp && (V.mlp_all || !S.cached[p])) want |= 1u << j;  // never a wall row
+        if ((want >> j) & 1u) S.mtile[p >> 4] = 1;
+      }
+      if (__syncthreads_or((int)want)) {
         // one warp per 16 contacts on the tensor cores, then the cone.  The
         // weights come from shared memory: W1, W4 and the small parameters
-        // in pmax/cmask (free after colouring and degrees), the hidden
-        // layers one after the other in wh.
-        const MlpStage ms = mlp_stage_at(S.pmax);
+        // in stage, W2 in wh, W3 in the space of the velocities.
+        const MlpStage ms = mlp_stage_at(S.stage);
+        __nv_bfloat16* w3s = reinterpret_cast<__nv_bfloat16*>(S.vel);
+        float* pred = V.pred + sh.base;
         stage_small(ms, V.mlp);  // W2 is already on its way (start of the solve)
+        stage_bf16(w3s, kWhLd, V.mlp.w3, kMlpH, kMlpH);
         stage_wait();
         __syncthreads();
-        const int row0 = (t >> 5) * 16, lane = t & 31;
-        const bool mine = row0 < C && S.mtile[t >> 5];
         const MlpSmall q = ms.small();
-        unsigned a[8][4];
-        if (mine) {
-          mlp_layer1(ms.w1, kW1Ld, q, S.feat, kSmallC, row0, C, lane, a);
+        const int lane = t & 31;
+        for (int tile = t >> 5; tile * 16 < Cl; tile += blockDim.x >> 5) {
+          if (!S.mtile[tile]) continue;
+          unsigned a[8][4];
+          mlp_layer1(ms.w1, kW1Ld, q, feat, V.ccap, tile * 16, Cl, lane, a);
           hidden_layer(a, S.wh, kWhLd, q.b2, lane);
+          hidden_layer(a, w3s, kWhLd, q.b3, lane);
+          mlp_layer4(a, ms.w4, kWhLd, q, pred, V.ccap, tile * 16, Cl, lane);
         }
         __syncthreads();
-        stage_bf16(S.wh, kWhLd, V.mlp.w3, kMlpH, kMlpH);
-        stage_wait();
-        __syncthreads();
-        if (mine) {
-          hidden_layer(a, S.wh, kWhLd, q.b3, lane);
-          mlp_layer4(a, ms.w4, kWhLd, q, S.pred, kSmallC, row0, C, lane);
+        for (int j = 0; j < nt; ++j) {
+          if (!((want >> j) & 1u)) continue;
+          const int p = j * kPairs + pair;
+          if (nt == 1) mlp_apply(row.ln, row.l1, row.l2, pred, V.ccap, p, cfg.nsc_mu);
+          else if (side == 0) mlp_apply(R.lam[p], R.lam[cc + p], R.lam[2 * cc + p], pred, V.ccap, p, cfg.nsc_mu);
         }
-        __syncthreads();
-        if (want) mlp_apply(R, S.pred, kSmallC, t, cfg.nsc_mu);
-        __syncthreads();
       }
     }
   }
   if (mlp_gate) stage_wait();  // no copy outlives the solve
+  // body velocities on chip (the keys and the third layer are done with)
+  __syncthreads();
+  for (int s = t; s < S.nbody; s += blockDim.x) {
+    const int x = S.body[s];
+    slot_st(&S.vel[6 * s], V.st.v.ld(x), V.st.w.ld(x));
+  }
+  __syncthreads();
   pc.mark(3);
-  Vel Vv{Vec3A{S.vel, S.vel + kSmallB, S.vel + 2 * kSmallB},
-         Vec3A{S.vel + 3 * kSmallB, S.vel + 4 * kSmallB, S.vel + 5 * kSmallB}};
-  const double omega = cfg.nsc_omega, cfm = cfg.nsc_cfm, mu = cfg.nsc_mu;
-  const int p = t;
-  const int c = p < C ? S.order[p] : 0;
-  int my_color = -1;
-  if (p < C)
-    for (int k = 0; k < K; ++k)
-      if (p >= S.coff[k] && p < S.coff[k + 1]) my_color = k;
+  // ---- PSOR ----
+  const double cfm = cfg.nsc_cfm, mu = cfg.nsc_mu, tol = cfg.nsc_tol;
   if (cfg.nsc_warm_start != RG_WARM_NONE) {
-    for (int k = 0; k < K; ++k) {
-      if (my_color == k) warm_apply(R, Vv, p, S.la[c], S.lb[c]);
+    for (int k = 0; k < sh.colors; ++k) {
+      for (int j = 0; j < nt; ++j) {
+        const int p = j * kPairs + pair;
+        if (p >= Cl || S.pcol[p] != k || (S.pa[p] == S.pb[p] && side)) continue;
+        double* vs = &S.vel[6 * (size_t)(side ? S.pb[p] : S.pa[p])];
+        if (nt == 1) {
+          warm_half(row, vs, side);
+        } else {
+          VelRow g;
+          g.load(R, p, side);
+          warm_half(g, vs, side);
+        }
+      }
       __syncthreads();
     }
   }
   double res = 0.0;
   int sweeps = 0;
-  for (int it = 0; C > 0 && it < cfg.nsc_velocity_iters; ++it) {
-    double loc = 0.0;
-    for (int k = 0; k < K; ++k) {
-      if (my_color == k) loc = psor_row(R, Vv, p, S.la[c], S.lb[c], omega, cfm, mu);
-      __syncthreads();
-    }
-    res = small_block_max(loc, S);
-    sweeps = it + 1;
-    if (res < cfg.nsc_tol) break;
-  }
-  __syncthreads();
+  const bool ok = sweep_until(
+      T, sh, 3, cfg.nsc_velocity_iters, tol, 8, chunk,
+      [&](const Sweep& w) {
+        if (nt > 1) return vel_sweep_rows(w, Cl, R, cfm, mu);
+        return Cl <= 16 ? vel_sweep<true>(w, Cl, row, cfm, mu) : vel_sweep<false>(w, Cl, row, cfm, mu);
+      },
+      [&](const double* o) {
+        if (pair < Cl) row.back(o, pair);
+      },
+      res, sweeps);
+  if (!ok) return false;
   pc.mark(4);
   // velocities back; warm cache and impulse sums (contact order)
-  for (int s = t; s < S.nloc; s += blockDim.x) {
-    int x = S.body[s];
-    if (x < 0) continue;
-    V.st.v.st(x, mk3(S.vel[s], S.vel[kSmallB + s], S.vel[2 * kSmallB + s]));
-    V.st.w.st(x, mk3(S.vel[3 * kSmallB + s], S.vel[4 * kSmallB + s], S.vel[5 * kSmallB + s]));
-  }
-  small_unmap(V, S);
-  if (V.rec_cap > 0 && C > 0) {
-    // records (features, converged impulses) in slot order
-    const int base = *(volatile int*)&ctl->rec_n;
-    if (p < C && base + p < V.rec_cap) {
-      const size_t r = (size_t)(base + p);
-      for (int k = 0; k < kMlpIn; ++k) V.rec_x[r * kMlpIn + k] = S.feat[k * kSmallC + p];
-      for (int k = 0; k < kMlpOut; ++k) V.rec_y[r * kMlpOut + k] = (float)S.lam[k * kSmallC + p];
-    }
-    __syncthreads();
-    if (t == 0) ctl->rec_n = base + C;
+  for (int s = t; s < S.nbody; s += blockDim.x) {
+    if (!S.dyn[s]) continue;
+    const int x = S.body[s];
+    d3 v, w;
+    slot_ld(&S.vel[6 * s], v, w);
+    V.st.v.st(x, v);
+    V.st.w.st(x, w);
   }
   double jn = 0, jt = 0;
-  if (p < C) {
-    double l0 = S.lam[p], l1 = S.lam[kSmallC + p], l2 = S.lam[2 * kSmallC + p];
+  for (int j = 0; j < nt && side == 0; ++j) {
+    const int p = j * kPairs + pair;
+    if (p >= Cl) break;
+    const int c = S.order[p];
+    const bool reg = nt == 1;
+    const double l0 = reg ? row.ln : R.lam[p], l1 = reg ? row.l1 : R.lam[cc + p], l2 = reg ? row.l2 : R.lam[2 * cc + p];
     if (c < Cp) {  // wall rows start cold every step: they stay out of the cache
       V.wkey[c] = ((unsigned long long)(unsigned)V.con.a[c] << 32) | (unsigned)V.con.b[c];
       V.wlam[c] = l0;
       V.wlam[V.wcap + c] = l1;
       V.wlam[2 * V.wcap + c] = l2;
-      reinterpret_cast<int*>(V.wlam + 3 * (size_t)V.wcap)[c] = S.color[c];
-      if (V.xrow) export_row(V.xrow, V.wcap, c, R, p);
+      reinterpret_cast<int*>(V.wlam + 3 * (size_t)V.wcap)[c] = S.pcol[p];
     }
-    jn = fabs(l0);  // profile-CSV sums of main.cpp:3339-3343
-    jt = fabs(l1) + fabs(l2);
+    if (V.rec_cap > 0 && rec_base + p < V.rec_cap) {
+      // record (features, converged impulses) in slot order
+      const size_t r = (size_t)(rec_base + p);
+      for (int k = 0; k < kMlpIn; ++k) V.rec_x[r * kMlpIn + k] = feat[(size_t)k * cc + p];
+      V.rec_y[r * kMlpOut] = (float)l0;
+      V.rec_y[r * kMlpOut + 1] = (float)l1;
+      V.rec_y[r * kMlpOut + 2] = (float)l2;
+    }
+    jn += fabs(l0);  // profile-CSV sums of main.cpp:3339-3343
+    jt += fabs(l1) + fabs(l2);
   }
   jn = warp_sum(jn);
   jt = warp_sum(jt);
@@ -1113,7 +1746,9 @@ __device__ __noinline__ bool small_solve(const NscView& V, int C, int Cp, SmallS
     atomicAdd(&ctl->jn_sum, jn);
     atomicAdd(&ctl->jt_sum, jt);
   }
-  if (t == 0) {
+  __syncthreads();
+  if (t == 0 && T.rank() == 0) {
+    if (V.rec_cap > 0 && C > 0) ctl->rec_n = rec_base + C;
     *V.wn = Cp;
     ctl->vel_contacts = C;
     ctl->residual = res;
@@ -1129,116 +1764,236 @@ __device__ __noinline__ bool small_solve(const NscView& V, int C, int Cp, SmallS
   return true;
 }
 
-// Position projection for C <= kSmallC (nsc_contact.cpp:698-879).
-__device__ __noinline__ bool small_project(const NscView& V, int C, SmallSmem& S) {
+// One side of a projection row: normal, arm, inertia-applied arm, inverse
+// mass, phi + slop, omega / g and the accumulated correction.
+struct HalfPos {
+  d3 n, r, In;
+  double im, phi, og, l;
+};
+// What a lane keeps of its body and contact over the projection passes.
+struct PosSide {
+  d3 Iinv;
+  double im, h, rsum;
+};
+// The row of a contact for one side at its body's position x, q (lane pairs
+// of whole warps call it): the geometry the detection computes, from the
+// pair's own positions.  Returns 1 when the contact penetrates.
+__device__ __noinline__ int build_half_pos(const NscView& V, const d3 x, const dq q, const PosSide& b, int side,
+                                           HalfPos& h) {
+  const rg_config& cfg = V.cfg;
+  const unsigned all = 0xffffffffu;
+  const d3 u = axis_y(q);
+  const d3 xo = shfl_pair(all, x), uo = shfl_pair(all, u);
+  const double ho = __shfl_xor_sync(all, b.h, 1), imo = __shfl_xor_sync(all, b.im, 1);
+  const d3 xa = side ? xo : x, ua = side ? uo : u, xb = side ? x : xo, ub = side ? u : uo;
+  const Seg A{xa.x, xa.y, xa.z, side ? ho : b.h, ua.x, ua.y, ua.z, 0.0};
+  const Seg B{xb.x, xb.y, xb.z, side ? b.h : ho, ub.x, ub.y, ub.z, 0.0};
+  const Narrow nr = narrow_pair(A, B, V.box);
+  const d3 diff = nr.pb - nr.pa;
+  const double dist = len(diff);
+  const double phi = dist - b.rsum;
+  const int act = phi < -cfg.nsc_slop ? 1 : 0;
+  if (!__any_sync(all, act)) return 0;
+  const d3 nv = dist > 1e-10 ? diff / dist : mk3(1, 0, 0);
+  const d3 r = side ? nr.pb - (xb + nr.sh) : nr.pa - xa;
+  const d3 rn = cross(r, nv);
+  h.n = nv; h.r = r;
+  h.im = b.im;
+  h.In = b.im <= 0.0 ? mk3(0, 0, 0) : rot_diag_apply(q, b.Iinv, rn);
+  const double mine = dot(rn, h.In), other = __shfl_xor_sync(all, mine, 1);
+  const double g = (side ? imo : h.im) + (side ? h.im : imo) + (side ? other : mine) + (side ? mine : other) + cfg.nsc_cfm;
+  h.og = cfg.nsc_omega / smax(g, 1e-12);
+  h.phi = phi + cfg.nsc_slop;
+  h.l = 0.0;
+  return act;
+}
+__device__ inline void half_pos_store(const RowIO& R, int p, int side, const HalfPos& h) {
+  if (side == 0) {
+    R.w3(R_N, p, h.n);
+    R.r(R_PHI, p) = h.phi;
+    R.r(R_GN, p) = h.og;
+    R.lam[p] = h.l;
+  }
+  R.w3(side ? R_RB : R_RA, p, h.r);
+  R.w3(side ? R_IBN : R_IAN, p, h.In);
+  R.r(side ? R_IMB : R_IMA, p) = h.im;
+}
+__device__ inline void half_pos_load(const RowIO& R, int p, int side, HalfPos& h) {
+  h.n = R.r3(R_N, p);
+  h.phi = R.r(R_PHI, p);
+  h.og = R.r(R_GN, p);
+  h.l = R.lam[p];
+  h.r = R.r3(side ? R_RB : R_RA, p);
+  h.In = R.r3(side ? R_IBN : R_IAN, p);
+  h.im = R.r(side ? R_IMB : R_IMA, p);
+}
+// One projection row update by a lane pair; vs: dx, dθ of this side's slot.
+// Returns |dλ|.
+__device__ __forceinline__ double pos_half(HalfPos& h, double* vs, int side, unsigned act, int penetrates, double cfm) {
+  d3 dx, dt;
+  slot_ld(vs, dx, dt);
+  const d3 cr = cross(dt, h.r);
+  // n . (((dx_b + dθ_b x r_b) - dx_a) - dθ_a x r_a)
+  const d3 mine = side ? dx + cr : dx;
+  const d3 other = shfl_pair(act, mine), cro = shfl_pair(act, cr);
+  const d3 rel = side ? (mine - other) - cro : (other - mine) - cr;
+  if (!penetrates) return 0.0;
+  const double r = dot(h.n, rel) + h.phi + cfm * h.l;
+  const double nl = smax(0.0, h.l + -h.og * r);
+  const double dl = nl - h.l;
+  if (dl != 0.0) {
+    h.l = nl;
+    const d3 ddx = h.n * (dl * h.im), ddt = h.In * dl;
+    slot_st(vs, side ? dx + ddx : dx - ddx, side ? dt + ddt : dt - ddt);
+  }
+  return fabs(dl);
+}
+
+struct PosRow : HalfPos {
+  int act;  // 1: the contact penetrates
+  __device__ void keep(double* o, int p) const { o[p] = l; }
+  __device__ void load(const RowIO& R, int p, int side) {
+    half_pos_load(R, p, side, *this);
+    act = og != 0.0;
+  }
+  __device__ void put(const RowIO& R, int p) const { R.lam[p] = l; }
+};
+template <bool ONE>
+__device__ __noinline__ int pos_sweep(const Sweep w, int C, PosRow& row, double cfm) {
+  PosRow h = row;
+  const int made = sweep_share<ONE>(w, C, h, [&](PosRow& r, double* vs, int side, bool, unsigned act) {
+    return pos_half(r, vs, side, act, r.act, cfm);
+  });
+  row.l = h.l;
+  return made;
+}
+__device__ __noinline__ int pos_sweep_rows(const Sweep w, int C, const RowIO R, double cfm) {
+  return sweep_rows<PosRow>(w, C, R, [&](PosRow& r, double* vs, int side, bool, unsigned act) {
+    return pos_half(r, vs, side, act, r.act, cfm);
+  });
+}
+
+// Position projection for C <= kSmallC (nsc_contact.cpp:698-879), split as
+// the velocity solve.
+__device__ __noinline__ bool small_project(const Team& team, const NscView& V, int C, unsigned& chunk) {
+  SmallSmem& S = small_smem();
+  if (solo(C, false) && team.rank() != 0) return true;
+  Team T = team;
+  if (solo(C, false)) T.nb = 1;
   const rg_config& cfg = V.cfg;
   const State& st = V.st;
-  const int t = threadIdx.x;
-  small_map(V, C, S);
-  int K = small_color(V, C, S);
+  const int t = threadIdx.x, pair = t >> 1, side = t & 1;
+  if (C == 0) return true;
+  small_map(V, C);
+  const int K = small_color(V, C, T.rank() == 0);
   if (K < 0) return false;
-  const double omega = cfg.nsc_omega, cfm = cfg.nsc_cfm, slop = cfg.nsc_slop;
-  double* PR = S.row;  // kPosComps x kSmallC
-  double* DX = S.vel;  // 6 x kSmallB: dx, dθ per local slot
-  const int p = t;
-  const int c = p < C ? S.order[p] : 0;
-  int my_color = -1;
-  if (p < C)
-    for (int k = 0; k < K; ++k)
-      if (p >= S.coff[k] && p < S.coff[k + 1]) my_color = k;
-  const int sa = p < C ? S.la[c] : 0, sb = p < C ? S.lb[c] : 0;
-  const int a = p < C ? V.con.a[c] : 0, b = p < C ? V.con.b[c] : 0;
-  for (int outer = 0; outer < cfg.nsc_position_iters; ++outer) {
-    int act = 0;
-    if (p < C) {
-      d3 xa = st.x.ld(a), xb = st.x.ld(b);
-      d3 nv, ra, rb;
-      double phi;
-      if (outer == 0) {
-        phi = V.con.comp(12)[c] - V.con.comp(13)[c];
-        nv = mk3(V.con.comp(6)[c], V.con.comp(7)[c], V.con.comp(8)[c]);
-        d3 pa{V.con.comp(0)[c], V.con.comp(1)[c], V.con.comp(2)[c]};
-        d3 pb{V.con.comp(3)[c], V.con.comp(4)[c], V.con.comp(5)[c]};
-        d3 sh{V.con.comp(9)[c], V.con.comp(10)[c], V.con.comp(11)[c]};
-        ra = pa - xa;
-        rb = pb - (xb + sh);
-      } else {
-        Seg A = make_seg(st, a), B = make_seg(st, b);
-        Narrow nr = narrow_pair(A, B, V.box);
-        d3 diff = nr.pb - nr.pa;
-        double dist = len(diff);
-        phi = dist - V.con.comp(13)[c];
-        nv = dist > 1e-10 ? diff / dist : mk3(1, 0, 0);
-        ra = nr.pa - xa;
-        rb = nr.pb - (xb + nr.sh);
-      }
-      act = phi < -slop ? 1 : 0;
-      if (act) {
-        PR[P_N * kSmallC + p] = nv.x; PR[(P_N + 1) * kSmallC + p] = nv.y; PR[(P_N + 2) * kSmallC + p] = nv.z;
-        PR[P_RA * kSmallC + p] = ra.x; PR[(P_RA + 1) * kSmallC + p] = ra.y; PR[(P_RA + 2) * kSmallC + p] = ra.z;
-        PR[P_RB * kSmallC + p] = rb.x; PR[(P_RB + 1) * kSmallC + p] = rb.y; PR[(P_RB + 2) * kSmallC + p] = rb.z;
-        PR[P_PHI * kSmallC + p] = phi + slop;
-        PR[P_G * kSmallC + p] = diag_of(st, a, b, ra, rb, nv, cfm);
-        PR[P_L * kSmallC + p] = 0.0;
-      }
+  const Share sh = small_split(T, C, K);
+  const int Cl = sh.count;
+  const double cfm = cfg.nsc_cfm;
+  const RowIO R{V.row + sh.base, V.lam + sh.base, V.ccap};
+  const int nt = (Cl + kPairs - 1) / kPairs;
+  // Positions over the passes: in shared memory (the network's space) when
+  // the share has one contact per lane pair, else in the state arrays.
+  double* pos = reinterpret_cast<double*>(S.wh);
+  static_assert(sizeof(S.wh) >= sizeof(double) * 7 * 2 * kPairs, "positions of a one-tier share");
+  const bool chip = nt <= 1;
+  auto side_of = [&](int p) {
+    const int c = S.order[p], bd = S.body[side ? S.pb[p] : S.pa[p]];
+    return PosSide{st.Iinv.ld(bd), st.inv_mass[bd], st.h[bd], V.con.comp(13)[c]};
+  };
+  PosSide mine = {};
+  const int own = pair < Cl ? pair : Cl - 1;  // (unused lanes follow the last contact)
+  if (Cl > 0 && chip) {
+    mine = side_of(own);
+    for (int s = t; s < S.nbody; s += blockDim.x) {
+      const int x = S.body[s];
+      const d3 p = st.x.ld(x);
+      const dq q = st.q.ld(x);
+      double* o = pos + 7 * s;
+      o[0] = p.x; o[1] = p.y; o[2] = p.z; o[3] = q.w; o[4] = q.x; o[5] = q.y; o[6] = q.z;
     }
-    for (int s = t; s < S.nloc; s += blockDim.x)
-      for (int k = 0; k < 6; ++k) DX[k * kSmallB + s] = 0.0;
-    int nact = __syncthreads_count(act);
-    if (nact == 0) break;  // nothing penetrates
-    for (int it = 0; it < cfg.nsc_position_psor_iters; ++it) {
-      double loc = 0.0;
-      for (int k = 0; k < K; ++k) {
-        if (my_color == k && act) {
-          d3 nv{PR[P_N * kSmallC + p], PR[(P_N + 1) * kSmallC + p], PR[(P_N + 2) * kSmallC + p]};
-          d3 ra{PR[P_RA * kSmallC + p], PR[(P_RA + 1) * kSmallC + p], PR[(P_RA + 2) * kSmallC + p]};
-          d3 rb{PR[P_RB * kSmallC + p], PR[(P_RB + 1) * kSmallC + p], PR[(P_RB + 2) * kSmallC + p]};
-          d3 dxa{DX[sa], DX[kSmallB + sa], DX[2 * kSmallB + sa]};
-          d3 dta{DX[3 * kSmallB + sa], DX[4 * kSmallB + sa], DX[5 * kSmallB + sa]};
-          d3 dxb{DX[sb], DX[kSmallB + sb], DX[2 * kSmallB + sb]};
-          d3 dtb{DX[3 * kSmallB + sb], DX[4 * kSmallB + sb], DX[5 * kSmallB + sb]};
-          double l = PR[P_L * kSmallC + p];
-          double corr = dot(nv, ((dxb + cross(dtb, rb)) - dxa) - cross(dta, ra));
-          double r = corr + PR[P_PHI * kSmallC + p] + cfm * l;
-          double d = -(omega / PR[P_G * kSmallC + p]) * r;
-          double nl = smax(0.0, l + d);
-          double dl = nl - l;
-          if (dl != 0.0) {
-            PR[P_L * kSmallC + p] = nl;
-            d3 rAxn = cross(ra, nv);
-            dxa = dxa - nv * (dl * st.inv_mass[a]);
-            dta = dta - iinv_apply(st, a, rAxn) * dl;
-            d3 rBxn = cross(rb, nv);
-            dxb = dxb + nv * (dl * st.inv_mass[b]);
-            dtb = dtb + iinv_apply(st, b, rBxn) * dl;
-            DX[sa] = dxa.x; DX[kSmallB + sa] = dxa.y; DX[2 * kSmallB + sa] = dxa.z;
-            DX[3 * kSmallB + sa] = dta.x; DX[4 * kSmallB + sa] = dta.y; DX[5 * kSmallB + sa] = dta.z;
-            DX[sb] = dxb.x; DX[kSmallB + sb] = dxb.y; DX[2 * kSmallB + sb] = dxb.z;
-            DX[3 * kSmallB + sb] = dtb.x; DX[4 * kSmallB + sb] = dtb.y; DX[5 * kSmallB + sb] = dtb.z;
-          }
-          loc = fabs(dl);
-        }
-        __syncthreads();
-      }
-      double res = small_block_max(loc, S);
-      if (res < 1e-8) break;
-    }
-    __syncthreads();
-    for (int s = t; s < S.nloc; s += blockDim.x) {
-      int x = S.body[s];
-      if (x < 0 || !S.dyn[s]) continue;
-      if (V.moved) V.moved[x] = 1;
-      st.x.st(x, st.x.ld(x) + mk3(DX[s], DX[kSmallB + s], DX[2 * kSmallB + s]));
-      d3 th{DX[3 * kSmallB + s], DX[4 * kSmallB + s], DX[5 * kSmallB + s]};
-      double ang = len(th);
-      if (ang > 1e-8) {
-        d3 ax = th / ang;
-        st.q.st(x, qnormalize(qmul(angle_axis(ang, ax), st.q.ld(x))));
-      }
-    }
-    __syncthreads();
   }
-  small_unmap(V, S);
+  bool moved = false;
+  __syncthreads();
+  for (int outer = 0; outer < cfg.nsc_position_iters; ++outer) {
+    int any = 0;
+    PosRow row = {};
+#pragma unroll 1
+    for (int j = 0; j < nt; ++j) {
+      if (j * kPairs + (t >> 5) * 16 >= Cl) continue;  // no contact in this warp
+      const int p = j * kPairs + pair;
+      const bool valid = p < Cl;
+      if (chip) {
+        const double* o = pos + 7 * (side ? S.pb[own] : S.pa[own]);
+        row.act = build_half_pos(V, mk3(o[0], o[1], o[2]), dq{o[3], o[4], o[5], o[6]}, mine, side, row);
+      } else {
+        const int pc = valid ? p : Cl - 1, bd = S.body[side ? S.pb[pc] : S.pa[pc]];
+        const PosSide b = side_of(pc);
+        row.act = build_half_pos(V, st.x.ld(bd), st.q.ld(bd), b, side, row);
+      }
+      if (!valid) continue;
+      any |= row.act;
+      if (!row.act) row.og = 0.0;
+      if (nt > 1) half_pos_store(R, p, side, row);
+    }
+    for (int s = t; s < 6 * S.nbody; s += blockDim.x) S.vel[s] = 0.0;
+    any = __syncthreads_or(any);
+    if (T.nb == 1 && !any) break;  // nothing penetrates
+    Share act = sh;
+    if (!any) act.count = 0;  // nothing of this share moves, now or in a later pass
+    double res;
+    int its = 0;
+    // a team's blocks learn whether anything penetrates from the first
+    // sweep's residual: it is above zero exactly when something does.  Most
+    // passes stop after one or two sweeps.
+    const bool ok = sweep_until(
+        T, act, 1, cfg.nsc_position_psor_iters, 1e-8, 2, chunk,
+        [&](const Sweep& w) {
+          if (nt > 1) return pos_sweep_rows(w, Cl, R, cfm);
+          return Cl <= 16 ? pos_sweep<true>(w, Cl, row, cfm) : pos_sweep<false>(w, Cl, row, cfm);
+        },
+        [&](const double* o) {
+          if (pair < Cl) row.l = o[pair];
+        },
+        res, its);
+    if (!ok) return false;
+    if (any) {
+      moved = true;
+      for (int s = t; s < S.nbody; s += blockDim.x) {
+        if (!S.dyn[s]) continue;
+        const int x = S.body[s];
+        double* o = pos + 7 * s;
+        d3 dx, th;
+        slot_ld(&S.vel[6 * s], dx, th);
+        d3 p = chip ? mk3(o[0], o[1], o[2]) : st.x.ld(x);
+        dq q = chip ? dq{o[3], o[4], o[5], o[6]} : st.q.ld(x);
+        p = p + dx;
+        const double ang = len(th);
+        if (ang > 1e-8) {
+          const d3 ax = th / ang;
+          q = qnormalize(qmul(angle_axis(ang, ax), q));
+        }
+        if (chip) {
+          o[0] = p.x; o[1] = p.y; o[2] = p.z; o[3] = q.w; o[4] = q.x; o[5] = q.y; o[6] = q.z;
+        } else {
+          st.x.st(x, p);
+          st.q.st(x, q);
+        }
+      }
+    }
+    __syncthreads();
+    if (T.nb > 1 && its == 1 && res == 0.0) break;  // nothing penetrated anywhere
+  }
+  if (moved)
+    for (int s = t; s < S.nbody; s += blockDim.x) {
+      if (!S.dyn[s]) continue;
+      const int x = S.body[s];
+      if (V.moved) V.moved[x] = 1;
+      if (!chip) continue;
+      const double* o = pos + 7 * s;
+      st.x.st(x, mk3(o[0], o[1], o[2]));
+      st.q.st(x, dq{o[3], o[4], o[5], o[6]});
+    }
   return true;
 }
 
@@ -1326,7 +2081,8 @@ __device__ __noinline__ int wall_phase(const Team& T, const NscView& V, int Cp, 
 // ---------------------------------------------------------------------------
 // One NSC step of one system by one team.
 // ---------------------------------------------------------------------------
-__device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, SmallSmem& S, bool first) {
+__device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, unsigned& chunk, bool first) {
+  SmallSmem& S = small_smem();
   Ctl* ctl = V.ctl;
   const State& st = V.st;
   const rg_config& cfg = V.cfg;
@@ -1380,12 +2136,10 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, SmallSmem
   pc.mark(1);
   const bool small = C <= kSmallC;
   if (small) {
-    // colouring, rows, PSOR and warm cache in one block, on chip
-    bool ok = true;
+    // colouring, rows, PSOR and warm cache on chip
     const unsigned long long ts = (rank == 0 && threadIdx.x == 0) ? gtimer() : 0ull;
-    if (rank == 0) ok = small_solve(V, C, Cp, S, pc);
+    if (!small_solve(T, V, C, Cp, chunk, pc)) return false;
     if (rank == 0 && threadIdx.x == 0) ctl->serial_ns += (long long)(gtimer() - ts);
-    if (!ok) atomicOr(&ctl->err, ERR_COLOR);
     pc.mark(10);
     if (!team_sync(T)) return false;
     pc.mark(11);
@@ -1426,10 +2180,10 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, SmallSmem
         // each warp of the team evaluates tiles of 16 slots on the tensor
         // cores; its own lanes then apply the tile's predictions.  Every
         // block stages the whole network in its (here unused) small-solve
-        // shared memory: W1, W4 and the small parameters in pmax/cmask, W2
-        // in wh, W3 over the rows.
-        const MlpStage ms = mlp_stage_at(S.pmax);
-        __nv_bfloat16* w3s = reinterpret_cast<__nv_bfloat16*>(S.row);
+        // shared memory: W1, W4 and the small parameters in stage, W2 in wh,
+        // W3 in the space of the velocities.
+        const MlpStage ms = mlp_stage_at(S.stage);
+        __nv_bfloat16* w3s = reinterpret_cast<__nv_bfloat16*>(S.vel);
         stage_small(ms, V.mlp);
         stage_bf16(S.wh, kWhLd, V.mlp.w2, kMlpH, kMlpH);
         stage_bf16(w3s, kWhLd, V.mlp.w3, kMlpH, kMlpH);
@@ -1449,7 +2203,8 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, SmallSmem
           hidden_layer(a, w3s, kWhLd, q.b3, lane);
           mlp_layer4(a, ms.w4, kWhLd, q, V.pred, V.ccap, row0, C, lane);
           __syncwarp();
-          if (want) mlp_apply(R, V.pred, V.ccap, p, cfg.nsc_mu);
+          if (want)
+            mlp_apply(R.lam[p], R.lam[R.ccap + p], R.lam[2 * (size_t)R.ccap + p], V.pred, V.ccap, p, cfg.nsc_mu);
           __syncwarp();
         }
       }
@@ -1536,11 +2291,9 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, SmallSmem
     if (C2 < 0) return false;
     pc.mark(6);
     if (C2 <= kSmallC) {
-      bool ok = true;
       const unsigned long long ts = (rank == 0 && threadIdx.x == 0) ? gtimer() : 0ull;
-      if (rank == 0) ok = small_project(V, C2, S);
+      if (!small_project(T, V, C2, chunk)) return false;
       if (rank == 0 && threadIdx.x == 0) ctl->serial_ns += (long long)(gtimer() - ts);
-      if (!ok) atomicOr(&ctl->err, ERR_COLOR);
       if (!team_sync(T)) return false;
     } else {
       if (!color_phase(T, V, C2, sm)) return false;
@@ -1560,11 +2313,6 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, SmallSmem
   return true;
 }
 
-#ifndef RG_NSC_BLOCK
-#define RG_NSC_BLOCK (2 * kTile)
-#endif
-constexpr int kBlock = RG_NSC_BLOCK;  // threads per block of the persistent step
-
 // Each block finds its team (teams are sorted by b0), then runs nsteps steps
 // of the team's systems, one system after the other within a step.  A
 // system whose step failed (error bits set) returns at once from its later
@@ -1575,8 +2323,6 @@ constexpr int kBlock = RG_NSC_BLOCK;  // threads per block of the persistent ste
 __global__ void __launch_bounds__(kBlock, RG_NSC_MIN_BLOCKS) k_nsc_run(const NscView* views, const TeamDesc* teams, int nteams,
                                                    const int* members, int nsteps) {
   __shared__ SmemNsc sm;
-  extern __shared__ __align__(16) unsigned char dyn_smem[];
-  SmallSmem& S = *reinterpret_cast<SmallSmem*>(dyn_smem);
   int lo = 0, hi = nteams;  // last team with b0 <= blockIdx.x
   while (hi - lo > 1) {
     int m = (lo + hi) >> 1;
@@ -1587,16 +2333,29 @@ __global__ void __launch_bounds__(kBlock, RG_NSC_MIN_BLOCKS) k_nsc_run(const Nsc
   if ((int)blockIdx.x < td.b0 || (int)blockIdx.x >= td.b0 + td.nb) return;
   const bool team_timer = td.t_ns && threadIdx.x == 0 && (int)blockIdx.x == td.b0;
   const unsigned long long t_start = team_timer ? gtimer() : 0ull;
+  // The view is read in every phase, right after a barrier whose acquire has
+  // emptied the L1 cache: from shared memory a field costs 30 cycles instead
+  // of an L2 round trip in front of the load that needs it.
+  __shared__ __align__(16) unsigned char view_words[sizeof(NscView)];
+  const NscView& V = *reinterpret_cast<const NscView*>(view_words);
+  unsigned chunk = 0;  // chunks of the split solve so far (all blocks of a team count alike)
   for (int s = 0; s < nsteps; ++s) {
     bool any = false;
     for (int m = td.first; m < td.first + td.count; ++m) {
-      const NscView& V = views[members ? members[m] : m];
+      if (s == 0 || td.count > 1) {
+        static_assert(sizeof(NscView) % 8 == 0, "copied in 8-byte words");
+        const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&views[members ? members[m] : m]);
+        __syncthreads();  // the member before is done with its view
+        for (int k = threadIdx.x; k < (int)(sizeof(NscView) / 8); k += blockDim.x)
+          reinterpret_cast<unsigned long long*>(view_words)[k] = src[k];
+        __syncthreads();
+      }
       Team T{td.b0, td.nb, td.bar, &V.ctl->err,
              V.cfg.spin_limit > 0 ? (long long)V.cfg.spin_limit : kSpinLimit,
              V.cfg.test_absent_blocks > 0 ? (unsigned)V.cfg.test_absent_blocks : 0u};
       const bool timer = threadIdx.x == 0 && (int)blockIdx.x == td.b0;
       const unsigned long long t0 = timer ? gtimer() : 0ull;
-      any |= nsc_step(T, V, sm, S, s == 0);
+      any |= nsc_step(T, V, sm, chunk, s == 0);
       if (timer) V.ctl->member_ns += (long long)(gtimer() - t0);  // one writer per system
     }
     if (!any) break;
@@ -1632,7 +2391,6 @@ NscView make_view(rg_system* s) {
   V.dx = N.dx; V.prow = N.prow; V.pactive = N.pactive;
   V.ccap = s->ccap;
   V.blk = N.blk;
-  V.slot_of = N.slot_of;
   V.near = d.near;
   V.ref2 = d.ref2;
   V.moved = d.moved;
@@ -1680,7 +2438,7 @@ void nsc_run_launch(rg_system* s, int nsteps) {
   TeamDesc td{0, nb, 0, 1, s->nsc.bar};
   cudaMemcpyAsync(s->nsc.view_dev, &V, sizeof(NscView), cudaMemcpyHostToDevice, s->stream);
   cudaMemcpyAsync(s->nsc.team_dev, &td, sizeof(TeamDesc), cudaMemcpyHostToDevice, s->stream);
-  cudaMemsetAsync(s->nsc.bar, 0, 4 * sizeof(unsigned int), s->stream);
+  cudaMemsetAsync(s->nsc.bar, 0, kTeamBarBytes, s->stream);
   const NscView* views = reinterpret_cast<const NscView*>(s->nsc.view_dev);
   const TeamDesc* teams = reinterpret_cast<const TeamDesc*>(s->nsc.team_dev);
   int nteams = 1;

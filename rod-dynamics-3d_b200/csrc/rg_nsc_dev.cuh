@@ -193,16 +193,14 @@ __device__ inline void export_row(double* xrow, int wcap, int c, const RowIO& R,
   for (int k = 0; k < kExportComps; ++k) xrow[(size_t)k * wcap + c] = R.r(src[k], p);
 }
 
-// Learned warm start of slot p: previous impulse (already in R.lam) plus the
-// network's predicted change, projected onto the friction cone.
-__device__ inline void mlp_apply(const RowIO& R, const float* pred, int pld, int p, double mu) {
-  double ln = R.lam[p] + (double)pred[p];
-  double l1 = R.lam[R.ccap + p] + (double)pred[pld + p];
-  double l2 = R.lam[2 * R.ccap + p] + (double)pred[2 * pld + p];
-  cone_clamp(ln, l1, l2, mu);
-  R.lam[p] = ln;
-  R.lam[R.ccap + p] = l1;
-  R.lam[2 * R.ccap + p] = l2;
+// Learned warm start of slot p: previous impulse plus the network's predicted
+// change, projected onto the friction cone.
+__device__ inline void mlp_apply(double& l0, double& l1, double& l2, const float* pred, int pld, int p, double mu) {
+  double n = l0 + (double)pred[p], t1 = l1 + (double)pred[pld + p], t2 = l2 + (double)pred[2 * (size_t)pld + p];
+  cone_clamp(n, t1, t2, mu);
+  l0 = n;
+  l1 = t1;
+  l2 = t2;
 }
 
 struct Vel {
@@ -524,7 +522,6 @@ struct NscView {
   int* pactive;
   int ccap;
   int* blk;      // per-block scratch of the team
-  int* slot_of;  // per-body local slot of the in-block solver (-1 when unused)
   int2* near;    // near list (see Detector); null: test the whole lists
   double* ref2;
   unsigned char* moved;  // see Detector
@@ -546,7 +543,7 @@ struct NscView {
 // several blocks runs exactly one system.
 struct TeamDesc {
   int b0, nb, first, count;
-  unsigned int* bar;  // 4 words: full-team count/gen, subset count/gen
+  unsigned int* bar;  // kTeamBarBytes: full-team count/gen, subset count/gen, residual ring
   long long* t_ns;    // optional: the team's device time for the launch
 };
 
