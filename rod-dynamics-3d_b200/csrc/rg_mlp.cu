@@ -644,7 +644,9 @@ size_t rg_mlp_param_count(void) { return (size_t)kMlpParams; }
 int rg_mlp_set_params(rg_system* s, const float* params, size_t n) {
   if (!s || !params || n != (size_t)kMlpParams) return RG_ERR_ARG;
   if (ensure_net(s)) return RG_ERR_CUDA;
-  cudaMemcpy(host_of(s).P, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice);
+  // on the system's stream: a default-stream copy from pageable memory may
+  // still be on its way when the conversion starts on the non-blocking stream
+  cudaMemcpyAsync(host_of(s).P, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice, s->stream);
   refresh_bf16(s);
   if (cudaStreamSynchronize(s->stream)) return RG_ERR_CUDA;
   s->mlp_ready = true;
@@ -695,8 +697,8 @@ int rg_mlp_grad(rg_system* s, const float* features, const float* targets, size_
   if (ensure_workspace(s)) return RG_ERR_CUDA;
   float *df = nullptr, *dt = nullptr;
   if (cudaMalloc(&df, sizeof(float) * kMlpIn * n) || cudaMalloc(&dt, sizeof(float) * kMlpOut * n)) return RG_ERR_CUDA;
-  cudaMemcpy(df, features, sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(dt, targets, sizeof(float) * kMlpOut * n, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(df, features, sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(dt, targets, sizeof(float) * kMlpOut * n, cudaMemcpyHostToDevice, s->stream);
   const int nblk = forward_backward(s, df, dt, nullptr, (int)n);
   cudaMemsetAsync(H.G, 0, sizeof(float) * kMlpParams, s->stream);
   RGL k_mlp_grad_sum<<<grid_for(kGradParams, 256), 256, 0, s->stream>>>(H.part, nblk, H.G);
@@ -715,7 +717,7 @@ int rg_mlp_train(rg_system* s, const float* features, const float* targets, size
   MlpHost& H = host_of(s);
   std::vector<float> P;
   init_params(P, features, targets, n, seed);
-  cudaMemcpy(H.P, P.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(H.P, P.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice, s->stream);
   refresh_bf16(s);
   if (batch > (int)n) batch = (int)n;
   if (ensure_workspace(s)) return RG_ERR_CUDA;
@@ -726,10 +728,10 @@ int rg_mlp_train(rg_system* s, const float* features, const float* targets, size
       return RG_ERR_CUDA;
     H.nfeat = n;
   }
-  cudaMemcpy(H.feat, features, sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(H.tgt, targets, sizeof(float) * kMlpOut * n, cudaMemcpyHostToDevice);
-  cudaMemset(H.Am, 0, sizeof(float) * kMlpParams);
-  cudaMemset(H.Av, 0, sizeof(float) * kMlpParams);
+  cudaMemcpyAsync(H.feat, features, sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(H.tgt, targets, sizeof(float) * kMlpOut * n, cudaMemcpyHostToDevice, s->stream);
+  cudaMemsetAsync(H.Am, 0, sizeof(float) * kMlpParams, s->stream);
+  cudaMemsetAsync(H.Av, 0, sizeof(float) * kMlpParams, s->stream);
   if (H.nidx < n) {
     cudaFree(H.idx);
     if (cudaMalloc(&H.idx, sizeof(int) * n)) return RG_ERR_CUDA;
@@ -776,7 +778,7 @@ int rg_mlp_infer(rg_system* s, const float* features, float* out, size_t n) {
   std::vector<float> t(kMlpIn * n);
   for (size_t i = 0; i < n; ++i)
     for (int k = 0; k < kMlpIn; ++k) t[(size_t)k * n + i] = features[i * kMlpIn + k];
-  cudaMemcpy(fT, t.data(), sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice);
+  cudaMemcpyAsync(fT, t.data(), sizeof(float) * kMlpIn * n, cudaMemcpyHostToDevice, s->stream);
   int warps = (int)((n + 15) / 16);
   RGL k_mlp_infer<<<(warps + 7) / 8, 256, 0, s->stream>>>(mlp_dev(s), fT, (int)n, oT);
   std::vector<float> o(kMlpOut * n);
