@@ -89,6 +89,7 @@ void free_contact_buffers(rg_system* s) {
   cudaFree(s->d_cf);
   s->d_cf = nullptr;
   s->scan.free_();
+  s->vteam.free_();
   cudaFree(s->d_feat); cudaFree(s->d_pred);
   s->d_feat = nullptr; s->d_pred = nullptr;
 }
@@ -147,6 +148,9 @@ cudaError_t alloc_contact_buffers(rg_system* s, int ccap, int hcap) {
   if ((e = cudaMalloc(&s->d_cf, sizeof(double) * (13 * (size_t)ccap + 64)))) return e;
   if ((e = cudaMalloc(&s->d_feat, sizeof(float) * 8 * (size_t)ccap))) return e;
   if ((e = cudaMalloc(&s->d_pred, sizeof(float) * 3 * (size_t)ccap))) return e;
+  if ((s->cfg.model == RG_MODEL_HARMONIC || s->cfg.model == RG_MODEL_HERTZ_MINDLIN) && n <= kVerletTeamRods &&
+      (e = s->vteam.alloc(n, ccap)))
+    return e;
   int scap = ccap + 1;
   if (hcap + 1 > scap) scap = hcap + 1;
   if (n + 1 > scap) scap = n + 1;
@@ -312,6 +316,7 @@ __global__ void k_ctl_reset(Ctl* const* ctls, int n) {
     c->serial_ns = 0;
     c->det_valid = 0;
     c->bar_count = 0;
+    c->ins_n[0] = c->ins_n[1] = 0;
   }
 }
 
@@ -507,7 +512,7 @@ int rg_set_bodies(rg_system* s, const double* radius, const double* half_height,
   force_rebuild(s);
   RG_TRY(cudaStreamSynchronize(s->stream), "set_bodies sync");
   s->bodies_set = true;
-  s->contacts_fresh = false;
+  s->contacts_fresh = Fresh::kNo;
   return RG_OK;
 }
 
@@ -538,7 +543,7 @@ int rg_set_state(rg_system* s, const double* x, const double* q, const double* v
                          s->stream), "upload state");
   RG_TRY(cudaStreamSynchronize(s->stream), "set_state sync");
   s->state_set = true;
-  s->contacts_fresh = false;
+  s->contacts_fresh = Fresh::kNo;
   return RG_OK;
 }
 
@@ -575,9 +580,9 @@ namespace rg {
 // evaluation); the per-body sums are fused into the two kick kernels.
 static void verlet_step(rg_system* s) {
   force_eval_launch(s, EvalTail::kHalfPos);  // forces at t (reuses fresh contacts), kick and drift
-  s->contacts_fresh = false;
+  s->contacts_fresh = Fresh::kNo;
   force_eval_launch(s, EvalTail::kSecondHalf, true);  // forces at t + dt, second kick
-  s->contacts_fresh = true;  // positions unchanged until the next drift
+  s->contacts_fresh = Fresh::kCsr;  // positions unchanged until the next drift
 }
 
 // Captures one Verlet step (entered with fresh contacts) as a CUDA graph.
@@ -602,7 +607,7 @@ static bool capture_verlet_step(rg_system* s) {
   g_launches = l0;  // counted when the graph runs
   if (e == cudaSuccess) e = cudaGraphInstantiate(&s->vgraph, g, 0);
   if (g) cudaGraphDestroy(g);
-  if (e != cudaSuccess || s->hist.cur != cur || !s->contacts_fresh) {
+  if (e != cudaSuccess || s->hist.cur != cur || s->contacts_fresh != Fresh::kCsr) {
     cudaGetLastError();
     if (s->vgraph) cudaGraphExecDestroy(s->vgraph);
     s->vgraph = nullptr;
@@ -621,8 +626,12 @@ void launch_steps(rg_system* s, int nsteps) {
     return;
   }
   if (model != RG_MODEL_HARMONIC && model != RG_MODEL_HERTZ_MINDLIN) return;
+  if (verlet_team_fits(s)) {  // one persistent launch for all steps
+    if (nsteps > 0) verlet_run_launch(s, nsteps);
+    return;
+  }
   int k = 0;
-  if (nsteps > 0 && !s->contacts_fresh) {  // the first evaluation detects
+  if (nsteps > 0 && s->contacts_fresh != Fresh::kCsr) {  // the first evaluation detects
     verlet_step(s);
     k = 1;
   }
@@ -714,6 +723,7 @@ cudaError_t reset_call_ctl(rg_system* s, const Snapshot& sn) {
   h->serial_ns = 0;
   h->det_valid = 0;
   h->bar_count = 0;
+  h->ins_n[0] = h->ins_n[1] = 0;
   return cudaMemcpyAsync(s->d_ctl, h, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream);
 }
 
@@ -730,7 +740,7 @@ int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   if (err & (ERR_TIMEOUT | ERR_NONFINITE | ERR_COLOR)) {
     std::memcpy(s->h_ctl, sn.ctl.data(), s->ctl_bytes);
     reinterpret_cast<Ctl*>(s->h_ctl)->rebuild = 1;
-    s->contacts_fresh = false;
+    s->contacts_fresh = Fresh::kNo;
     e = cudaMemcpyAsync(s->d_ctl, s->h_ctl, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream);
     if (!e) e = cudaStreamSynchronize(s->stream);
     if (e) return cuda_fail(s, e, "restore control words");
@@ -742,7 +752,7 @@ int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   e = take_snapshot(s, sn);
   if (e) return cuda_fail(s, e, "snapshot");
   reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
-  s->contacts_fresh = false;
+  s->contacts_fresh = Fresh::kNo;
   *retry = true;
   return RG_OK;
 }
@@ -835,7 +845,7 @@ int rg_detect(rg_system* s, double delta, int32_t* pairs, double* geom, double* 
     if (!grow(s, h->err)) return fail(s, RG_ERR_CAPACITY, "could not grow device buffers");
     force_rebuild(s);
   }
-  s->contacts_fresh = false;  // the force path must rebuild its CSR
+  s->contacts_fresh = Fresh::kNo;  // the force path must rebuild its CSR
   const int C = s->h_ctl->contacts;
   if (C < 0 || C > s->ccap) return fail(s, RG_ERR_CAPACITY, "contact count exceeds the contact buffer");
   *n = (size_t)C;
@@ -967,7 +977,7 @@ int rg_compute_forces(rg_system* s, double* f, double* tau, double* pe) {
     h->err = 0;
     RG_TRY(cudaMemcpyAsync(s->d_ctl, h, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream), "ctl");
     clear_forces_launch(s);
-    s->contacts_fresh = false;
+    s->contacts_fresh = Fresh::kNo;
     force_eval_launch(s);
     RG_TRY(cudaGetLastError(), "force launch");
     RG_TRY(cudaMemcpyAsync(h, s->d_ctl, s->ctl_bytes, cudaMemcpyDeviceToHost, s->stream), "ctl");
@@ -983,7 +993,7 @@ int rg_compute_forces(rg_system* s, double* f, double* tau, double* pe) {
     RG_TRY(take_snapshot(s, sn), "snapshot");
     reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
   }
-  s->contacts_fresh = true;
+  s->contacts_fresh = Fresh::kCsr;
   if (pe) *pe = s->h_ctl->pe;
   return rg_get_state(s, nullptr, nullptr, nullptr, nullptr, f, tau);
 }

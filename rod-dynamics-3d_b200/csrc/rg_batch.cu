@@ -8,8 +8,9 @@
 // error words) on one shared stream.  NSC members run as teams of the
 // persistent step kernel in ONE cooperative launch for all requested
 // steps; that launch (with the reset of the team barriers) is captured in a
-// CUDA graph and replayed.  Members with the Verlet models run their
-// multi-kernel step on the same stream after it.
+// CUDA graph and replayed.  Members with the Verlet models run as teams of
+// one launch of the persistent Verlet kernel after it (those too large for
+// that form one after the other).
 //
 // Schedule: each member's work is its rod count until the device has timed
 // its steps (every call records each member's own step time), then that
@@ -32,7 +33,7 @@
 #include <vector>
 
 #include "rg_internal.cuh"
-#include "rg_nsc_dev.cuh"
+#include "rg_verlet_dev.cuh"
 
 using namespace rg;
 
@@ -81,6 +82,11 @@ struct rg_batch {
   unsigned char* h_ctlbuf = nullptr;
   std::vector<size_t> ctl_off;
   size_t ctlbuf_bytes = 0;
+  // persistent Verlet launch: views, teams, member order, barrier words
+  VerletView* d_vviews = nullptr;
+  TeamDesc* d_vteams = nullptr;
+  int* d_vmembers = nullptr;
+  unsigned int* d_vbars = nullptr;
   // bulk state transfer: member table and device staging (x, q, v, w)
   void* d_bulk = nullptr;
   double* d_stage = nullptr;
@@ -375,6 +381,7 @@ cudaError_t ensure_dev(rg_batch* b, size_t nteams, size_t nmembers) {
 // Uploads the views of all members (buffer addresses change when buffers
 // grow) and the team plan.  The views array is indexed by member number.
 cudaError_t upload(rg_batch* b, std::vector<TeamDesc>& teams, const std::vector<int>& members) {
+  if (members.empty()) return cudaSuccess;  // no NSC member
   const int cm = b->cap_members, ct = b->cap_teams;
   cudaError_t e = ensure_dev(b, teams.size(), members.size());
   if (e) return e;
@@ -436,6 +443,75 @@ cudaError_t launch_nsc(rg_batch* b, int nteams, int grid, int nsteps, bool graph
     b->graph_steps = nsteps;
   }
   RGL cudaGraphLaunch(b->graph, b->stream);
+  return cudaGetLastError();
+}
+
+// Teams of the Verlet members `which`: every member a block, the others dealt
+// out by rod count, at most one block per kVerletRodsPerBlock rods; with more
+// members than blocks, single-block teams packed longest-first.  (A step's
+// time is its phases' latency plus the rods per block, so rod counts divide
+// the blocks well enough without timed costs.)
+void plan_verlet(const rg_batch* b, const std::vector<int>& which, std::vector<TeamDesc>& teams,
+                 std::vector<int>& members, int& grid) {
+  const int budget = b->sys[0]->sm_count, m = (int)which.size();
+  grid = 0;
+  if (m <= budget) {
+    double total = 0.0;
+    for (int k : which) total += b->sys[k]->n;
+    for (int i = 0; i < m; ++i) {
+      const int n = b->sys[which[i]]->n;
+      const int share = 1 + (int)((budget - m) * (n / total));
+      const int nb = std::min(share, (n + kVerletRodsPerBlock - 1) / kVerletRodsPerBlock);
+      teams.push_back(TeamDesc{grid, nb, i, 1, nullptr, nullptr});
+      members.push_back(i);
+      grid += nb;
+    }
+    return;
+  }
+  std::vector<int> order(m);
+  std::iota(order.begin(), order.end(), 0);
+  std::vector<double> w(m);
+  for (int i = 0; i < m; ++i) w[i] = b->sys[which[i]]->n;
+  std::sort(order.begin(), order.end(), [&](int x, int y) { return w[x] != w[y] ? w[x] > w[y] : x < y; });
+  std::vector<std::vector<int>> bins;
+  pack_lpt(order, w, budget, bins);
+  for (const std::vector<int>& bin : bins) {
+    teams.push_back(TeamDesc{grid++, 1, (int)members.size(), (int)bin.size(), nullptr, nullptr});
+    members.insert(members.end(), bin.begin(), bin.end());
+  }
+}
+
+// nsteps steps of the members in `todo` that run a Verlet model.
+cudaError_t launch_verlet(rg_batch* b, const std::vector<int>& todo, int nsteps) {
+  if (nsteps <= 0) return cudaSuccess;
+  std::vector<int> which;
+  for (int k : todo) {
+    rg_system* s = b->sys[k];
+    if (s->cfg.model == RG_MODEL_NSC) continue;
+    if (verlet_team_fits(s)) which.push_back(k);
+    else launch_steps(s, nsteps);
+  }
+  if (which.empty()) return cudaGetLastError();
+  cudaError_t e;
+  if (!b->d_vviews) {
+    const int bars = std::max(b->n, b->sys[0]->sm_count);
+    if ((e = cudaMalloc(&b->d_vviews, sizeof(VerletView) * b->n)) || (e = cudaMalloc(&b->d_vmembers, sizeof(int) * b->n)) ||
+        (e = cudaMalloc(&b->d_vteams, sizeof(TeamDesc) * bars)) || (e = cudaMalloc(&b->d_vbars, kTeamBarBytes * bars)))
+      return e;
+  }
+  std::vector<TeamDesc> teams;
+  std::vector<int> members;
+  int grid = 0;
+  plan_verlet(b, which, teams, members, grid);
+  std::vector<VerletView> views;
+  for (int k : which) views.push_back(make_verlet_view(b->sys[k]));
+  for (size_t t = 0; t < teams.size(); ++t) teams[t].bar = b->d_vbars + kTeamBarBytes / sizeof(unsigned int) * t;
+  cudaMemcpyAsync(b->d_vviews, views.data(), sizeof(VerletView) * views.size(), cudaMemcpyHostToDevice, b->stream);
+  cudaMemcpyAsync(b->d_vteams, teams.data(), sizeof(TeamDesc) * teams.size(), cudaMemcpyHostToDevice, b->stream);
+  cudaMemcpyAsync(b->d_vmembers, members.data(), sizeof(int) * members.size(), cudaMemcpyHostToDevice, b->stream);
+  cudaMemsetAsync(b->d_vbars, 0, kTeamBarBytes * teams.size(), b->stream);
+  verlet_launch(b->d_vviews, b->d_vteams, (int)teams.size(), b->d_vmembers, grid, nsteps, b->stream);
+  for (int k : which) verlet_launched(b->sys[k], nsteps);
   return cudaGetLastError();
 }
 
@@ -569,16 +645,16 @@ int batch_call(rg_batch* b, int nsteps, rg_step_stats* per, bool restore_after =
     if (warm_steps > 0) {  // untimed lead-in (autotuner trials)
       cudaError_t ew = launch_nsc(b, (int)teams.size(), grid, warm_steps, false);
       if (ew) return bfail(b, RG_ERR_CUDA, std::string("persistent launch: ") + cudaGetErrorString(ew));
-      for (int k : todo)
-        if (b->sys[k]->cfg.model != RG_MODEL_NSC) launch_steps(b->sys[k], warm_steps);
+      if ((ew = launch_verlet(b, todo, warm_steps)))
+        return bfail(b, RG_ERR_CUDA, std::string("Verlet launch: ") + cudaGetErrorString(ew));
       ctl_zero_time_launch(b->d_ctls, b->n, b->stream);  // costs count the timed steps only
     }
     const long long l0 = g_launches;
     cudaEventRecord(b->ev0, b->stream);
     cudaError_t e = launch_nsc(b, (int)teams.size(), grid, nsteps, full);
     if (e) return bfail(b, RG_ERR_CUDA, std::string("persistent launch: ") + cudaGetErrorString(e));
-    for (int k : todo)
-      if (b->sys[k]->cfg.model != RG_MODEL_NSC) launch_steps(b->sys[k], nsteps);
+    if ((e = launch_verlet(b, todo, nsteps)))
+      return bfail(b, RG_ERR_CUDA, std::string("Verlet launch: ") + cudaGetErrorString(e));
     cudaEventRecord(b->ev1, b->stream);
     if ((e = cudaGetLastError())) return bfail(b, RG_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     if (read_ctls(b, todo) != RG_OK) return RG_ERR_CUDA;
@@ -633,7 +709,7 @@ int batch_call(rg_batch* b, int nsteps, rg_step_stats* per, bool restore_after =
       const int one = 1;
       if (restore_snapshot(s, sn[k]) || cudaMemcpy(&s->d_ctl->rebuild, &one, sizeof(int), cudaMemcpyHostToDevice))
         return bfail(b, RG_ERR_CUDA, "restore");
-      s->contacts_fresh = false;
+      s->contacts_fresh = Fresh::kNo;
     }
     return RG_OK;
   }
@@ -692,6 +768,7 @@ int rg_batch_destroy(rg_batch* b) {
     rg_destroy(s);
   }
   cudaFree(b->d_views); cudaFree(b->d_teams); cudaFree(b->d_members); cudaFree(b->d_bars); cudaFree(b->d_team_ns);
+  cudaFree(b->d_vviews); cudaFree(b->d_vteams); cudaFree(b->d_vmembers); cudaFree(b->d_vbars);
   cudaFree(b->d_bulk); cudaFree(b->d_stage); cudaFree(b->d_bulk_bad);
   if (b->h_bulk_bad) cudaFreeHost(b->h_bulk_bad);
   cudaFree(b->d_segs); cudaFree(b->d_ctls); cudaFree(b->d_ctlbuf);
@@ -779,7 +856,7 @@ int rg_batch_set_state_all(rg_batch* b, const double* x, const double* q, const 
   if (*b->h_bulk_bad) return bfail(b, RG_ERR_NONFINITE, "non-finite component in the uploaded states (nothing changed)");
   for (rg_system* s : b->sys) {
     s->state_set = true;
-    s->contacts_fresh = false;
+    s->contacts_fresh = Fresh::kNo;
   }
   return RG_OK;
 }

@@ -16,7 +16,7 @@
 // Forces are reduced per body in contact order through a body->contact CSR,
 // which makes the sums deterministic and equal in order to the reference's
 // sequential accumulation.
-#include "rg_internal.cuh"
+#include "rg_verlet_dev.cuh"
 
 namespace rg {
 
@@ -86,19 +86,6 @@ void csr_launch(rg_system* s, bool counted) {
 // ---------------------------------------------------------------------------
 // History lookup / merge.
 // ---------------------------------------------------------------------------
-__device__ inline unsigned long long pkey(int a, int b) {
-  return ((unsigned long long)(unsigned)a << 32) | (unsigned long long)(unsigned)b;
-}
-__device__ inline int lower_bound_u64(const unsigned long long* k, int n, unsigned long long v) {
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    int m = (lo + hi) >> 1;
-    if (k[m] < v) lo = m + 1;
-    else hi = m;
-  }
-  return lo;
-}
-
 // kept[e]: entries retained if untouched (HM: 4-frame retention; Cundall:
 // all); the force kernel that follows clears the touched ones.  fr is the
 // frame this evaluation opens (the force kernel advances ctl->frame).
@@ -197,12 +184,14 @@ __device__ inline d3 ldc(const ForceIO& io, int k, int c) {
   return {io.g[(size_t)k * io.ccap + c], io.g[(size_t)(k + 1) * io.ccap + c],
           io.g[(size_t)(k + 2) * io.ccap + c]};
 }
-__device__ inline void st_cf(const ForceIO& io, int c, d3 fa, d3 ta, d3 fb, d3 tb) {
+// Outputs of contact c (hf: its table entry, or -1).
+__device__ inline void st_pair(const ForceIO& io, int c, int hf, const PairForce& p) {
   const int cc = io.ccap;
-  io.cf[c] = fa.x; io.cf[cc + c] = fa.y; io.cf[2 * cc + c] = fa.z;
-  io.cf[3 * cc + c] = ta.x; io.cf[4 * cc + c] = ta.y; io.cf[5 * cc + c] = ta.z;
-  io.cf[6 * cc + c] = fb.x; io.cf[7 * cc + c] = fb.y; io.cf[8 * cc + c] = fb.z;
-  io.cf[9 * cc + c] = tb.x; io.cf[10 * cc + c] = tb.y; io.cf[11 * cc + c] = tb.z;
+  store_addends(io.cf, cc, c, p);
+  io.touched[c] = p.touch;
+  if (p.touch && hf >= 0) io.kept[hf] = 0;  // the touched entry is rewritten, not retained
+  io.newval[c] = p.hist.x; io.newval[cc + c] = p.hist.y; io.newval[2 * cc + c] = p.hist.z;
+  io.pe[c] = p.pe;
 }
 
 __global__ void k_soft_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
@@ -210,103 +199,13 @@ __global__ void k_soft_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
   if (ctl->err) return;
   const int C = ctl->contacts, H = ctl->hist_n;
   eval_begin(ctl);
-  const double dt = cfg.dt;
-  const double K1 = 15.0 / cfg.soft_delta;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
     const int a = io.ca[c], b = io.cb[c];
     const int hf = hist_find(io, a, b, H);
-    d3 pa = ldc(io, 0, c), pb = ldc(io, 3, c), nrm = ldc(io, 6, c), sh = ldc(io, 9, c);
-    double dist = io.g[(size_t)12 * io.ccap + c], hs = io.g[(size_t)13 * io.ccap + c];
-    // potentialGradient / potentialEnergy
-    double grad, U;
-    if (dist > hs - cfg.soft_delta) {
-      double arg = K1 * (hs - dist);
-      double e = exp(arg);
-      double lt = log(1.0 + e);
-      grad = -2.0 / (K1 * K1) * lt * e / (1.0 + e);
-      double base = lt / K1;
-      U = base * base;
-    } else {
-      grad = -2.0 * (hs - dist);
-      double pen = hs - dist;
-      U = pen * pen;
-    }
-    double fm = -cfg.soft_k_scaler * grad;
-    d3 fa = nrm * (-fm);
-    d3 fb = nrm * fm;
-    d3 xa = st.x.ld(a), xb = st.x.ld(b);
-    d3 ra = pa - xa;
-    d3 rb = pb - (xb + sh);
-    d3 va = st.v.ld(a) + cross(st.w.ld(a), ra);
-    d3 vb = st.v.ld(b) + cross(st.w.ld(b), rb);
-    d3 vrel = va - vb;
-    if (cfg.soft_damping > 1e-9) {
-      double vn = dot(vrel, nrm);
-      d3 fd = nrm * (-cfg.soft_damping * vn);
-      fa = fa + fd;
-      fb = fb - fd;
-    }
-    d3 fra{0, 0, 0};
-    int touch = 0;
-    d3 nv{0, 0, 0};
-    if (cfg.soft_enable_friction) {
-      double fn_mag = len(fa);
-      d3 vt = vrel - nrm * dot(vrel, nrm);
-      double vtm = len(vt);
-      if (!(vtm < 1e-10)) {
-        if (cfg.soft_friction_mode == RG_FRICTION_CUNDALL) {
-          const int f = hf;
-          d3 old{0, 0, 0};
-          if (f >= 0) old = mk3(io.hval[f], io.hval[io.hcap + f], io.hval[2 * io.hcap + f]);
-          d3 ft = old - vt * (cfg.soft_kt * dt);
-          double ncmp = dot(ft, nrm);
-          ft = ft - nrm * ncmp;
-          double ftm = len(ft);
-          double lim = cfg.soft_mu * fn_mag;
-          if (ftm > lim) {
-            if (ftm > 1e-8) ft = ft * (lim / ftm);
-            else ft = mk3(0, 0, 0);
-          }
-          nv = ft;
-          touch = 1;
-          fra = ft;
-        } else if (cfg.soft_friction_mode == RG_FRICTION_KARNOPP) {
-          if (vtm < cfg.soft_vel_deadband) {
-            double ma = st.inv_mass[a] > 0 ? st.mass[a] : 0.0;
-            double mb = st.inv_mass[b] > 0 ? st.mass[b] : 0.0;
-            double meff = 0;
-            if (ma > 0 && mb > 0) meff = (ma * mb) / (ma + mb);
-            else if (ma > 0) meff = ma;
-            else if (mb > 0) meff = mb;
-            d3 fstop = vt * (-(meff / dt));
-            d3 gv{cfg.gravity[0], cfg.gravity[1], cfg.gravity[2]};
-            d3 gt = gv - nrm * dot(gv, nrm);
-            d3 fdrive = gt * meff;
-            d3 freq = fstop - fdrive;
-            double frm = len(freq);
-            double maxs = cfg.soft_mu_static * fn_mag;
-            if (frm <= maxs) fra = freq;
-            else if (frm > 1e-12) fra = freq * (maxs / frm);
-          } else {
-            fra = (vt * -1.0 / vtm) * (cfg.soft_mu * fn_mag);
-          }
-        } else {
-          double K2 = 15.0 / cfg.soft_nu;
-          double gamma = vtm > cfg.soft_nu ? 1.0 : 2.0 / (1.0 + exp(-K2 * vtm)) - 1.0;
-          double mu_eff = cfg.soft_mu;
-          if (cfg.soft_mu_static > cfg.soft_mu)
-            mu_eff = cfg.soft_mu + (cfg.soft_mu_static - cfg.soft_mu) * exp(-vtm / cfg.soft_nu);
-          d3 dir = (-vt) / vtm;
-          fra = dir * (mu_eff * gamma * fn_mag);
-        }
-      }
-    }
-    d3 ta = fa + fra, tb = fb - fra;
-    st_cf(io, c, ta, cross(ra, ta), tb, cross(rb, tb));
-    io.touched[c] = touch;
-    if (touch && hf >= 0) io.kept[hf] = 0;  // the touched entry is rewritten, not retained
-    io.newval[c] = nv.x; io.newval[io.ccap + c] = nv.y; io.newval[2 * io.ccap + c] = nv.z;
-    io.pe[c] = cfg.soft_k_scaler * U;
+    const d3 old = hf >= 0 ? mk3(io.hval[hf], io.hval[io.hcap + hf], io.hval[2 * io.hcap + hf]) : mk3(0, 0, 0);
+    const PairForce p = soft_pair(st, cfg, a, b, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
+                                  io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, true);
+    st_pair(io, c, hf, p);
   }
 }
 
@@ -315,81 +214,14 @@ __global__ void k_hm_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
   if (ctl->err) return;
   const int C = ctl->contacts, H = ctl->hist_n;
   eval_begin(ctl);
-  const double dt = cfg.dt;
-  const double nu = cfg.hm_poisson_ratio;
-  const double Es = cfg.hm_youngs_modulus / (2.0 * (1.0 - nu * nu));
-  const double Gs = cfg.hm_youngs_modulus / (2.0 * (1.0 + nu));
-  double gam = 0.0;
-  if (cfg.hm_restitution < 1.0) {
-    double l = log(cfg.hm_restitution);
-    gam = -l / sqrt(M_PI * M_PI + l * l);
-  }
+  const HmConst k = hm_const(cfg);
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
     const int a = io.ca[c], b = io.cb[c];
     const int hf = hist_find(io, a, b, H);
-    d3 pa = ldc(io, 0, c), pb = ldc(io, 3, c), nrm = ldc(io, 6, c), sh = ldc(io, 9, c);
-    double dist = io.g[(size_t)12 * io.ccap + c], hs = io.g[(size_t)13 * io.ccap + c];
-    double ra_ = st.r[a], rb_ = st.r[b], ma = st.mass[a], mb = st.mass[b];
-    double delta = hs - dist;
-    double Rs = (ra_ * rb_) / (ra_ + rb_);
-    double ms = (ma * mb) / (ma + mb);
-    double sd = smax(delta, 0.0);
-    double sqd = sqrt(sd);
-    double sqR = sqrt(smax(Rs, 0.0));
-    double kn = (4.0 / 3.0) * Es * sqR * sqd;
-    double Fel = kn * sd * sqd;
-    d3 xa = st.x.ld(a), xb = st.x.ld(b);
-    d3 ra = pa - xa;
-    d3 rb = pb - (xb + sh);
-    d3 wa = st.w.ld(a), wb = st.w.ld(b);
-    d3 va = st.v.ld(a) + cross(wa, ra);
-    d3 vb = st.v.ld(b) + cross(wb, rb);
-    d3 vrel = vb - va;
-    double vn = dot(vrel, nrm);
-    double Cn = gam * 2.0 * sqrt(ms * kn);
-    double Fn = smax(0.0, Fel + (-Cn * vn));
-    d3 fn = nrm * Fn;
-    d3 ft{0, 0, 0};
-    const int f = hf;
-    d3 xi{0, 0, 0};
-    if (f >= 0) xi = mk3(io.hval[f], io.hval[io.hcap + f], io.hval[2 * io.hcap + f]);
-    if (cfg.hm_enable_tangential) {
-      double kt = 8.0 * Gs * sqR * sqd;
-      d3 vt = vrel - nrm * vn;
-      xi = xi + vt * dt;
-      d3 fel = xi * (-kt);
-      double Ct = gam * 2.0 * sqrt(ms * kt);
-      ft = fel - vt * Ct;
-      double vtm = len(vt);
-      double mu_eff = cfg.hm_friction;
-      if (cfg.hm_friction_static > cfg.hm_friction && cfg.hm_friction_transition_vel > 0.0)
-        mu_eff += (cfg.hm_friction_static - cfg.hm_friction) * exp(-vtm / cfg.hm_friction_transition_vel);
-      double fnm = len(fn);
-      double ftm = len(ft);
-      double ftmax = mu_eff * fnm;
-      if (ftm > ftmax && ftm > 1e-10) {
-        ft = ft * (ftmax / ftm);
-        if (kt > 1e-10) xi = ft / (-kt);
-      }
-    }
-    d3 tra{0, 0, 0}, trb{0, 0, 0};
-    if (cfg.hm_enable_rolling) {
-      d3 wr = wa - wb;
-      double wm = len(wr);
-      if (!(wm < 1e-10)) {
-        d3 wh = wr / wm;
-        double trm = cfg.hm_rolling_friction * Rs * len(fn);
-        d3 tr = wh * (-trm);
-        tra = tr * 0.5;
-        trb = tr * -0.5;
-      }
-    }
-    d3 F = fn + ft;
-    st_cf(io, c, -F, cross(ra, -F) + tra, F, cross(rb, F) + trb);
-    io.touched[c] = 1;
-    if (hf >= 0) io.kept[hf] = 0;  // the touched entry is rewritten, not retained
-    io.newval[c] = xi.x; io.newval[io.ccap + c] = xi.y; io.newval[2 * io.ccap + c] = xi.z;
-    io.pe[c] = (8.0 / 15.0) * Es * sqrt(Rs) * pow(delta, 2.5);
+    const d3 old = hf >= 0 ? mk3(io.hval[hf], io.hval[io.hcap + hf], io.hval[2 * io.hcap + hf]) : mk3(0, 0, 0);
+    const PairForce p = hm_pair(st, cfg, k, a, b, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
+                                io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, true);
+    st_pair(io, c, hf, p);
   }
 }
 
@@ -453,7 +285,7 @@ void force_eval_launch(rg_system* s, EvalTail tail, bool seg_ready) {
   const bool hm = c.model == RG_MODEL_HERTZ_MINDLIN;
   cudaStream_t st = s->stream;
   const int bs = 256;
-  if (!s->contacts_fresh) {
+  if (s->contacts_fresh != Fresh::kCsr) {
     ProfScope p(s, ST_DETECT);
     detect_launch(s, hm ? 0.0 : c.soft_delta, true, seg_ready, true);
     csr_launch(s, true);

@@ -5,28 +5,9 @@
 // flight and position update of App::physicsStep (src/app/main.cpp:4397-4408,
 // :4469-4483) and its PBC wrap (:4508-4517).  State is structure-of-arrays
 // FP64, so every load and store is a fully coalesced 8-byte access.
-#include "rg_nsc_dev.cuh"
+#include "rg_verlet_dev.cuh"
 
 namespace rg {
-
-// Iinv = 1/I per principal axis for a dynamic body (0 when I = 0), as the
-// state's stored inverse (rg_set_bodies), recomputed here to save its load.
-__device__ inline d3 ang_accel(const State& st, int i, dq q, d3 w, d3 tau) {
-  const d3 I = st.I.ld(i);
-  const d3 Iinv{I.x > 0.0 ? 1.0 / I.x : 0.0, I.y > 0.0 ? 1.0 / I.y : 0.0, I.z > 0.0 ? 1.0 / I.z : 0.0};
-  d3 Iw_w = rot_diag_apply(q, I, w);
-  d3 gyro = cross(w, Iw_w);
-  return rot_diag_apply(q, Iinv, tau - gyro);
-}
-
-__device__ inline void rotate_by_omega(dq& q, d3 w, double dt) {
-  double wl = len(w);
-  if (wl > 1e-8) {
-    double ang = wl * dt;
-    d3 ax = w / wl;
-    q = qnormalize(qmul(angle_axis(ang, ax), q));
-  }
-}
 
 // Resident 256-thread blocks per SM the streaming body kernels are compiled
 // for (register budget 65536 / (256 * this)); they are latency-bound at
@@ -42,12 +23,6 @@ __device__ inline void rotate_by_omega(dq& q, d3 w, double dt) {
 // and the displacement bound against the list reference (k_disp_check's
 // check, rg_detect.cu) are written in the same pass, so the detection at
 // t + dt starts at the cell/list stage.
-struct DriftOut {
-  Seg* seg;           // segment records of the drifted positions (n)
-  const double* ref;  // list reference segments (6n), or null: no check
-  const double* ref2; // near-list reference segments (6n), or null
-  double skin;
-};
 __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
     k_reduce_drift(State st, Box box, rg_config cfg, const int* off, const int* ent, const double* cf,
                    int ccap, int wall, DriftOut o, HistFinish hf, Ctl* ctl) {
@@ -55,37 +30,16 @@ __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
   if (ctl->err) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) hist_finish(hf, ctl);
   __shared__ double sm[32], sm2[32];
-  const d3 g{cfg.gravity[0], cfg.gravity[1], cfg.gravity[2]};
-  const double dt = cfg.dt, hdt = 0.5 * cfg.dt;
   const d3 ax = wall ? soft_wall_axis(cfg) : mk3(0, 0, 0);
   const int n = st.n;
   double m = 0.0, m2 = 0.0;
+  double invL[3] = {1.0, 1.0, 1.0};
+  for (int k = 0; k < 3; ++k)
+    if (box.L[k] > 0.0) invL[k] = 1.0 / box.L[k];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    d3 x = st.x.ld(i);
-    dq q = st.q.ld(i);
-    if (st.inv_mass[i] > 0.0) {
-      d3 f{0, 0, 0}, t{0, 0, 0};
-      body_sum(off, ent, cf, ccap, i, f, t);
-      d3 v = st.v.ld(i), w = st.w.ld(i);
-      if (wall) soft_wall_apply(cfg, ax, st.r[i], x, v, f);
-      d3 al = f / st.mass[i] + g;
-      d3 aa = ang_accel(st, i, q, w, t);
-      v = v + al * hdt;
-      w = w + aa * hdt;
-      x = x + v * dt;
-      wrap_pos(box, x);
-      rotate_by_omega(q, w, dt);
-      st.v.st(i, v);
-      st.w.st(i, w);
-      st.x.st(i, x);
-      st.q.st(i, q);
-    }
-    const Seg sg = seg_of(x, q, st.h[i], st.r[i]);
-    o.seg[i] = sg;
-    if (o.ref) {
-      m = fmax(m, seg_disp(sg, o.ref, n, i, box));  // non-finite state: 1e300 forces a rebuild
-      if (o.ref2) m2 = fmax(m2, seg_disp(sg, o.ref2, n, i, box));
-    }
+    d3 f{0, 0, 0}, t{0, 0, 0};
+    if (st.inv_mass[i] > 0.0) body_sum(off, ent, cf, ccap, i, f, t);
+    drift_rod(st, box, cfg, ax, wall, i, f, t, o, invL, m, m2);
   }
   if (!o.ref) return;
   m = warp_max(m);
@@ -117,30 +71,13 @@ __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
   griddep_wait();
   if (ctl->err) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) hist_finish(hf, ctl);
-  const d3 g{cfg.gravity[0], cfg.gravity[1], cfg.gravity[2]};
-  const double hdt = 0.5 * cfg.dt;
   const double el = exp(-cfg.lin_damp * cfg.dt), ea = exp(-cfg.ang_damp * cfg.dt);
   const d3 ax = wall ? soft_wall_axis(cfg) : mk3(0, 0, 0);
   int bad = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < st.n; i += gridDim.x * blockDim.x) {
     d3 f{0, 0, 0}, t{0, 0, 0};
     body_sum(off, ent, cf, ccap, i, f, t);
-    if (st.inv_mass[i] > 0.0) {
-      dq q = st.q.ld(i);
-      d3 v = st.v.ld(i), w = st.w.ld(i);
-      if (wall) soft_wall_apply(cfg, ax, st.r[i], st.x.ld(i), v, f);
-      d3 al = f / st.mass[i] + g;
-      d3 aa = ang_accel(st, i, q, w, t);
-      v = v + al * hdt;
-      w = w + aa * hdt;
-      if (cfg.lin_damp > 0.0) v = v * el;
-      if (cfg.ang_damp > 0.0) w = w * ea;
-      double wl = len(w);
-      if (wl > cfg.w_max) w = w * (cfg.w_max / wl);
-      st.v.st(i, v);
-      st.w.st(i, w);
-      if (!(v.x == v.x && v.y == v.y && v.z == v.z)) bad = 1;
-    }
+    bad |= kick_rod(st, cfg, ax, wall, i, f, t, el, ea);
     st.f.st(i, f);
     st.tau.st(i, t);
   }

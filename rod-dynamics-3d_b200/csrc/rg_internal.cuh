@@ -59,6 +59,7 @@ struct Ctl {
   int det_valid;        // 1: the near-pair hit bits hold the position-level
                         // detection of this call's last step
   unsigned int bar_count, bar_gen;  // grid barrier
+  int ins_n[2];         // pairs an evaluation adds to the history (by parity)
   double res_sweep[1];  // per-sweep residual slots follow (velocity_iters)
 };
 
@@ -172,6 +173,25 @@ struct Nsc {
 // bytes behind a team's barrier words (zeroed before every launch): 4 words
 // and the residual ring of the split solve (rg_nsc.cu)
 constexpr size_t kTeamBarBytes = 1024;
+// Contact bookkeeping of the persistent Verlet step (rg_verlet.cu).
+struct VerletTeam {
+  // two contact lists (before and after a detection): per rod the first of
+  // its contacts, per contact its second body and its history entry (-1: none)
+  int *off[2] = {nullptr, nullptr}, *pb[2] = {nullptr, nullptr}, *hidx[2] = {nullptr, nullptr};
+  int cb = 0;                            // the current one
+  int *head = nullptr, *next = nullptr;  // per rod: list of the contacts it is second body of
+  int* ins = nullptr;                    // contacts whose pair an evaluation adds
+  void* view_dev = nullptr;
+  cudaError_t alloc(int n, int ccap);
+  void free_();
+};
+// Largest system whose Verlet steps run in the persistent form, and the rods
+// a block of its team takes.
+constexpr int kVerletTeamRods = 600000, kVerletRodsPerBlock = 128;
+// What the contact buffers hold: nothing current, the contacts of the current
+// positions with the body CSR (multi-kernel form), or with the persistent
+// form's bookkeeping.
+enum class Fresh { kNo, kCsr, kTeam };
 constexpr int kRowComps = 42;
 constexpr int kExportComps = 11;
 constexpr int kPosComps = 12;
@@ -186,7 +206,7 @@ struct rg_system {
   cudaStream_t stream = nullptr;
   std::string err_text;
   bool bodies_set = false, state_set = false;
-  bool contacts_fresh = false;  // contacts match the current positions
+  rg::Fresh contacts_fresh = rg::Fresh::kNo;  // contacts match the current positions
 
   double* d_state = nullptr;  // 19 n
   double* d_props = nullptr;  // 11 n
@@ -202,6 +222,7 @@ struct rg_system {
   rg::BodyCSR csr;
   rg::History hist;
   rg::Nsc nsc;
+  rg::VerletTeam vteam;
   rg::Scan scan;
   double* d_cf = nullptr;     // per-contact force/torque addends, 12 * ccap
 
@@ -359,6 +380,10 @@ int nsc_team_blocks(const rg_system* s);
 int nsc_blocks_per_sm();
 size_t nsc_view_bytes();
 size_t nsc_team_bytes();
+// rg_verlet.cu
+bool verlet_team_fits(const rg_system* s);  // its Verlet steps run in the persistent form
+void verlet_run_launch(rg_system* s, int nsteps);
+void verlet_launched(rg_system* s, int nsteps);
 // rg_mlp.cu
 void mlp_free(rg_system* s);
 

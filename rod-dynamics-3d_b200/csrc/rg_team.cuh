@@ -1,0 +1,265 @@
+// rg_team.cuh - what the persistent step kernels (rg_nsc.cu, rg_verlet.cu)
+// share: teams of co-resident blocks, their bounded barriers, scans and phase
+// clocks, and the neighbour-list rebuild of one system by its team.
+#pragma once
+#include "rg_nsc_dev.cuh"
+
+namespace rg {
+
+// ---------------------------------------------------------------------------
+// Teams and team barriers.
+// ---------------------------------------------------------------------------
+struct Team {
+  int b0, nb;
+  unsigned int* bar;      // 4 barrier words, then the residual ring
+  int* err;
+  long long spin_limit;   // polls per barrier wait before ERR_TIMEOUT
+  unsigned int absent;    // test hook: blocks the barriers wait for in vain
+  __device__ int rank() const { return (int)blockIdx.x - b0; }
+  __device__ int tid() const { return rank() * (int)blockDim.x + (int)threadIdx.x; }
+  __device__ int size() const { return nb * (int)blockDim.x; }
+  // residuals of the split solve's chunks: three buffers of kChunk, zero at
+  // the start of a launch
+  __device__ double* ring() const { return reinterpret_cast<double*>(bar + 4); }
+};
+
+// Barrier of the whole team.  The arrivals are counted, never reset: barrier k
+// of a launch is over when the count reaches (k + 1) times the blocks, so a
+// block needs one atomic and then only reads (the sense-reversing grid_sync
+// also reads the generation and the error word first, each a round trip to
+// L2).  The count starts at zero (memset before the launch) and every block
+// keeps k in shared memory (team_barriers_reset at kernel start).  Bounded
+// like grid_sync.  Measured
+// with 148 blocks, waits for slower blocks included: 3.0 -> 1.9 us.
+static __shared__ unsigned team_barrier_k;
+__device__ inline void team_barriers_reset() {
+  if (threadIdx.x == 0) team_barrier_k = 0;
+  __syncthreads();
+}
+__device__ inline bool team_sync(const Team& T) {
+  __syncthreads();
+  const unsigned nb = (unsigned)T.nb + T.absent;
+  if (nb <= 1) return !(*(volatile int*)T.err & ERR_TIMEOUT);
+  int ok = 1;
+  if (threadIdx.x == 0) {
+    cuda::atomic_ref<unsigned, cuda::thread_scope_device> count(*T.bar);
+    const unsigned target = (++team_barrier_k) * nb;  // modulo 2^32, as the count
+    count.fetch_add(1u, cuda::memory_order_release);
+    long long it = 0;
+    while ((int)(count.load(cuda::memory_order_acquire) - target) < 0) {
+      ++it;
+      if ((it & 63) == 0 && (*(volatile int*)T.err & ERR_TIMEOUT)) { ok = 0; break; }
+      if (it > T.spin_limit) {
+        atomicOr(T.err, ERR_TIMEOUT);
+        ok = 0;
+        break;
+      }
+      if (it > 256) __nanosleep(32);
+    }
+  }
+  return __syncthreads_and(ok) != 0;
+}
+// Barrier among the first nsub blocks of the team (the others must not call it).
+__device__ inline bool team_sync_sub(const Team& T, int nsub) {
+  GridBar g{T.bar + 2, T.bar + 3, T.err, T.spin_limit, T.absent};
+  return grid_sync(g, (unsigned)nsub);
+}
+
+__device__ inline double block_reduce_max(double v, double* sm) {
+  v = warp_max(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double r = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
+  if (threadIdx.x < 32) r = warp_max(r);
+  return r;  // valid in thread 0
+}
+__device__ inline int block_reduce_sum_i(int v, int* sm) {
+  v = warp_sum_i(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int r = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0;
+  if (threadIdx.x < 32) r = warp_sum_i(r);
+  return r;  // valid in thread 0
+}
+
+// Phase timers (team rank 0, thread 0; %globaltimer in ns) when enabled.
+// ---------------------------------------------------------------------------
+__device__ inline unsigned long long gtimer() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+struct PhaseClock {
+  Ctl* ctl;
+  bool on;
+  unsigned long long t;
+  __device__ PhaseClock(Ctl* c, bool enabled) : ctl(c), on(enabled), t(enabled ? gtimer() : 0) {}
+  __device__ void mark(int k) {
+    if (!on) return;
+    unsigned long long u = gtimer();
+    ctl->phase_ns[k] += (long long)(u - t);
+    t = u;
+  }
+};
+
+// Dynamic shared memory of the persistent kernels: the list-build tiles while
+// a rebuild runs (NSC: the small-solve arrays at other times).
+extern __shared__ __align__(16) unsigned char team_dyn_smem[];
+// list-build candidate queues, after the tiles
+constexpr int kBuildQ = 4096;
+constexpr size_t kBuildQOff = (sizeof(BuildSmem) + 15) & ~(size_t)15;
+
+struct SmemNsc {
+  double red_d[32];
+  int red_i[32];
+  int scan_w[32];
+  int pre[32];
+  int coff[kMaxColors + 1];
+  int bcast;
+};
+
+// Every block computes Σ blk[0..rank) and Σ blk[0..nb).
+__device__ inline void block_prefix(const int* blk, int nb, int rank, int& prefix, int& total, SmemNsc& sm) {
+  int a = 0, b = 0;
+  for (int r = threadIdx.x; r < nb; r += blockDim.x) {
+    int v = *(volatile const int*)&blk[r];
+    b += v;
+    if (r < rank) a += v;
+  }
+  int pa = warp_sum_i(a), pb = warp_sum_i(b);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    sm.pre[threadIdx.x >> 5] = pa;
+    sm.red_i[threadIdx.x >> 5] = pb;
+  }
+  __syncthreads();
+  int x = 0, y = 0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+    x += sm.pre[w];
+    y += sm.red_i[w];
+  }
+  prefix = x;
+  total = y;
+  __syncthreads();
+}
+
+// Exclusive scan of in[0..m) into out[0..m], out[m] = total (team, blocked).
+__device__ inline bool team_excl_scan(const Team& T, const int* in, int* out, int m, int* blk, SmemNsc& sm) {
+  const int rank = T.rank();
+  const int seg = (m + T.nb - 1) / T.nb;
+  const int lo = rank * seg < m ? rank * seg : m;
+  const int hi = lo + seg < m ? lo + seg : m;
+  int s = 0;
+  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) s += in[i];
+  int bsum = block_reduce_sum_i(s, sm.red_i);
+  if (threadIdx.x == 0) blk[rank] = bsum;
+  if (!team_sync(T)) return false;
+  int prefix, total;
+  block_prefix(blk, T.nb, rank, prefix, total, sm);
+  int run = prefix;
+  for (int base = lo; base < hi; base += blockDim.x) {
+    int i = base + threadIdx.x;
+    int v = i < hi ? in[i] : 0;
+    int tot;
+    int ex = block_excl_scan(v, sm.scan_w, tot);
+    if (i < hi) out[i] = run + ex;
+    run += tot;
+  }
+  if (rank == 0 && threadIdx.x == 0) out[m] = total;
+  return team_sync(T);
+}
+
+// ---------------------------------------------------------------------------
+// Detection inside the persistent kernel.
+// ---------------------------------------------------------------------------
+static __device__ __noinline__ bool rebuild_phase(const Team& T, const NscView& V, SmemNsc& sm) {
+  Ctl* ctl = V.ctl;
+  const int n = V.st.n;
+  const int tid = T.tid(), TS = T.size(), rank = T.rank();
+  if (!V.box.pbc) {
+    if (rank == 0 && threadIdx.x < 3) {
+      V.bounds[threadIdx.x] = ~0ull;
+      V.bounds[3 + threadIdx.x] = 0ull;
+    }
+    if (!team_sync(T)) return false;
+    for (int i = tid; i < n; i += TS) {
+      Seg s = V.seg[i];
+      atomicMin(&V.bounds[0], ord_key(s.cx)); atomicMax(&V.bounds[3], ord_key(s.cx));
+      atomicMin(&V.bounds[1], ord_key(s.cy)); atomicMax(&V.bounds[4], ord_key(s.cy));
+      atomicMin(&V.bounds[2], ord_key(s.cz)); atomicMax(&V.bounds[5], ord_key(s.cz));
+    }
+    if (!team_sync(T)) return false;
+    if (rank == 0 && threadIdx.x == 0) open_grid(V.bounds, V.bounds + 3, V.cut_center, 64, V.grid);
+    if (!team_sync(T)) return false;
+  }
+  GridDev g;
+  {
+    const volatile GridDev* vg = V.grid;
+    for (int k = 0; k < 3; ++k) {
+      g.lo[k] = vg->lo[k];
+      g.cell[k] = vg->cell[k];
+      g.n[k] = vg->n[k];
+    }
+    g.ncells = vg->ncells;
+  }
+  unsigned long long t_start = (ctl->prof_phases && rank == 0 && threadIdx.x == 0) ? gtimer() : 0;
+  for (int c = tid; c <= g.ncells; c += TS) {
+    V.cell_cnt[c] = 0;
+    V.cell_fill[c] = 0;
+  }
+  for (int i = tid; i < n; i += TS) V.nbr_cnt[i] = 0;
+  if (!team_sync(T)) return false;
+  for (int i = tid; i < n; i += TS) {
+    Seg s = V.seg[i];
+    int cx = cell_coord(s.cx, g.lo[0], g.cell[0], g.n[0], V.box.pbc);
+    int cy = cell_coord(s.cy, g.lo[1], g.cell[1], g.n[1], V.box.pbc);
+    int cz = cell_coord(s.cz, g.lo[2], g.cell[2], g.n[2], V.box.pbc);
+    int c = (cz * g.n[1] + cy) * g.n[0] + cx;
+    V.cell_of[i] = c;
+    atomicAdd(&V.cell_cnt[c], 1);
+  }
+  if (!team_sync(T)) return false;
+  if (!team_excl_scan(T, V.cell_cnt, V.cell_start, g.ncells, V.blk, sm)) return false;
+  for (int i = tid; i < n; i += TS) {
+    int c = V.cell_of[i];
+    V.cell_rods[V.cell_start[c] + atomicAdd(&V.cell_fill[c], 1)] = i;
+  }
+  if (!team_sync(T)) return false;
+  int overflow = 0;
+  double invL[3] = {1.0, 1.0, 1.0};
+  for (int k = 0; k < 3; ++k)
+    if (V.box.L[k] > 0.0) invL[k] = 1.0 / V.box.L[k];
+  if (n < 48 * g.ncells) {
+    // sparse cells: one thread per home rod
+    for (int i = tid; i < n; i += TS)
+      build_rod_list(i, V.seg, g, V.box, invL, V.cell_of, V.cell_start, V.cell_rods, V.margin, V.skin,
+                     V.all_pairs, V.nbr_cnt, V.nbr, V.maxnb, overflow);
+  } else {
+    // crowded cells: the block splits the pairs of one home cell at a time
+    for (int cell = rank; cell < g.ncells; cell += T.nb)
+      build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin, V.all_pairs,
+                       V.nbr_cnt, V.nbr, V.maxnb, cell, *reinterpret_cast<BuildSmem*>(team_dyn_smem),
+                       reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff),
+                       reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff) + kBuildQ, kBuildQ, overflow);
+  }
+  if (!team_sync(T)) return false;
+  for (int i = tid; i < n; i += TS) {
+    sort_list(V.nbr, V.nbr_cnt, V.maxnb, i, overflow);
+    Seg s = V.seg[i];
+    V.ref[i] = s.cx; V.ref[n + i] = s.cy; V.ref[2 * n + i] = s.cz;
+    V.ref[3 * n + i] = s.ux; V.ref[4 * n + i] = s.uy; V.ref[5 * n + i] = s.uz;
+  }
+  if (overflow) atomicOr(&ctl->err, ERR_NBR_CAP);
+  if (!team_sync(T)) return false;
+  if (*(volatile int*)&ctl->err) return false;
+  if (rank == 0 && threadIdx.x == 0) {
+    ctl->rebuild = 0;
+    ctl->rebuilds += 1;
+    if (t_start) ctl->phase_ns[9] += (long long)(gtimer() - t_start);
+  }
+  return true;
+}
+
+}  // namespace rg

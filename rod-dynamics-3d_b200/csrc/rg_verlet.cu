@@ -1,0 +1,617 @@
+// rg_verlet.cu - the velocity-Verlet step (soft and Hertz-Mindlin models) as
+// one persistent kernel for small and medium systems.
+//
+// The same step as the multi-kernel form (rg_api.cu verlet_step; App::
+// physicsStep, src/app/main.cpp:4529-4810): forces at t, half kick and drift,
+// detection, forces at t + dt, second half kick - the same expressions in the
+// same order, so states, contacts and histories are bit-identical.  A team of
+// co-resident blocks runs all steps of a call in one cooperative launch, with
+// five bounded team barriers a step where the multi-kernel form has 25
+// dependent kernels.  Teams of one launch are independent systems (batches).
+//
+// What makes five barriers enough:
+//  * a contact's force is computed by the thread that writes the contact, in
+//    the pass after the hit counts are known; the forces at the next step's
+//    start reuse those contacts in place;
+//  * a body's contacts are found without a sorted incidence table: those where
+//    it is the first body are a contiguous range of the (a, b)-sorted list,
+//    those where it is the second hang off it in a short linked list, walked
+//    in ascending order; together the contact order of the reference's sums;
+//  * the history entry of a persisting contact is found through the previous
+//    contact list (same first body, a handful of candidates) and rewritten in
+//    place; the sorted table is merged only in evaluations that add a pair,
+//    and entries past their retention are only passed over until the call
+//    ends (or the table fills up), when they are removed.
+//
+// Bound: instruction and L2 latency of the five phases plus the barriers (1 to
+// 2 us each).  Measured, multi-kernel form -> this one, us per step: 1,000
+// rods 80 -> 38, 5,000 (soft) 104 -> 39, 20,000 103 -> 52, 100,000 130 -> 82,
+// 400,000 279 -> 238, 1,000,000 441 -> 507 (sparse contacts) and 641 -> 606
+// (80,000 contacts).  The line between them (kVerletTeamRods) lies where the
+// multi-kernel form, with more warps on an SM for the per-rod passes, draws
+// level.
+#include <cstring>
+#include <vector>
+
+#include "rg_team.cuh"
+#include "rg_verlet_dev.cuh"
+
+namespace rg {
+
+constexpr int kVBlock = 2 * kTile;  // threads per block
+constexpr int kIns = 512;           // inserted pairs sorted on chip
+
+// Where one team stands in its system's call (the same in every block).
+struct VerletRun {
+  int H, cur;      // history entries (dead ones included), current table
+  int C, cb;       // contacts, current contact-index buffer
+  long long fr;    // evaluation counter
+  bool idx_ok;     // hidx[cb] names the contacts' table entries
+  int lo, hi;      // this block's rods
+  HmConst hm;
+};
+struct VerletSmem {
+  SmemNsc s;
+  unsigned long long key[kIns], sorted[kIns];
+};
+
+__device__ inline bool v_is_hm(const VerletView& W) { return W.v.cfg.model == RG_MODEL_HERTZ_MINDLIN; }
+
+// Entry of the current table, or -1.
+__device__ inline int v_find(const VerletView& W, const VerletRun& r, int a, int b) {
+  const unsigned long long k = pkey(a, b);
+  const int p = lower_bound_u64(W.hkey[r.cur], r.H, k);
+  return (p < r.H && W.hkey[r.cur][p] == k) ? p : -1;
+}
+
+// Force of contact c with table entry f (-1: none); updates the entry, or
+// lists the pair for insertion.  energy: the contact's potential energy is
+// wanted (of a call only the last evaluation's sum is kept).
+__device__ inline void v_eval(const VerletView& W, const VerletRun& r, int c, int f, bool energy) {
+  const NscView& V = W.v;
+  const Contacts& con = V.con;
+  const int a = con.a[c], b = con.b[c], hc = W.hcap, cc = V.ccap;
+  double* hv = W.hval[r.cur];
+  long long* hf = W.hframe[r.cur];
+  const bool hm = v_is_hm(W);
+  d3 old{0, 0, 0};
+  // an entry past its retention was dropped by the evaluation before this one
+  if (f >= 0 && (!hm || r.fr - hf[f] <= 5)) old = mk3(hv[f], hv[hc + f], hv[2 * (size_t)hc + f]);
+  const d3 pa{con.comp(0)[c], con.comp(1)[c], con.comp(2)[c]}, pb{con.comp(3)[c], con.comp(4)[c], con.comp(5)[c]};
+  const d3 nrm{con.comp(6)[c], con.comp(7)[c], con.comp(8)[c]}, sh{con.comp(9)[c], con.comp(10)[c], con.comp(11)[c]};
+  const double dist = con.comp(12)[c], hs = con.comp(13)[c];
+  const PairForce p = hm ? hm_pair(V.st, V.cfg, r.hm, a, b, pa, pb, nrm, sh, dist, hs, old, energy)
+                         : soft_pair(V.st, V.cfg, a, b, pa, pb, nrm, sh, dist, hs, old, energy);
+  store_addends(W.cf, cc, c, p);
+  if (energy) W.cf[12 * (size_t)cc + c] = p.pe;
+  int added = 0;
+  if (p.touch) {
+    if (f >= 0) {
+      hv[f] = p.hist.x; hv[hc + f] = p.hist.y; hv[2 * (size_t)hc + f] = p.hist.z;
+      hf[f] = r.fr;
+    } else {
+      W.newval[c] = p.hist.x; W.newval[cc + c] = p.hist.y; W.newval[2 * (size_t)cc + c] = p.hist.z;
+      W.ins[atomicAdd(&V.ctl->ins_n[r.fr & 1], 1)] = c;
+      added = 1;
+    }
+  }
+  W.touched[c] = added;
+  W.hidx[r.cb][c] = f;
+}
+
+// Removes the entries past their retention (Hertz-Mindlin) after evaluation
+// r.fr; keeps the contacts' indices.
+__device__ __noinline__ bool v_purge(const Team& T, const VerletView& W, VerletRun& r, SmemNsc& sm) {
+  if (!v_is_hm(W) || r.H == 0) return true;
+  const int tid = T.tid(), TS = T.size(), hc = W.hcap, src = r.cur, dst = 1 - r.cur;
+  for (int e = tid; e < r.H; e += TS) W.kept[e] = r.fr - W.hframe[src][e] <= 4 ? 1 : 0;
+  if (!team_sync(T)) return false;
+  if (!team_excl_scan(T, W.kept, W.kept_off, r.H, W.v.blk, sm)) return false;
+  const int K = W.kept_off[r.H];
+  if (K == r.H) return true;
+  for (int e = tid; e < r.H; e += TS) {
+    if (!W.kept[e]) continue;
+    const int p = W.kept_off[e];
+    W.hkey[dst][p] = W.hkey[src][e];
+    for (int k = 0; k < 3; ++k) W.hval[dst][(size_t)k * hc + p] = W.hval[src][(size_t)k * hc + e];
+    W.hframe[dst][p] = W.hframe[src][e];
+  }
+  for (int c = tid; c < r.C; c += TS) {
+    const int f = W.hidx[r.cb][c];
+    if (f >= 0) W.hidx[r.cb][c] = W.kept[f] ? W.kept_off[f] : -1;
+  }
+  if (!team_sync(T)) return false;
+  r.cur = dst;
+  r.H = K;
+  return true;
+}
+
+// Merges the pairs that evaluation r.fr added into the sorted table (every
+// block past a barrier since); the next evaluation is behind another barrier.
+__device__ __noinline__ bool v_insert(const Team& T, const VerletView& W, VerletRun& r, VerletSmem& S, int added) {
+  const NscView& V = W.v;
+  const int tid = T.tid(), TS = T.size(), t = threadIdx.x, hc = W.hcap, cc = V.ccap;
+  if (r.H + added > hc - hc / 4 && !v_purge(T, W, r, S.s)) return false;
+  if (r.H + added > hc) {
+    if (T.rank() == 0 && t == 0) atomicOr(&V.ctl->err, ERR_HIST_CAP);
+    return false;
+  }
+  const int src = r.cur, dst = 1 - r.cur;
+  const unsigned long long* ok = W.hkey[src];
+  const bool chip = added <= kIns;
+  if (chip) {  // every block sorts the added keys by counting
+    for (int i = t; i < added; i += blockDim.x) {
+      const int c = W.ins[i];
+      S.key[i] = pkey(V.con.a[c], V.con.b[c]);
+    }
+    __syncthreads();
+    for (int i = t; i < added; i += blockDim.x) {
+      int rank = 0;
+      for (int j = 0; j < added; ++j) rank += S.key[j] < S.key[i];
+      S.sorted[rank] = S.key[i];
+    }
+    __syncthreads();
+  } else if (!team_excl_scan(T, W.touched, W.touched_off, r.C, V.blk, S.s)) {
+    return false;
+  }
+  for (int e = tid; e < r.H; e += TS) {
+    const unsigned long long k = ok[e];
+    int before;
+    if (chip) {
+      before = lower_bound_u64(S.sorted, added, k);
+    } else {
+      int lo = 0, hi = r.C;  // contacts are sorted by key
+      while (lo < hi) {
+        const int m = (lo + hi) >> 1;
+        if (pkey(V.con.a[m], V.con.b[m]) < k) lo = m + 1;
+        else hi = m;
+      }
+      before = W.touched_off[lo];
+    }
+    const int p = e + before;
+    W.hkey[dst][p] = k;
+    for (int j = 0; j < 3; ++j) W.hval[dst][(size_t)j * hc + p] = W.hval[src][(size_t)j * hc + e];
+    W.hframe[dst][p] = W.hframe[src][e];
+  }
+  for (int c = tid; c < r.C; c += TS) {
+    const int f = W.hidx[r.cb][c];
+    const bool in = W.touched[c];
+    if (!in && f < 0) continue;
+    const unsigned long long k = pkey(V.con.a[c], V.con.b[c]);
+    const int before = chip ? lower_bound_u64(S.sorted, added, k) : W.touched_off[c];
+    const int p = before + (in ? lower_bound_u64(ok, r.H, k) : f);
+    W.hidx[r.cb][c] = p;
+    if (!in) continue;
+    W.hkey[dst][p] = k;
+    for (int j = 0; j < 3; ++j) W.hval[dst][(size_t)j * hc + p] = W.newval[(size_t)j * cc + c];
+    W.hframe[dst][p] = r.fr;
+  }
+  __syncthreads();  // the on-chip keys are free again
+  r.cur = dst;
+  r.H += added;
+  return true;
+}
+
+// Sums of body i's contact addends in contact order.
+__device__ inline void v_body_sum(const VerletView& W, const VerletRun& r, int i, d3& f, d3& t) {
+  const size_t cc = (size_t)W.v.ccap;
+  const int* next = W.next;
+  const int h0 = W.head[i];
+  for (int last = -1; h0 >= 0;) {  // second body of: ascending walk of the list
+    int c = 0x7fffffff;
+    for (int k = h0; k >= 0; k = next[k])
+      if (k > last && k < c) c = k;
+    if (c == 0x7fffffff) break;
+    const double* g = W.cf + 6 * cc + c;
+    f.x = f.x + g[0]; f.y = f.y + g[cc]; f.z = f.z + g[2 * cc];
+    t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
+    last = c;
+  }
+  const int* off = W.off[r.cb];
+  const int e = off[i + 1];
+  for (int c = off[i]; c < e; ++c) {  // first body of
+    const double* g = W.cf + c;
+    f.x = f.x + g[0]; f.y = f.y + g[cc]; f.z = f.z + g[2 * cc];
+    t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
+  }
+}
+
+// The largest displacement bounds of the block's rods.
+__device__ inline void v_publish_disp(const NscView& V, double m, double m2, SmemNsc& sm) {
+  m = block_reduce_max(m, sm.red_d);
+  m2 = block_reduce_max(m2, sm.red_d);
+  if (threadIdx.x == 0) {
+    atomic_max_nonneg(&V.ctl->maxdisp, m);
+    atomic_max_nonneg(&V.ctl->near_disp, m2);
+  }
+}
+
+// Detection at the current segment records (every block past a barrier since
+// they and the displacement bounds were written), and evaluation r.fr on the
+// contacts found.
+template <int G>
+__device__ __forceinline__ int v_count(const VerletView& W, const VerletRun& r, const int* cnt, const int* nbr,
+                                       int prefilter) {
+  const NscView& V = W.v;
+  int mine = 0;
+  for (int base = r.lo; base < r.hi; base += blockDim.x / G) {
+    const int i = base + threadIdx.x / G;
+    const bool valid = i < r.hi;
+    const int c = narrow_count_lanes<G>(i, valid, V.seg, V.st.inv_mass, V.box, W.delta, cnt, nbr, V.maxnb, V.words,
+                                        V.mask, prefilter);
+    if (valid && (threadIdx.x & (G - 1)) == 0) {
+      V.hit_cnt[i] = c;
+      W.head[i] = -1;
+      mine += c;
+    }
+  }
+  return mine;
+}
+__device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, VerletRun& r, VerletSmem& S,
+                                           bool energy) {
+  const NscView& V = W.v;
+  Ctl* ctl = V.ctl;
+  const int n = V.st.n, rank = T.rank(), t = threadIdx.x;
+  const bool need = *(volatile int*)&ctl->rebuild ||
+                    (!V.all_pairs && *(volatile double*)&ctl->maxdisp >= 0.5 * V.skin * (1.0 - 1e-9));
+  const bool near = W.near_cnt != nullptr;
+  const bool due = near && (need || !*(volatile int*)&ctl->near_valid ||
+                            *(volatile double*)&ctl->near_disp >= 0.5 * V.near_skin * (1.0 - 1e-9));
+  if (need && !rebuild_phase(T, V, S.s)) return false;
+  if (due) {
+    const double* im = V.st.inv_mass;
+    for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+      const Seg A = V.seg[i];
+      const bool a_static = !(im[i] > 0.0);
+      const int cnt = V.nbr_cnt[i];
+      const int* list = V.nbr + (size_t)i * V.maxnb;
+      int* out = W.near_nbr + (size_t)i * V.maxnb;
+      int m = 0;
+      for (int k = 0; k < cnt; ++k) {
+        const int j = list[k];
+        if (a_static && !(im[j] > 0.0)) continue;
+        const Seg B = V.seg[j];
+        const d3 xa{A.cx, A.cy, A.cz}, xb{B.cx, B.cy, B.cz};
+        if (seg_far(A, B, (xb - xa) + min_image_shift(V.box, xa, xb), A.r + B.r + W.extra)) continue;
+        out[m++] = j;
+      }
+      W.near_cnt[i] = m;
+      V.ref2[i] = A.cx; V.ref2[n + i] = A.cy; V.ref2[2 * n + i] = A.cz;
+      V.ref2[3 * n + i] = A.ux; V.ref2[4 * n + i] = A.uy; V.ref2[5 * n + i] = A.uz;
+    }
+    if (!team_sync(T)) return false;
+    if (rank == 0 && t == 0) {  // every block has read them
+      ctl->near_valid = 1;
+      ctl->near_disp = 0.0;
+      ctl->near_rebuilds += 1;
+    }
+  }
+  const int* cnt = near ? W.near_cnt : V.nbr_cnt;
+  const int* nbr = near ? W.near_nbr : V.nbr;
+  // four lanes a rod while they fill the block in one round
+  const int pre = near ? 0 : (V.all_pairs ? 2 : 1);
+  const int mine = 4 * (r.hi - r.lo) <= (int)blockDim.x || !near ? v_count<4>(W, r, cnt, nbr, pre)
+                                                                : v_count<1>(W, r, cnt, nbr, pre);
+  const int bsum = block_reduce_sum_i(mine, S.s.red_i);
+  if (t == 0) V.blk[rank] = bsum;
+  if (!team_sync(T)) return false;
+  if (rank == 0 && t == 0) ctl->maxdisp = 0.0;
+  int prefix, total;
+  block_prefix(V.blk, T.nb, rank, prefix, total, S.s);
+  if (total > V.ccap) {
+    if (rank == 0 && t == 0) atomicOr(&ctl->err, ERR_CONTACT_CAP);
+    return false;
+  }
+  const int ob = r.cb, cb = 1 - r.cb;  // the contact lists before and now
+  int* off = W.off[cb];
+  int run = prefix;
+  for (int base = r.lo; base < r.hi; base += blockDim.x) {
+    const int i = base + t;
+    const int c = i < r.hi ? V.hit_cnt[i] : 0;
+    int tot;
+    int o = run + block_excl_scan(c, S.s.scan_w, tot);
+    if (i < r.hi) off[i] = o;
+    if (c) {
+      const int* list = nbr + (size_t)i * V.maxnb;
+      for (int w = 0; w * 64 < cnt[i]; ++w)
+        for (unsigned long long m = __ldcg(&V.mask[(size_t)i * V.words + w]); m; m &= m - 1) {
+          V.con.a[o] = i;
+          V.con.b[o] = list[w * 64 + __ffsll((long long)m) - 1];
+          ++o;
+        }
+    }
+    run += tot;
+  }
+  if (rank == 0 && t == 0) {
+    off[n] = total;
+    ctl->contacts = total;
+    ctl->contact_steps += total;
+  }
+  r.C = total;
+  r.cb = cb;
+  __syncthreads();
+  for (int c = prefix + t; c < run; c += blockDim.x) {
+    const int a = V.con.a[c], b = V.con.b[c];
+    const Seg A = V.seg[a], B = V.seg[b];
+    const Narrow nr = narrow_pair(A, B, V.box);
+    write_contact(V.con, c, a, b, A.r + B.r, nr);
+    W.pb[cb][c] = b;
+    W.next[c] = atomicExch(&W.head[b], c);
+    int f = -1;
+    bool known = false;
+    if (r.idx_ok)
+      for (int k = W.off[ob][a]; k < W.off[ob][a + 1]; ++k)
+        if (W.pb[ob][k] == b) {
+          f = W.hidx[ob][k];
+          known = true;
+        }
+    if (!known && r.H > 0) f = v_find(W, r, a, b);
+    v_eval(W, r, c, f, energy);
+  }
+  r.idx_ok = true;
+  return true;
+}
+
+// Potential energy in the order of the multi-kernel form's one 1024-thread
+// block (k_pe_sum), by the first block.
+__device__ inline void v_energy(const VerletView& W, int C, SmemNsc& sm) {
+  const double* pe = W.cf + 12 * (size_t)W.v.ccap;
+  const int t = threadIdx.x, warp = t >> 5;
+  for (int h = 0; h < 1024; h += blockDim.x) {
+    double v = 0;
+    for (int c = h + t; c < C; c += 1024) v += pe[c];
+    v = warp_sum(v);
+    if ((t & 31) == 0) sm.red_d[(h >> 5) + warp] = v;
+  }
+  __syncthreads();
+  if (t < 32) {
+    const double u = warp_sum(sm.red_d[t]);
+    if (t == 0) W.v.ctl->pe = u;
+  }
+  __syncthreads();
+}
+
+// nsteps steps of one system by its team.
+__device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nsteps, VerletSmem& S) {
+  const NscView& V = W.v;
+  const State& st = V.st;
+  const rg_config& cfg = V.cfg;
+  Ctl* ctl = V.ctl;
+  const int n = st.n, rank = T.rank(), t = threadIdx.x;
+  const int seg = (n + T.nb - 1) / T.nb;
+  VerletRun r;
+  r.lo = min(rank * seg, n);
+  r.hi = min(r.lo + seg, n);
+  r.H = ctl->hist_n;
+  r.cur = W.hcur;
+  r.cb = W.cb;
+  r.C = ctl->contacts;
+  r.fr = ctl->frame;
+  r.idx_ok = W.fresh != 0;
+  r.hm = hm_const(cfg);
+  const bool wall = !v_is_hm(W) && cfg.cylinder_enabled;
+  const d3 ax = wall ? soft_wall_axis(cfg) : mk3(0, 0, 0);
+  const double el = exp(-cfg.lin_damp * cfg.dt), ea = exp(-cfg.ang_damp * cfg.dt);
+  double invL[3] = {1.0, 1.0, 1.0};
+  for (int k = 0; k < 3; ++k)
+    if (V.box.L[k] > 0.0) invL[k] = 1.0 / V.box.L[k];
+  const DriftOut out{V.seg, V.all_pairs ? nullptr : V.ref, V.all_pairs || !W.near_cnt ? nullptr : V.ref2, V.skin};
+  if (!W.fresh) {  // segment records and displacement bounds of the first detection
+    double m = 0.0, m2 = 0.0;
+    for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+      const Seg s = make_seg(st, i);
+      V.seg[i] = s;
+      if (out.ref) m = fmax(m, seg_disp(s, out.ref, n, i, V.box));
+      if (out.ref2) m2 = fmax(m2, seg_disp(s, out.ref2, n, i, V.box));
+    }
+    v_publish_disp(V, m, m2, S.s);
+  }
+  // (every block has read the control words before the first one changes any)
+  if (!team_sync(T)) return false;
+  for (int step = 0; step < nsteps; ++step) {
+    const bool last = step == nsteps - 1;
+    // forces at t: with the first detection, or on the contacts in place
+    ++r.fr;
+    if (step == 0 && !W.fresh) {
+      if (!v_detect_eval(T, W, r, S, false)) return false;
+    } else {
+      const int c1 = W.off[r.cb][r.hi];
+      for (int c = W.off[r.cb][r.lo] + t; c < c1; c += blockDim.x) v_eval(W, r, c, W.hidx[r.cb][c], false);
+      if (rank == 0 && t == 0) ctl->contact_steps += r.C;
+    }
+    if (!team_sync(T)) return false;
+    // half kick and drift
+    {
+      const int added = *(volatile int*)&ctl->ins_n[r.fr & 1];
+      if (rank == 0 && t == 0) ctl->ins_n[(r.fr + 1) & 1] = 0;
+      double m = 0.0, m2 = 0.0;
+      for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+        d3 f{0, 0, 0}, tq{0, 0, 0};
+        if (st.inv_mass[i] > 0.0) v_body_sum(W, r, i, f, tq);
+        drift_rod(st, V.box, cfg, ax, wall, i, f, tq, out, invL, m, m2);
+      }
+      if (out.ref) v_publish_disp(V, m, m2, S.s);
+      if (added && !v_insert(T, W, r, S, added)) return false;
+    }
+    if (!team_sync(T)) return false;
+    // forces at t + dt
+    ++r.fr;
+    if (!v_detect_eval(T, W, r, S, last)) return false;
+    if (!team_sync(T)) return false;
+    // second half kick
+    {
+      const int added = *(volatile int*)&ctl->ins_n[r.fr & 1];
+      if (rank == 0 && t == 0) ctl->ins_n[(r.fr + 1) & 1] = 0;
+      int bad = 0;
+      for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+        d3 f{0, 0, 0}, tq{0, 0, 0};
+        v_body_sum(W, r, i, f, tq);
+        bad |= kick_rod(st, cfg, ax, wall, i, f, tq, el, ea);
+        if (last) {  // the forces that the call's last kick used
+          st.f.st(i, f);
+          st.tau.st(i, tq);
+        }
+      }
+      if (bad) atomicOr(&ctl->err, ERR_NONFINITE);
+      if (last && rank == 0) v_energy(W, r.C, S.s);
+      if (added && !v_insert(T, W, r, S, added)) return false;
+    }
+    if (!team_sync(T)) return false;
+    if (*(volatile int*)&ctl->err) return false;
+  }
+  // the table in the buffer it was found in, without entries past retention
+  if (!v_purge(T, W, r, S.s)) return false;
+  if (r.cur != W.hcur) {
+    const int hc = W.hcap, src = r.cur, dst = W.hcur;
+    for (int e = T.tid(); e < r.H; e += T.size()) {
+      W.hkey[dst][e] = W.hkey[src][e];
+      for (int k = 0; k < 3; ++k) W.hval[dst][(size_t)k * hc + e] = W.hval[src][(size_t)k * hc + e];
+      W.hframe[dst][e] = W.hframe[src][e];
+    }
+  }
+  if (rank == 0 && t == 0) {
+    ctl->hist_n = r.H;
+    ctl->frame = r.fr;
+  }
+  return true;
+}
+
+// A team's systems one after the other, each through all steps.
+__global__ void __launch_bounds__(kVBlock, 1) k_verlet_run(const VerletView* views, const TeamDesc* teams, int nteams,
+                                                           const int* members, int nsteps) {
+  __shared__ VerletSmem S;
+  __shared__ __align__(16) unsigned char view_words[sizeof(VerletView)];
+  int lo = 0, hi = nteams;  // last team with b0 <= blockIdx.x
+  while (hi - lo > 1) {
+    const int m = (lo + hi) >> 1;
+    if (teams[m].b0 <= (int)blockIdx.x) lo = m;
+    else hi = m;
+  }
+  const TeamDesc td = teams[lo];
+  if ((int)blockIdx.x < td.b0 || (int)blockIdx.x >= td.b0 + td.nb) return;
+  team_barriers_reset();
+  static_assert(sizeof(VerletView) % 8 == 0, "copied in 8-byte words");
+  for (int m = td.first; m < td.first + td.count; ++m) {
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&views[members ? members[m] : m]);
+    __syncthreads();  // the system before is done with its view
+    for (int k = threadIdx.x; k < (int)(sizeof(VerletView) / 8); k += blockDim.x)
+      reinterpret_cast<unsigned long long*>(view_words)[k] = src[k];
+    __syncthreads();
+    const VerletView& W = *reinterpret_cast<const VerletView*>(view_words);
+    const Team T{td.b0, td.nb, td.bar, &W.v.ctl->err,
+                 W.v.cfg.spin_limit > 0 ? (long long)W.v.cfg.spin_limit : kSpinLimit,
+                 W.v.cfg.test_absent_blocks > 0 ? (unsigned)W.v.cfg.test_absent_blocks : 0u};
+    if (*(volatile int*)&W.v.ctl->err == 0) v_run(T, W, nsteps, S);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Host side.
+// ---------------------------------------------------------------------------
+constexpr size_t kVSmem = kBuildQOff + 2 * sizeof(unsigned) * kBuildQ;
+
+VerletView make_verlet_view(rg_system* s) {
+  VerletView W;
+  std::memset(&W, 0, sizeof(W));
+  W.v = make_view(s);
+  const Detector& d = s->det;
+  W.near_cnt = d.near_cnt;
+  W.near_nbr = d.near_nbr;
+  W.extra = d.margin + d.near_skin;
+  W.delta = s->cfg.model == RG_MODEL_HERTZ_MINDLIN ? 0.0 : s->cfg.soft_delta;
+  W.cf = s->d_cf;
+  const History& H = s->hist;
+  for (int k = 0; k < 2; ++k) {
+    W.hkey[k] = H.key[k];
+    W.hval[k] = H.val[k];
+    W.hframe[k] = H.frame[k];
+    W.off[k] = s->vteam.off[k];
+    W.pb[k] = s->vteam.pb[k];
+    W.hidx[k] = s->vteam.hidx[k];
+  }
+  W.hcap = H.cap;
+  W.hcur = H.cur;
+  W.touched = H.touched;
+  W.touched_off = H.touched_off;
+  W.kept = H.kept;
+  W.kept_off = H.kept_off;
+  W.newval = H.newval;
+  W.head = s->vteam.head;
+  W.next = s->vteam.next;
+  W.ins = s->vteam.ins;
+  W.fresh = s->contacts_fresh == Fresh::kTeam ? 1 : 0;
+  W.cb = s->vteam.cb;
+  return W;
+}
+
+// Bookkeeping of a launch of nsteps steps: the contacts it leaves.
+void verlet_launched(rg_system* s, int nsteps) {
+  const int detections = nsteps + (s->contacts_fresh == Fresh::kTeam ? 0 : 1);
+  s->vteam.cb = (s->vteam.cb + detections) & 1;
+  s->contacts_fresh = Fresh::kTeam;
+}
+
+bool verlet_team_fits(const rg_system* s) {
+  const int m = s->cfg.model;
+  return (m == RG_MODEL_HARMONIC || m == RG_MODEL_HERTZ_MINDLIN) && !s->prof_on && s->vteam.head &&
+         s->n <= kVerletTeamRods;
+}
+
+void verlet_launch(const VerletView* views, const TeamDesc* teams, int nteams, const int* members, int grid, int nsteps,
+                   cudaStream_t st) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaFuncSetAttribute((const void*)k_verlet_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmem);
+    attr_set = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kVBlock);
+  cfg.dynamicSmemBytes = kVSmem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&views, &teams, &nteams, &members, &nsteps};
+  RGL cudaLaunchKernelExC(&cfg, (const void*)k_verlet_run, args);
+}
+
+void verlet_run_launch(rg_system* s, int nsteps) {
+  int nb = s->team_blocks > 0 ? s->team_blocks : (s->n + kVerletRodsPerBlock - 1) / kVerletRodsPerBlock;
+  if (nb > s->sm_count) nb = s->sm_count;
+  const VerletView W = make_verlet_view(s);
+  const TeamDesc td{0, nb, 0, 1, s->nsc.bar, nullptr};
+  cudaMemcpyAsync(s->vteam.view_dev, &W, sizeof(W), cudaMemcpyHostToDevice, s->stream);
+  cudaMemcpyAsync(s->nsc.team_dev, &td, sizeof(td), cudaMemcpyHostToDevice, s->stream);
+  cudaMemsetAsync(s->nsc.bar, 0, kTeamBarBytes, s->stream);
+  verlet_launch(static_cast<const VerletView*>(s->vteam.view_dev), static_cast<const TeamDesc*>(s->nsc.team_dev), 1,
+                nullptr, nb, nsteps, s->stream);
+  verlet_launched(s, nsteps);
+}
+
+// One allocation behind all arrays (each a multiple of 16 bytes).
+cudaError_t VerletTeam::alloc(int n, int ccap) {
+  const size_t rods = ((size_t)n + 4) / 4 * 4, cons = ((size_t)ccap + 3) / 4 * 4;
+  const size_t view = (sizeof(VerletView) + 15) / 16 * 16;
+  const cudaError_t e = cudaMalloc(&view_dev, view + sizeof(int) * (3 * rods + 6 * cons));
+  if (e) return e;
+  int* p = reinterpret_cast<int*>(static_cast<char*>(view_dev) + view);
+  for (int k = 0; k < 2; ++k) {
+    off[k] = p;
+    pb[k] = p + rods;
+    hidx[k] = p + rods + cons;
+    p += rods + 2 * cons;
+  }
+  head = p;
+  next = p + rods;
+  ins = next + cons;
+  return cudaSuccess;
+}
+void VerletTeam::free_() {
+  cudaFree(view_dev);
+  *this = VerletTeam();
+}
+
+}  // namespace rg
