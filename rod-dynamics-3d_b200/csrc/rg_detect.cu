@@ -224,7 +224,8 @@ __global__ void k_seg(State st, Seg* seg) {
 
 // Largest displacement bound |Δx| + h|Δu| since the last build; sets the
 // rebuild flag when it reaches skin/2.  With ref2 (near lists), the largest
-// bound since the last near-list build goes to ctl->near_disp.
+// bound since the last near-list build goes to ctl->near_disp (ref null: an
+// all-pairs box, whose lists hold every pair for good).
 __global__ void k_disp_check(State st, const Seg* seg, const double* ref, const double* ref2, Box box,
                              double skin, Ctl* ctl) {
   griddep_wait();
@@ -234,7 +235,7 @@ __global__ void k_disp_check(State st, const Seg* seg, const double* ref, const 
   const int n = st.n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     Seg s = seg[i];
-    m = fmax(m, seg_disp(s, ref, n, i, box));  // non-finite state: 1e300 forces a rebuild
+    if (ref) m = fmax(m, seg_disp(s, ref, n, i, box));  // non-finite state: 1e300 forces a rebuild
     if (ref2) m2 = fmax(m2, seg_disp(s, ref2, n, i, box));
   }
   m = warp_max(m);
@@ -250,8 +251,8 @@ __global__ void k_disp_check(State st, const Seg* seg, const double* ref, const 
     v = warp_max(v);
     v2 = warp_max(v2);
     if (threadIdx.x == 0) {
-      atomic_max_nonneg(&ctl->maxdisp, v);
-      if (v >= 0.5 * skin * (1.0 - 1e-9)) atomicExch(&ctl->rebuild, 1);
+      if (ref) atomic_max_nonneg(&ctl->maxdisp, v);
+      if (ref && v >= 0.5 * skin * (1.0 - 1e-9)) atomicExch(&ctl->rebuild, 1);
       if (ref2) atomic_max_nonneg(&ctl->near_disp, v2);
     }
   }
@@ -564,17 +565,25 @@ cudaError_t detector_alloc(rg_system* s) {
   if ((e = cudaMalloc(&d.hit_off, sizeof(int) * (n + 1)))) return e;
   if ((e = cudaMalloc(&d.hit_mask, sizeof(unsigned long long) * (size_t)n * d.mask_words))) return e;
   if ((e = cudaMemset(d.nbr_cnt, 0, sizeof(int) * n))) return e;
-  if (c.model != RG_MODEL_NSC && !d.all_pairs && check_near_lists(c)) {
-    // near lists of the multi-kernel detection (the soft / HM step)
-    d.near_skin = (c.near_skin_pct > 0 ? 0.01 * c.near_skin_pct : 0.05) * d.skin;
+  // Near lists of the soft / HM detection.  In an all-pairs box a pair's
+  // minimum image may change while they are valid: that is harmless when
+  // half the box exceeds the contact reach by the near skin (a pair whose
+  // image flips is then out of reach in both images for as long as the lists
+  // hold), so they serve such boxes too, with a wider skin, as their build
+  // walks every pair (583 rods, AR 20, box side 2.45: 250 us a step over the
+  // whole lists).  Narrower boxes test every pair.
+  const double near_skin = (c.near_skin_pct > 0 ? 0.01 * c.near_skin_pct : (d.all_pairs ? 0.5 : 0.05)) * d.skin;
+  bool near_ok = check_near_lists(c);
+  for (int k = 0; k < 3 && d.all_pairs; ++k)
+    if (0.5 * s->box.L[k] <= 2.0 * (hmax + rmax) + d.margin + near_skin) near_ok = false;
+  if (c.model != RG_MODEL_NSC && near_ok) {
+    d.near_skin = near_skin;
     if ((e = cudaMalloc(&d.near_cnt, sizeof(int) * n))) return e;
     if ((e = cudaMalloc(&d.near_nbr, sizeof(int) * (size_t)n * d.maxnb))) return e;
     if ((e = cudaMalloc(&d.ref2, sizeof(double) * 6 * (size_t)n))) return e;
   }
   if (c.model == RG_MODEL_NSC) {
-    // all-pairs boxes rebuild the near list from every pair: a wider near
-    // skin makes those rebuilds rare
-    d.near_skin = (c.near_skin_pct > 0 ? 0.01 * c.near_skin_pct : (d.all_pairs ? 0.5 : 0.05)) * d.skin;
+    d.near_skin = near_skin;
     if ((e = cudaMalloc(&d.near, sizeof(int2) * (size_t)n * d.maxnb))) return e;
     if ((e = cudaMalloc(&d.ref2, sizeof(double) * 6 * (size_t)n))) return e;
     if ((e = cudaMalloc(&d.moved, (size_t)n))) return e;
@@ -616,8 +625,9 @@ void detect_launch(rg_system* s, double delta, bool check_rebuild, bool seg_read
   const bool near = d.near_cnt != nullptr;
   if (!seg_ready) {
     RGL launch_dep(k_seg, g, bs, st, s->st, d.seg);
-    if (check_rebuild && !d.all_pairs) {
-      RGL launch_dep(k_disp_check, g, bs, st, s->st, d.seg, d.ref, near ? d.ref2 : nullptr, s->box, d.skin, ctl);
+    if (check_rebuild && (!d.all_pairs || near)) {
+      const double* ref = d.all_pairs ? nullptr : d.ref;
+      RGL launch_dep(k_disp_check, g, bs, st, s->st, d.seg, ref, near ? d.ref2 : nullptr, s->box, d.skin, ctl);
     }
   }
   // --- rebuild: every kernel below returns at once unless ctl->rebuild ---

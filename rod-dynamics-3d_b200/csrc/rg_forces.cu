@@ -203,7 +203,7 @@ __global__ void k_soft_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
     const int a = io.ca[c], b = io.cb[c];
     const int hf = hist_find(io, a, b, H);
     const d3 old = hf >= 0 ? mk3(io.hval[hf], io.hval[io.hcap + hf], io.hval[2 * io.hcap + hf]) : mk3(0, 0, 0);
-    const PairForce p = soft_pair(st, cfg, a, b, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
+    const PairForce p = soft_pair(load_pair(st, a, b), cfg, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
                                   io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, true);
     st_pair(io, c, hf, p);
   }
@@ -219,7 +219,7 @@ __global__ void k_hm_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
     const int a = io.ca[c], b = io.cb[c];
     const int hf = hist_find(io, a, b, H);
     const d3 old = hf >= 0 ? mk3(io.hval[hf], io.hval[io.hcap + hf], io.hval[2 * io.hcap + hf]) : mk3(0, 0, 0);
-    const PairForce p = hm_pair(st, cfg, k, a, b, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
+    const PairForce p = hm_pair(load_pair(st, a, b), cfg, k, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
                                 io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, true);
     st_pair(io, c, hf, p);
   }

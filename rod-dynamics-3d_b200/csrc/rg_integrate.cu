@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
     if (st.inv_mass[i] > 0.0) body_sum(off, ent, cf, ccap, i, f, t);
     drift_rod(st, box, cfg, ax, wall, i, f, t, o, invL, m, m2);
   }
-  if (!o.ref) return;
+  if (!o.ref && !o.ref2) return;
   m = warp_max(m);
   m2 = warp_max(m2);
   if ((threadIdx.x & 31) == 0) {
@@ -55,8 +55,8 @@ __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
     v = warp_max(v);
     v2 = warp_max(v2);
     if (threadIdx.x == 0) {
-      atomic_max_nonneg(&ctl->maxdisp, v);
-      if (v >= 0.5 * o.skin * (1.0 - 1e-9)) atomicExch(&ctl->rebuild, 1);
+      if (o.ref) atomic_max_nonneg(&ctl->maxdisp, v);
+      if (o.ref && v >= 0.5 * o.skin * (1.0 - 1e-9)) atomicExch(&ctl->rebuild, 1);
       if (o.ref2) atomic_max_nonneg(&ctl->near_disp, v2);
     }
   }
@@ -124,7 +124,7 @@ void reduce_drift_launch(rg_system* s, bool wall, HistFinish hf) {
   DriftOut o;
   o.seg = d.seg;
   o.ref = d.all_pairs ? nullptr : d.ref;
-  o.ref2 = (d.all_pairs || !d.near_cnt) ? nullptr : d.ref2;
+  o.ref2 = d.near_cnt ? d.ref2 : nullptr;
   o.skin = d.skin;
   RGL launch_dep(k_reduce_drift, body_grid(s), 256, s->stream, s->st, s->box, s->cfg, s->csr.off, s->csr.ent,
                                                           s->d_cf, s->ccap, wall ? 1 : 0, o, hf, s->d_ctl);

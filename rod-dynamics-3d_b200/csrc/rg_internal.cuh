@@ -90,7 +90,7 @@ struct Detector {
   double near_skin = 0;
   // near lists of the multi-kernel detection (soft / HM models): per rod,
   // the ascending list entries within reach + near_skin (same layout as
-  // nbr); null when the full lists are used (NSC models, all-pairs boxes)
+  // nbr); null when the full lists are used (NSC models, very narrow boxes)
   int* near_cnt = nullptr;        // n
   int* near_nbr = nullptr;        // n * maxnb
   // 1: rod moved (position projection or periodic wrap) since the

@@ -64,39 +64,59 @@ __device__ inline int v_find(const VerletView& W, const VerletRun& r, int a, int
   return (p < r.H && W.hkey[r.cur][p] == k) ? p : -1;
 }
 
-// Force of contact c with table entry f (-1: none); updates the entry, or
-// lists the pair for insertion.  energy: the contact's potential energy is
-// wanted (of a call only the last evaluation's sum is kept).
-__device__ inline void v_eval(const VerletView& W, const VerletRun& r, int c, int f, bool energy) {
-  const NscView& V = W.v;
-  const Contacts& con = V.con;
-  const int a = con.a[c], b = con.b[c], hc = W.hcap, cc = V.ccap;
-  double* hv = W.hval[r.cur];
-  long long* hf = W.hframe[r.cur];
+// Geometry of a contact.
+struct VContact {
+  d3 pa, pb, n, sh;
+  double dist, surf;
+};
+// Force of contact c of bodies in `in`, with table entry f (-1: none) whose
+// value and frame are `old`, `frame`; updates the entry, or lists the pair
+// for insertion.  energy: the contact's potential energy is wanted (of a call
+// only the last evaluation's sum is kept).
+__device__ inline void v_eval(const VerletView& W, const VerletRun& r, int c, const PairIn& in, const VContact& g, int f,
+                              d3 old, long long frame, bool energy) {
+  const int hc = W.hcap, cc = W.v.ccap;
   const bool hm = v_is_hm(W);
-  d3 old{0, 0, 0};
   // an entry past its retention was dropped by the evaluation before this one
-  if (f >= 0 && (!hm || r.fr - hf[f] <= 5)) old = mk3(hv[f], hv[hc + f], hv[2 * (size_t)hc + f]);
-  const d3 pa{con.comp(0)[c], con.comp(1)[c], con.comp(2)[c]}, pb{con.comp(3)[c], con.comp(4)[c], con.comp(5)[c]};
-  const d3 nrm{con.comp(6)[c], con.comp(7)[c], con.comp(8)[c]}, sh{con.comp(9)[c], con.comp(10)[c], con.comp(11)[c]};
-  const double dist = con.comp(12)[c], hs = con.comp(13)[c];
-  const PairForce p = hm ? hm_pair(V.st, V.cfg, r.hm, a, b, pa, pb, nrm, sh, dist, hs, old, energy)
-                         : soft_pair(V.st, V.cfg, a, b, pa, pb, nrm, sh, dist, hs, old, energy);
+  if (f < 0 || (hm && r.fr - frame > 5)) old = mk3(0, 0, 0);
+  const PairForce p = hm ? hm_pair(in, W.v.cfg, r.hm, g.pa, g.pb, g.n, g.sh, g.dist, g.surf, old, energy)
+                         : soft_pair(in, W.v.cfg, g.pa, g.pb, g.n, g.sh, g.dist, g.surf, old, energy);
   store_addends(W.cf, cc, c, p);
   if (energy) W.cf[12 * (size_t)cc + c] = p.pe;
   int added = 0;
   if (p.touch) {
     if (f >= 0) {
+      double* hv = W.hval[r.cur];
       hv[f] = p.hist.x; hv[hc + f] = p.hist.y; hv[2 * (size_t)hc + f] = p.hist.z;
-      hf[f] = r.fr;
+      W.hframe[r.cur][f] = r.fr;
     } else {
       W.newval[c] = p.hist.x; W.newval[cc + c] = p.hist.y; W.newval[2 * (size_t)cc + c] = p.hist.z;
-      W.ins[atomicAdd(&V.ctl->ins_n[r.fr & 1], 1)] = c;
+      W.ins[atomicAdd(&W.v.ctl->ins_n[r.fr & 1], 1)] = c;
       added = 1;
     }
   }
   W.touched[c] = added;
   W.hidx[r.cb][c] = f;
+}
+__device__ inline d3 v_old(const VerletView& W, const VerletRun& r, int f, long long& frame) {
+  if (f < 0) return mk3(0, 0, 0);
+  const double* hv = W.hval[r.cur];
+  const int hc = W.hcap;
+  frame = W.hframe[r.cur][f];
+  return mk3(hv[f], hv[hc + f], hv[2 * (size_t)hc + f]);
+}
+// Evaluation r.fr of a contact already in place (every load before the first
+// store: the loads then overlap).
+__device__ inline void v_eval_again(const VerletView& W, const VerletRun& r, int c) {
+  const Contacts& con = W.v.con;
+  const int f = W.hidx[r.cb][c], a = con.a[c], b = con.b[c];
+  const VContact g{{con.comp(0)[c], con.comp(1)[c], con.comp(2)[c]}, {con.comp(3)[c], con.comp(4)[c], con.comp(5)[c]},
+                   {con.comp(6)[c], con.comp(7)[c], con.comp(8)[c]}, {con.comp(9)[c], con.comp(10)[c], con.comp(11)[c]},
+                   con.comp(12)[c], con.comp(13)[c]};
+  const PairIn in = load_pair(W.v.st, a, b);
+  long long frame = 0;
+  const d3 old = v_old(W, r, f, frame);
+  v_eval(W, r, c, in, g, f, old, frame, false);
 }
 
 // Removes the entries past their retention (Hertz-Mindlin) after evaluation
@@ -130,7 +150,7 @@ __device__ __noinline__ bool v_purge(const Team& T, const VerletView& W, VerletR
 // block past a barrier since); the next evaluation is behind another barrier.
 __device__ __noinline__ bool v_insert(const Team& T, const VerletView& W, VerletRun& r, VerletSmem& S, int added) {
   const NscView& V = W.v;
-  const int tid = T.tid(), TS = T.size(), t = threadIdx.x, hc = W.hcap, cc = V.ccap;
+  const int t = threadIdx.x, hc = W.hcap, cc = V.ccap;
   if (r.H + added > hc - hc / 4 && !v_purge(T, W, r, S.s)) return false;
   if (r.H + added > hc) {
     if (T.rank() == 0 && t == 0) atomicOr(&V.ctl->err, ERR_HIST_CAP);
@@ -154,7 +174,10 @@ __device__ __noinline__ bool v_insert(const Team& T, const VerletView& W, Verlet
   } else if (!team_excl_scan(T, W.touched, W.touched_off, r.C, V.blk, S.s)) {
     return false;
   }
-  for (int e = tid; e < r.H; e += TS) {
+  // each block an equal range (a table of a few hundred entries would
+  // otherwise be moved by the first block alone)
+  const int he = (r.H + T.nb - 1) / T.nb, ce = (r.C + T.nb - 1) / T.nb, rank = T.rank();
+  for (int e = rank * he + t; e < min((rank + 1) * he, r.H); e += blockDim.x) {
     const unsigned long long k = ok[e];
     int before;
     if (chip) {
@@ -173,7 +196,7 @@ __device__ __noinline__ bool v_insert(const Team& T, const VerletView& W, Verlet
     for (int j = 0; j < 3; ++j) W.hval[dst][(size_t)j * hc + p] = W.hval[src][(size_t)j * hc + e];
     W.hframe[dst][p] = W.hframe[src][e];
   }
-  for (int c = tid; c < r.C; c += TS) {
+  for (int c = rank * ce + t; c < min((rank + 1) * ce, r.C); c += blockDim.x) {
     const int f = W.hidx[r.cb][c];
     const bool in = W.touched[c];
     if (!in && f < 0) continue;
@@ -288,10 +311,11 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
   }
   const int* cnt = near ? W.near_cnt : V.nbr_cnt;
   const int* nbr = near ? W.near_nbr : V.nbr;
-  // four lanes a rod while they fill the block in one round
-  const int pre = near ? 0 : (V.all_pairs ? 2 : 1);
-  const int mine = 4 * (r.hi - r.lo) <= (int)blockDim.x || !near ? v_count<4>(W, r, cnt, nbr, pre)
-                                                                : v_count<1>(W, r, cnt, nbr, pre);
+  // lanes a rod: as many as one round of the block has (whole lists: four)
+  const int rods = r.hi - r.lo, threads = (int)blockDim.x, pre = near ? 0 : (V.all_pairs ? 2 : 1);
+  const int mine = 4 * rods <= threads || !near ? v_count<4>(W, r, cnt, nbr, pre)
+                   : 2 * rods <= threads        ? v_count<2>(W, r, cnt, nbr, pre)
+                                                : v_count<1>(W, r, cnt, nbr, pre);
   const int bsum = block_reduce_sum_i(mine, S.s.red_i);
   if (t == 0) V.blk[rank] = bsum;
   if (!team_sync(T)) return false;
@@ -331,22 +355,31 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
   r.cb = cb;
   __syncthreads();
   for (int c = prefix + t; c < run; c += blockDim.x) {
+    // every load that needs no result comes before the first store
     const int a = V.con.a[c], b = V.con.b[c];
     const Seg A = V.seg[a], B = V.seg[b];
-    const Narrow nr = narrow_pair(A, B, V.box);
-    write_contact(V.con, c, a, b, A.r + B.r, nr);
-    W.pb[cb][c] = b;
-    W.next[c] = atomicExch(&W.head[b], c);
+    const PairIn in = load_pair(V.st, a, b);
     int f = -1;
     bool known = false;
-    if (r.idx_ok)
-      for (int k = W.off[ob][a]; k < W.off[ob][a + 1]; ++k)
+    if (r.idx_ok) {
+      const int e = W.off[ob][a + 1];
+      for (int k = W.off[ob][a]; k < e; ++k)
         if (W.pb[ob][k] == b) {
           f = W.hidx[ob][k];
           known = true;
         }
+    }
     if (!known && r.H > 0) f = v_find(W, r, a, b);
-    v_eval(W, r, c, f, energy);
+    long long frame = 0;
+    const d3 old = v_old(W, r, f, frame);
+    const Narrow nr = narrow_pair(A, B, V.box);
+    const double dist = sqrt(nr.d2);
+    const d3 diff = nr.pb - nr.pa;
+    const VContact g{nr.pa, nr.pb, dist > 1e-10 ? diff / dist : mk3(1, 0, 0), nr.sh, dist, A.r + B.r};
+    W.next[c] = atomicExch(&W.head[b], c);
+    W.pb[cb][c] = b;
+    write_contact(V.con, c, a, b, g.surf, nr);
+    v_eval(W, r, c, in, g, f, old, frame, energy);
   }
   r.idx_ok = true;
   return true;
@@ -395,7 +428,7 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
   double invL[3] = {1.0, 1.0, 1.0};
   for (int k = 0; k < 3; ++k)
     if (V.box.L[k] > 0.0) invL[k] = 1.0 / V.box.L[k];
-  const DriftOut out{V.seg, V.all_pairs ? nullptr : V.ref, V.all_pairs || !W.near_cnt ? nullptr : V.ref2, V.skin};
+  const DriftOut out{V.seg, V.all_pairs ? nullptr : V.ref, W.near_cnt ? V.ref2 : nullptr, V.skin};
   if (!W.fresh) {  // segment records and displacement bounds of the first detection
     double m = 0.0, m2 = 0.0;
     for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
@@ -416,7 +449,7 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
       if (!v_detect_eval(T, W, r, S, false)) return false;
     } else {
       const int c1 = W.off[r.cb][r.hi];
-      for (int c = W.off[r.cb][r.lo] + t; c < c1; c += blockDim.x) v_eval(W, r, c, W.hidx[r.cb][c], false);
+      for (int c = W.off[r.cb][r.lo] + t; c < c1; c += blockDim.x) v_eval_again(W, r, c);
       if (rank == 0 && t == 0) ctl->contact_steps += r.C;
     }
     if (!team_sync(T)) return false;
@@ -430,7 +463,7 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
         if (st.inv_mass[i] > 0.0) v_body_sum(W, r, i, f, tq);
         drift_rod(st, V.box, cfg, ax, wall, i, f, tq, out, invL, m, m2);
       }
-      if (out.ref) v_publish_disp(V, m, m2, S.s);
+      if (out.ref || out.ref2) v_publish_disp(V, m, m2, S.s);
       if (added && !v_insert(T, W, r, S, added)) return false;
     }
     if (!team_sync(T)) return false;

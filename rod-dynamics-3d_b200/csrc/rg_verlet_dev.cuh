@@ -34,11 +34,21 @@ __device__ inline void store_addends(double* cf, int cc, int c, const PairForce&
   cf[9 * cc + c] = p.tb.x; cf[10 * cc + c] = p.tb.y; cf[11 * cc + c] = p.tb.z;
 }
 
+// What the force laws read of the two bodies.
+struct PairIn {
+  d3 xa, xb, va, wa, vb, wb;
+  double ra, rb, ma, mb;  // radii and masses (0: static body)
+};
+__device__ inline PairIn load_pair(const State& st, int a, int b) {
+  return PairIn{st.x.ld(a), st.x.ld(b), st.v.ld(a), st.w.ld(a), st.v.ld(b), st.w.ld(b),
+                st.r[a],    st.r[b],    st.mass[a], st.mass[b]};
+}
+
 // Soft penalty contact (SoftContactSolver::computeForces,
 // src/physics/soft_contact.cpp:80-486); old: the pair's history value;
 // energy: the potential energy is wanted.
-__device__ inline PairForce soft_pair(const State& st, const rg_config& cfg, int a, int b, d3 pa, d3 pb, d3 nrm,
-                                      d3 sh, double dist, double hs, d3 old, bool energy) {
+__device__ inline PairForce soft_pair(const PairIn& in, const rg_config& cfg, d3 pa, d3 pb, d3 nrm, d3 sh, double dist,
+                                      double hs, d3 old, bool energy) {
   const double dt = cfg.dt;
   const double K1 = 15.0 / cfg.soft_delta;
   // potentialGradient / potentialEnergy
@@ -58,11 +68,10 @@ __device__ inline PairForce soft_pair(const State& st, const rg_config& cfg, int
   double fm = -cfg.soft_k_scaler * grad;
   d3 fa = nrm * (-fm);
   d3 fb = nrm * fm;
-  d3 xa = st.x.ld(a), xb = st.x.ld(b);
-  d3 ra = pa - xa;
-  d3 rb = pb - (xb + sh);
-  d3 va = st.v.ld(a) + cross(st.w.ld(a), ra);
-  d3 vb = st.v.ld(b) + cross(st.w.ld(b), rb);
+  d3 ra = pa - in.xa;
+  d3 rb = pb - (in.xb + sh);
+  d3 va = in.va + cross(in.wa, ra);
+  d3 vb = in.vb + cross(in.wb, rb);
   d3 vrel = va - vb;
   if (cfg.soft_damping > 1e-9) {
     double vn = dot(vrel, nrm);
@@ -93,8 +102,8 @@ __device__ inline PairForce soft_pair(const State& st, const rg_config& cfg, int
         fra = ft;
       } else if (cfg.soft_friction_mode == RG_FRICTION_KARNOPP) {
         if (vtm < cfg.soft_vel_deadband) {
-          double ma = st.inv_mass[a] > 0 ? st.mass[a] : 0.0;
-          double mb = st.inv_mass[b] > 0 ? st.mass[b] : 0.0;
+          const double ma = in.ma;
+          const double mb = in.mb;
           double meff = 0;
           if (ma > 0 && mb > 0) meff = (ma * mb) / (ma + mb);
           else if (ma > 0) meff = ma;
@@ -143,10 +152,10 @@ __device__ inline HmConst hm_const(const rg_config& cfg) {
   }
   return k;
 }
-__device__ inline PairForce hm_pair(const State& st, const rg_config& cfg, const HmConst& k, int a, int b, d3 pa,
-                                    d3 pb, d3 nrm, d3 sh, double dist, double hs, d3 old, bool energy) {
+__device__ inline PairForce hm_pair(const PairIn& in, const rg_config& cfg, const HmConst& k, d3 pa, d3 pb, d3 nrm,
+                                    d3 sh, double dist, double hs, d3 old, bool energy) {
   const double dt = cfg.dt, Es = k.Es, Gs = k.Gs, gam = k.gam;
-  double ra_ = st.r[a], rb_ = st.r[b], ma = st.mass[a], mb = st.mass[b];
+  const double ra_ = in.ra, rb_ = in.rb, ma = in.ma, mb = in.mb;
   double delta = hs - dist;
   double Rs = (ra_ * rb_) / (ra_ + rb_);
   double ms = (ma * mb) / (ma + mb);
@@ -155,12 +164,11 @@ __device__ inline PairForce hm_pair(const State& st, const rg_config& cfg, const
   double sqR = sqrt(smax(Rs, 0.0));
   double kn = (4.0 / 3.0) * Es * sqR * sqd;
   double Fel = kn * sd * sqd;
-  d3 xa = st.x.ld(a), xb = st.x.ld(b);
-  d3 ra = pa - xa;
-  d3 rb = pb - (xb + sh);
-  d3 wa = st.w.ld(a), wb = st.w.ld(b);
-  d3 va = st.v.ld(a) + cross(wa, ra);
-  d3 vb = st.v.ld(b) + cross(wb, rb);
+  d3 ra = pa - in.xa;
+  d3 rb = pb - (in.xb + sh);
+  const d3 wa = in.wa, wb = in.wb;
+  d3 va = in.va + cross(wa, ra);
+  d3 vb = in.vb + cross(wb, rb);
   d3 vrel = vb - va;
   double vn = dot(vrel, nrm);
   double Cn = gam * 2.0 * sqrt(ms * kn);
@@ -282,10 +290,8 @@ __device__ inline void drift_rod(const State& st, const Box& box, const rg_confi
     const double rf[6] = {ref[i], ref[n + i], ref[2 * n + i], ref[3 * n + i], ref[4 * n + i], ref[5 * n + i]};
     return disp_from(sg, rf, box, invL);
   };
-  if (o.ref) {
-    m = fmax(m, bound(o.ref));
-    if (o.ref2) m2 = fmax(m2, bound(o.ref2));
-  }
+  if (o.ref) m = fmax(m, bound(o.ref));
+  if (o.ref2) m2 = fmax(m2, bound(o.ref2));
 }
 
 // Second half kick of rod i (integrateSecondHalf, integrator.cpp:136-159);

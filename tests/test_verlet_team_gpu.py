@@ -42,7 +42,8 @@ SOFT = dict(model="harmonic", dt=1e-4, soft_damping=0.3, soft_friction_mode="cun
 
 @pytest.mark.parametrize("model", [HM, SOFT], ids=["hm", "cundall"])
 @pytest.mark.parametrize("n,d,phi,squeeze,team,extra", [
-    (37, 0.1, 0.02, 0.8, 0, {}),                        # every pair listed, one partly filled block
+    (37, 0.1, 0.02, 0.8, 0, {}),                        # every pair listed and tested, one partly filled block
+    (580, 0.05, 0.08, 0.9, 0, {}),                      # every pair listed, near lists drawn from them
     (300, 0.1, 0.05, 0.9, 1, dict(pbc_enabled=0)),      # open box, one block
     (1500, 0.1, 0.10, 0.95, 3, dict(skin=0.02)),        # 500 rods a block, lists rebuilt in the call
     (1500, 0.1, 0.10, 0.95, 0, dict(near_skin_pct=-1)),  # full lists instead of near lists
@@ -61,6 +62,21 @@ def test_persistent_equals_multi_kernel(model, n, d, phi, squeeze, team, extra):
         contacts.add(st["contacts"])
         _same(a, b)
     assert st["contacts"] > 0 and (n < 300 or len(contacts) > 1)
+
+
+@pytest.mark.parametrize("model", [HM, SOFT], ids=["hm", "cundall"])
+def test_near_lists_of_an_all_pairs_box_lose_no_contact(model):
+    # half the box (1.22) is just above the contact reach plus the near skin;
+    # fast rods: minimum images flip while the near lists are valid
+    sc = packed_scene(580, d=0.05, phi=0.08, seed=54, squeeze=0.9, sigma_v=5.0, sigma_w=5.0)
+    assert 2.42 < sc["side"] < 2.5
+    a, b = _load(sc, **model), _load(sc, near_skin_pct=-1, **model)
+    near = 0
+    for _ in range(4):
+        near += a.step(80)["near_rebuilds"]
+        b.step(80)
+        _same(a, b)
+    assert near > 1
 
 
 def test_switching_between_the_forms():
