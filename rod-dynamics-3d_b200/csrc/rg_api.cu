@@ -577,15 +577,17 @@ namespace rg {
 // drift, forces at t + dt, second half kick.  Each evaluation starts from
 // zero forces (integrateSecondHalf clears them for the next frame,
 // integrator.cpp:156-158, and the step clears them again before the second
-// evaluation); the per-body sums are fused into the two kick kernels.
-static void verlet_step(rg_system* s) {
+// evaluation); the per-body sums are fused into the two kick kernels.  last:
+// the call ends with this step (forces and potential energy are kept).
+static void verlet_step(rg_system* s, bool last) {
   force_eval_launch(s, EvalTail::kHalfPos);  // forces at t (reuses fresh contacts), kick and drift
   s->contacts_fresh = Fresh::kNo;
-  force_eval_launch(s, EvalTail::kSecondHalf, true);  // forces at t + dt, second kick
+  force_eval_launch(s, EvalTail::kSecondHalf, true, last);  // forces at t + dt, second kick
   s->contacts_fresh = Fresh::kCsr;  // positions unchanged until the next drift
 }
 
-// Captures one Verlet step (entered with fresh contacts) as a CUDA graph.
+// Captures one Verlet step (entered with fresh contacts, not a call's last) as
+// a CUDA graph.
 // Every launch of the step is decided on the host from state that a whole
 // step leaves as it found it (fresh contacts, the history ping-pong index),
 // so the same graph serves every step until buffers are reallocated.
@@ -601,7 +603,7 @@ static bool capture_verlet_step(rg_system* s) {
     cudaGetLastError();
     return false;
   }
-  verlet_step(s);
+  verlet_step(s, false);
   cudaError_t e = cudaStreamEndCapture(s->stream, &g);
   s->vgraph_kernels = g_launches - l0;
   g_launches = l0;  // counted when the graph runs
@@ -632,20 +634,21 @@ void launch_steps(rg_system* s, int nsteps) {
   }
   int k = 0;
   if (nsteps > 0 && s->contacts_fresh != Fresh::kCsr) {  // the first evaluation detects
-    verlet_step(s);
+    verlet_step(s, nsteps == 1);
     k = 1;
   }
-  // The rest replay one captured step (stage timers need the plain launches).
-  if (nsteps - k >= 2 && !s->prof_on) {
+  // The steps before the last replay one captured step (stage timers need the
+  // plain launches).
+  if (nsteps - k >= 3 && !s->prof_on) {
     bool ok = s->vgraph && s->vgraph_gen == s->buf_gen && s->vgraph_cur == s->hist.cur;
     if (!ok) ok = capture_verlet_step(s);
     if (ok)
-      for (; k < nsteps; ++k) {
+      for (; k < nsteps - 1; ++k) {
         RGL cudaGraphLaunch(s->vgraph, s->stream);
         g_launches += s->vgraph_kernels - 1;
       }
   }
-  for (; k < nsteps; ++k) verlet_step(s);
+  for (; k < nsteps; ++k) verlet_step(s, k == nsteps - 1);
 }
 
 // Grows the buffer named by the error bits.  Returns false if nothing grew.

@@ -467,6 +467,7 @@ __device__ inline int narrow_count_rod(int i, const Seg* seg, const double* inv_
                                        double delta, const int* nbr_cnt, const int* nbr, int maxnb,
                                        int words, unsigned long long* mask) {
   int cnt = nbr_cnt[i];
+  if (cnt == 0) return 0;  // (half of a sparse system's rods: no record read)
   const int* list = nbr + (size_t)i * maxnb;
   Seg A = seg[i];
   bool a_static = !(inv_mass[i] > 0.0);

@@ -194,7 +194,7 @@ __device__ inline void st_pair(const ForceIO& io, int c, int hf, const PairForce
   io.pe[c] = p.pe;
 }
 
-__global__ void k_soft_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
+__global__ void k_soft_forces(State st, rg_config cfg, ForceIO io, int energy, Ctl* ctl) {
   griddep_wait();
   if (ctl->err) return;
   const int C = ctl->contacts, H = ctl->hist_n;
@@ -204,12 +204,12 @@ __global__ void k_soft_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
     const int hf = hist_find(io, a, b, H);
     const d3 old = hf >= 0 ? mk3(io.hval[hf], io.hval[io.hcap + hf], io.hval[2 * io.hcap + hf]) : mk3(0, 0, 0);
     const PairForce p = soft_pair(load_pair(st, a, b), cfg, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
-                                  io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, true);
+                                  io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, energy != 0);
     st_pair(io, c, hf, p);
   }
 }
 
-__global__ void k_hm_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
+__global__ void k_hm_forces(State st, rg_config cfg, ForceIO io, int energy, Ctl* ctl) {
   griddep_wait();
   if (ctl->err) return;
   const int C = ctl->contacts, H = ctl->hist_n;
@@ -220,7 +220,7 @@ __global__ void k_hm_forces(State st, rg_config cfg, ForceIO io, Ctl* ctl) {
     const int hf = hist_find(io, a, b, H);
     const d3 old = hf >= 0 ? mk3(io.hval[hf], io.hval[io.hcap + hf], io.hval[2 * io.hcap + hf]) : mk3(0, 0, 0);
     const PairForce p = hm_pair(load_pair(st, a, b), cfg, k, ldc(io, 0, c), ldc(io, 3, c), ldc(io, 6, c), ldc(io, 9, c),
-                                io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, true);
+                                io.g[(size_t)12 * io.ccap + c], io.g[(size_t)13 * io.ccap + c], old, energy != 0);
     st_pair(io, c, hf, p);
   }
 }
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kPeThreads) k_pe_sum(const double* pe, Ctl* ct
 //                at t are consumed there, not stored);
 //   kSecondHalf: reduction fused with the second half kick, then the
 //                potential energy.
-void force_eval_launch(rg_system* s, EvalTail tail, bool seg_ready) {
+void force_eval_launch(rg_system* s, EvalTail tail, bool seg_ready, bool results) {
   const rg_config& c = s->cfg;
   const bool hm = c.model == RG_MODEL_HERTZ_MINDLIN;
   cudaStream_t st = s->stream;
@@ -300,10 +300,11 @@ void force_eval_launch(rg_system* s, EvalTail tail, bool seg_ready) {
   io.hkey = H.key[cur]; io.kept = H.kept; io.hval = H.val[cur]; io.hcap = H.cap;
   io.newval = H.newval; io.touched = H.touched; io.cf = s->d_cf;
   io.pe = s->d_cf + 12 * (size_t)s->ccap;
+  const int energy = results && tail != EvalTail::kHalfPos ? 1 : 0;
   if (hm) {
-    RGL launch_dep(k_hm_forces, gc, bs, st, s->st, c, io, s->d_ctl);
+    RGL launch_dep(k_hm_forces, gc, bs, st, s->st, c, io, energy, s->d_ctl);
   } else {
-    RGL launch_dep(k_soft_forces, gc, bs, st, s->st, c, io, s->d_ctl);
+    RGL launch_dep(k_soft_forces, gc, bs, st, s->st, c, io, energy, s->d_ctl);
   }
   // history merge
   s->scan.run2(H.touched, H.touched_off, &s->d_ctl->contacts, H.kept, H.kept_off, &s->d_ctl->hist_n,
@@ -320,7 +321,7 @@ void force_eval_launch(rg_system* s, EvalTail tail, bool seg_ready) {
     return;
   }
   if (tail == EvalTail::kSecondHalf) {
-    reduce_kick_launch(s, wall, hf);
+    reduce_kick_launch(s, wall, hf, results);
   } else {
     RGL launch_dep(k_hist_finish, 1, 1, st, H.touched_off, H.kept_off, s->d_ctl);
     RGL launch_dep(k_body_reduce, grid_for(s->n, bs), bs, st, s->st, s->csr.off, s->csr.ent, s->d_cf, s->ccap,
@@ -329,7 +330,9 @@ void force_eval_launch(rg_system* s, EvalTail tail, bool seg_ready) {
       RGL launch_dep(k_soft_wall, grid_for(s->n, bs), bs, st, s->st, c, s->d_ctl);
     }
   }
-  RGL launch_dep(k_pe_sum, 1, kPeThreads, st, static_cast<const double*>(io.pe), s->d_ctl);
+  if (energy) {
+    RGL launch_dep(k_pe_sum, 1, kPeThreads, st, static_cast<const double*>(io.pe), s->d_ctl);
+  }
 }
 
 }  // namespace rg

@@ -64,10 +64,12 @@ __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
 
 // Velocity Verlet, second half (integrateSecondHalf, integrator.cpp:136-159):
 // the forces at t + dt summed per body (contact addends + soft wall) and
-// kept in f, tau; then the half kick, damping and the angular-speed clamp.
+// kept in f, tau when a call ends on them (48 B a rod otherwise written for
+// the next step to overwrite); then the half kick, damping and the
+// angular-speed clamp.
 __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
     k_reduce_kick(State st, rg_config cfg, const int* off, const int* ent, const double* cf, int ccap,
-                  int wall, HistFinish hf, Ctl* ctl) {
+                  int wall, int store, HistFinish hf, Ctl* ctl) {
   griddep_wait();
   if (ctl->err) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) hist_finish(hf, ctl);
@@ -78,8 +80,10 @@ __global__ void __launch_bounds__(256, RG_BODY_MIN_BLOCKS)
     d3 f{0, 0, 0}, t{0, 0, 0};
     body_sum(off, ent, cf, ccap, i, f, t);
     bad |= kick_rod(st, cfg, ax, wall, i, f, t, el, ea);
-    st.f.st(i, f);
-    st.tau.st(i, t);
+    if (store) {
+      st.f.st(i, f);
+      st.tau.st(i, t);
+    }
   }
   if (bad) atomicOr(&ctl->err, ERR_NONFINITE);
 }
@@ -129,9 +133,9 @@ void reduce_drift_launch(rg_system* s, bool wall, HistFinish hf) {
   RGL launch_dep(k_reduce_drift, body_grid(s), 256, s->stream, s->st, s->box, s->cfg, s->csr.off, s->csr.ent,
                                                           s->d_cf, s->ccap, wall ? 1 : 0, o, hf, s->d_ctl);
 }
-void reduce_kick_launch(rg_system* s, bool wall, HistFinish hf) {
+void reduce_kick_launch(rg_system* s, bool wall, HistFinish hf, bool store) {
   RGL launch_dep(k_reduce_kick, body_grid(s), 256, s->stream, s->st, s->cfg, s->csr.off, s->csr.ent, s->d_cf,
-                                                         s->ccap, wall ? 1 : 0, hf, s->d_ctl);
+                                                         s->ccap, wall ? 1 : 0, store ? 1 : 0, hf, s->d_ctl);
 }
 void clear_forces_launch(rg_system* s) {
   RGL launch_dep(k_clear_forces, body_grid(s), 256, s->stream, s->st, s->d_ctl);

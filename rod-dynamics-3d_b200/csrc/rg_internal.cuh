@@ -362,12 +362,14 @@ void force_rebuild(rg_system* s);
 // rg_forces.cu
 enum class EvalTail { kForces, kHalfPos, kSecondHalf };
 // detect (unless fresh) + forces; the tail (force_eval_launch in rg_forces.cu)
-void force_eval_launch(rg_system* s, EvalTail tail = EvalTail::kForces, bool seg_ready = false);
+// results: the potential energy and (kSecondHalf) the summed forces are wanted
+void force_eval_launch(rg_system* s, EvalTail tail = EvalTail::kForces, bool seg_ready = false, bool results = true);
 // forces at t reduced per body, first half kick and drift, segment records
 // and displacement check of the drifted positions (velocity Verlet)
 void reduce_drift_launch(rg_system* s, bool wall, rg::HistFinish hf);
-// forces at t + dt reduced per body (kept in f, tau) and the second half kick
-void reduce_kick_launch(rg_system* s, bool wall, rg::HistFinish hf);
+// forces at t + dt reduced per body (kept in f, tau when store) and the
+// second half kick
+void reduce_kick_launch(rg_system* s, bool wall, rg::HistFinish hf, bool store);
 void csr_launch(rg_system* s, bool counted = false);  // body CSR of the current contacts
 // rg_integrate.cu
 void clear_forces_launch(rg_system* s);
