@@ -98,7 +98,6 @@ void free_contact_buffers(rg_system* s) {
 cudaError_t alloc_contact_buffers(rg_system* s, int ccap, int hcap) {
   const int n = s->n;
   s->ccap = ccap;
-  ++s->buf_gen;
   cudaError_t e;
   if ((e = s->con.alloc(ccap))) return e;
   if ((e = cudaMalloc(&s->csr.cnt, sizeof(int) * (n + 1)))) return e;
@@ -148,7 +147,7 @@ cudaError_t alloc_contact_buffers(rg_system* s, int ccap, int hcap) {
   if ((e = cudaMalloc(&s->d_cf, sizeof(double) * (13 * (size_t)ccap + 64)))) return e;
   if ((e = cudaMalloc(&s->d_feat, sizeof(float) * 8 * (size_t)ccap))) return e;
   if ((e = cudaMalloc(&s->d_pred, sizeof(float) * 3 * (size_t)ccap))) return e;
-  if ((s->cfg.model == RG_MODEL_HARMONIC || s->cfg.model == RG_MODEL_HERTZ_MINDLIN) && n <= kVerletTeamRods &&
+  if ((s->cfg.model == RG_MODEL_HARMONIC || s->cfg.model == RG_MODEL_HERTZ_MINDLIN) &&
       (e = s->vteam.alloc(n, ccap)))
     return e;
   int scap = ccap + 1;
@@ -337,6 +336,51 @@ void ctl_reset_launch(Ctl* const* d_ctls, int n, cudaStream_t st) {
   RGL k_ctl_reset<<<(n + 127) / 128, 128, 0, st>>>(d_ctls, n);
 }
 
+// ---- state transfer of larger systems ------------------------------------------
+// The caller's arrays are interleaved per rod, the state is not.  From
+// kStageRods rods on the arrays cross the bus as they are (one copy into the
+// page-locked buffer, then the link) and a kernel turns them over; below, the
+// extra launch costs more than the host loop.  staged: x[3n] q[4n] v[3n]
+// w[3n] f[3n] tau[3n].
+constexpr int kStageRods = 4096;
+
+__global__ void k_state_check(const double* staged, long long count, int* bad) {
+  int any = 0;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < count; k += (long long)gridDim.x * blockDim.x)
+    any |= !isfinite(staged[k]);
+  if (__syncthreads_or(any) && threadIdx.x == 0) atomicOr(bad, 1);
+}
+// Offsets (in rods) of the staged arrays and their widths; component k of the
+// array starting at state component c0.
+struct StagePart {
+  int off, width, c0;
+};
+__device__ __constant__ const StagePart kStageParts[6] = {{0, 3, 0}, {3, 4, 3}, {7, 3, 7}, {10, 3, 10}, {13, 3, 13}, {16, 3, 16}};
+// Into the state (nothing when the check found a value that is not finite);
+// forces and torques are cleared.
+__global__ void k_state_in(double* state, const double* staged, int n, const int* bad) {
+  if (*(volatile const int*)bad) return;
+  const size_t N = (size_t)n;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
+    for (int p = 0; p < 4; ++p) {
+      const StagePart g = kStageParts[p];
+      const double* src = staged + g.off * N + g.width * i;
+      for (int k = 0; k < g.width; ++k) state[(g.c0 + k) * N + i] = src[k];
+    }
+    for (int c = 13; c < 19; ++c) state[c * N + i] = 0.0;
+  }
+}
+// Parts p0 <= p < p1 out of the state.
+__global__ void k_state_out(const double* state, double* staged, int n, int p0, int p1) {
+  const size_t N = (size_t)n;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x)
+    for (int p = p0; p < p1; ++p) {
+      const StagePart g = kStageParts[p];
+      double* dst = staged + g.off * N + g.width * i;
+      for (int k = 0; k < g.width; ++k) dst[k] = state[(g.c0 + k) * N + i];
+    }
+}
+
 cudaError_t take_snapshot(rg_system* s, Snapshot& sn, bool sync) {
   cudaError_t e = snapshot_alloc(s);
   if (e) return e;
@@ -455,8 +499,6 @@ int rg_create(const rg_config* cfg, rg_system** out) {
 
 int rg_destroy(rg_system* s) {
   if (!s) return RG_ERR_ARG;
-  if (s->graph) cudaGraphExecDestroy(s->graph);
-  if (s->vgraph) cudaGraphExecDestroy(s->vgraph);
   free_contact_buffers(s);
   detector_free(s);
   cudaFree(s->d_state); cudaFree(s->d_props); cudaFree(s->d_ctl); cudaFree(s->d_snap);
@@ -516,11 +558,45 @@ int rg_set_bodies(rg_system* s, const double* radius, const double* half_height,
   return RG_OK;
 }
 
+}  // extern "C"
+
+// Upload through the device (k_state_in).  The snapshot buffer, which is live
+// only inside a step call, holds the staged arrays.
+static int set_state_staged(rg_system* s, const double* x, const double* q, const double* v, const double* w) {
+  const size_t N = (size_t)s->n;
+  if (!s->d_snap) RG_TRY(cudaMalloc(&s->d_snap, sizeof(double) * 19 * N), "staging buffer");
+  double* b = s->h_stage;
+  const double* src[4] = {x, q, v, w};
+  const size_t off[5] = {0, 3 * N, 7 * N, 10 * N, 13 * N};
+  int* bad = &s->d_ctl->stage_bad;
+  RG_TRY(cudaMemsetAsync(bad, 0, sizeof(int), s->stream), "staging");
+  // copied piece by piece, each on its way while the next is copied
+  const size_t piece = (size_t)1 << 17;
+  for (int p = 0; p < 4; ++p)
+    for (size_t k = off[p]; k < off[p + 1]; k += piece) {
+      const size_t m = off[p + 1] - k < piece ? off[p + 1] - k : piece;
+      std::memcpy(b + k, src[p] + (k - off[p]), sizeof(double) * m);
+      RG_TRY(cudaMemcpyAsync(s->d_snap + k, b + k, sizeof(double) * m, cudaMemcpyHostToDevice, s->stream), "upload state");
+    }
+  RGL k_state_check<<<grid_for(13 * (long long)N, 256), 256, 0, s->stream>>>(s->d_snap, 13 * (long long)N, bad);
+  RGL k_state_in<<<grid_for((long long)N, 256), 256, 0, s->stream>>>(s->d_state, s->d_snap, s->n, bad);
+  RG_TRY(cudaMemcpyAsync(s->h_wn, bad, sizeof(int), cudaMemcpyDeviceToHost, s->stream), "upload state");
+  RG_TRY(cudaStreamSynchronize(s->stream), "set_state sync");
+  RG_TRY(cudaGetLastError(), "set_state");
+  if (*s->h_wn) return fail(s, RG_ERR_NONFINITE, "non-finite component in the uploaded state");
+  s->state_set = true;
+  s->contacts_fresh = Fresh::kNo;
+  return RG_OK;
+}
+
+extern "C" {
+
 int rg_set_state(rg_system* s, const double* x, const double* q, const double* v, const double* w,
                  const double* f, const double* tau) {
   if (!s || !x || !q || !v || !w) return RG_ERR_ARG;
   const int n = s->n;
   double* b = s->h_stage;
+  if (n >= kStageRods && !f && !tau) return set_state_staged(s, x, q, v, w);
   std::memset(b, 0, sizeof(double) * 19 * (size_t)n);
   for (int i = 0; i < n; ++i) {
     for (int k = 0; k < 3; ++k) {
@@ -551,6 +627,25 @@ int rg_get_state(const rg_system* s, double* x, double* q, double* v, double* w,
   if (!s) return RG_ERR_ARG;
   const int n = s->n;
   const double* b = s->h_stage;
+  if (n >= kStageRods) {
+    rg_system* m = const_cast<rg_system*>(s);
+    const size_t N = (size_t)n;
+    double* dst[6] = {x, q, v, w, f, tau};
+    const size_t off[7] = {0, 3 * N, 7 * N, 10 * N, 13 * N, 16 * N, 19 * N};
+    int p0 = 0, p1 = 6;  // the parts asked for lie in [p0, p1)
+    while (p0 < p1 && !dst[p0]) ++p0;
+    while (p1 > p0 && !dst[p1 - 1]) --p1;
+    if (p0 == p1) return RG_OK;
+    if (!s->d_snap) RG_TRY2(m, cudaMalloc(&m->d_snap, sizeof(double) * 19 * N), "staging buffer");
+    RGL k_state_out<<<grid_for((long long)N, 256), 256, 0, s->stream>>>(s->d_state, s->d_snap, n, p0, p1);
+    for (int p = p0; p < p1; ++p)
+      RG_TRY2(m, cudaMemcpyAsync(s->h_stage + off[p], s->d_snap + off[p], sizeof(double) * (off[p + 1] - off[p]),
+                                 cudaMemcpyDeviceToHost, s->stream), "download state");
+    RG_TRY2(m, cudaStreamSynchronize(s->stream), "download state");
+    for (int p = p0; p < p1; ++p)
+      if (dst[p]) std::memcpy(dst[p], b + off[p], sizeof(double) * (off[p + 1] - off[p]));
+    return RG_OK;
+  }
   cudaError_t e = cudaMemcpyAsync(s->h_stage, s->d_state, sizeof(double) * 19 * (size_t)n,
                                   cudaMemcpyDeviceToHost, s->stream);
   if (!e) e = cudaStreamSynchronize(s->stream);
@@ -586,41 +681,6 @@ static void verlet_step(rg_system* s, bool last) {
   s->contacts_fresh = Fresh::kCsr;  // positions unchanged until the next drift
 }
 
-// Captures one Verlet step (entered with fresh contacts, not a call's last) as
-// a CUDA graph.
-// Every launch of the step is decided on the host from state that a whole
-// step leaves as it found it (fresh contacts, the history ping-pong index),
-// so the same graph serves every step until buffers are reallocated.
-static bool capture_verlet_step(rg_system* s) {
-  if (s->vgraph) {
-    cudaGraphExecDestroy(s->vgraph);
-    s->vgraph = nullptr;
-  }
-  const long long l0 = g_launches;
-  const int cur = s->hist.cur;
-  cudaGraph_t g = nullptr;
-  if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  verlet_step(s, false);
-  cudaError_t e = cudaStreamEndCapture(s->stream, &g);
-  s->vgraph_kernels = g_launches - l0;
-  g_launches = l0;  // counted when the graph runs
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&s->vgraph, g, 0);
-  if (g) cudaGraphDestroy(g);
-  if (e != cudaSuccess || s->hist.cur != cur || s->contacts_fresh != Fresh::kCsr) {
-    cudaGetLastError();
-    if (s->vgraph) cudaGraphExecDestroy(s->vgraph);
-    s->vgraph = nullptr;
-    s->hist.cur = cur;
-    return false;
-  }
-  s->vgraph_gen = s->buf_gen;
-  s->vgraph_cur = cur;
-  return true;
-}
-
 void launch_steps(rg_system* s, int nsteps) {
   const int model = s->cfg.model;
   if (model == RG_MODEL_NSC) {
@@ -632,23 +692,8 @@ void launch_steps(rg_system* s, int nsteps) {
     if (nsteps > 0) verlet_run_launch(s, nsteps);
     return;
   }
-  int k = 0;
-  if (nsteps > 0 && s->contacts_fresh != Fresh::kCsr) {  // the first evaluation detects
-    verlet_step(s, nsteps == 1);
-    k = 1;
-  }
-  // The steps before the last replay one captured step (stage timers need the
-  // plain launches).
-  if (nsteps - k >= 3 && !s->prof_on) {
-    bool ok = s->vgraph && s->vgraph_gen == s->buf_gen && s->vgraph_cur == s->hist.cur;
-    if (!ok) ok = capture_verlet_step(s);
-    if (ok)
-      for (; k < nsteps - 1; ++k) {
-        RGL cudaGraphLaunch(s->vgraph, s->stream);
-        g_launches += s->vgraph_kernels - 1;
-      }
-  }
-  for (; k < nsteps; ++k) verlet_step(s, k == nsteps - 1);
+  // the multi-kernel form, whose launches the stage timers bracket
+  for (int k = 0; k < nsteps; ++k) verlet_step(s, k == nsteps - 1);
 }
 
 // Grows the buffer named by the error bits.  Returns false if nothing grew.

@@ -9,8 +9,8 @@
 // persistent step kernel in ONE cooperative launch for all requested
 // steps; that launch (with the reset of the team barriers) is captured in a
 // CUDA graph and replayed.  Members with the Verlet models run as teams of
-// one launch of the persistent Verlet kernel after it (those too large for
-// that form one after the other).
+// one launch of the persistent Verlet kernel after it (those with stage timers
+// on one after the other in the multi-kernel form).
 //
 // Schedule: each member's work is its rod count until the device has timed
 // its steps (every call records each member's own step time), then that

@@ -309,6 +309,7 @@ __global__ void k_lists_done(double near_skin, Ctl* ctl) {
   ctl->maxdisp = 0.0;
   if (near_due) {
     ctl->near_valid = 1;
+    ctl->flat_valid = 0;
     ctl->near_disp = 0.0;
     ctl->near_rebuilds += 1;
   }
@@ -379,6 +380,7 @@ __global__ void k_build_done(Ctl* ctl) {
     ctl->rebuilds += 1;
     ctl->rebuild = 0;
     ctl->near_valid = 0;  // near lists are drawn from the lists
+    ctl->flat_valid = 0;
   }
   ctl->maxdisp = 0.0;
 }
@@ -503,7 +505,6 @@ __global__ void k_grid_ncells(DetDev* dd, const Ctl* ctl) {
 static bool check_near_lists(const rg_config& c) { return c.near_skin_pct >= 0; }
 
 cudaError_t detector_alloc(rg_system* s) {
-  ++s->buf_gen;
   Detector& d = s->det;
   const int n = s->n;
   const rg_config& c = s->cfg;
@@ -582,6 +583,15 @@ cudaError_t detector_alloc(rg_system* s) {
     if ((e = cudaMalloc(&d.near_nbr, sizeof(int) * (size_t)n * d.maxnb))) return e;
     if ((e = cudaMalloc(&d.ref2, sizeof(double) * 6 * (size_t)n))) return e;
   }
+  if (c.model == RG_MODEL_HARMONIC || c.model == RG_MODEL_HERTZ_MINDLIN) {
+    // near lists hold a few pairs a rod; a list that does not fit grows with
+    // the neighbour lists (ERR_NBR_CAP)
+    const long long all = d.all_pairs ? (long long)n * n / 2 + 1 : (long long)n * d.maxnb;
+    const long long few = (long long)n * (d.maxnb / 8 > 1 ? d.maxnb / 8 : 1);
+    const long long cap = d.near_cnt && few < all ? few : all;
+    s->vteam.flat_cap = (int)(cap < 2000000000ll ? cap : 2000000000ll);
+    if ((e = cudaMalloc(&s->vteam.flat, sizeof(int2) * (size_t)s->vteam.flat_cap))) return e;
+  }
   if (c.model == RG_MODEL_NSC) {
     d.near_skin = near_skin;
     if ((e = cudaMalloc(&d.near, sizeof(int2) * (size_t)n * d.maxnb))) return e;
@@ -603,6 +613,8 @@ void detector_free(rg_system* s) {
   cudaFree(d.cell_rods); cudaFree(d.hit_cnt); cudaFree(d.hit_off); cudaFree(d.hit_mask);
   cudaFree(d.near); cudaFree(d.ref2); cudaFree(d.moved);
   cudaFree(d.near_cnt); cudaFree(d.near_nbr);
+  cudaFree(s->vteam.flat);
+  s->vteam.flat = nullptr;
   d = Detector();
 }
 

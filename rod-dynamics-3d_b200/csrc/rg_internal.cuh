@@ -60,6 +60,8 @@ struct Ctl {
                         // detection of this call's last step
   unsigned int bar_count, bar_gen;  // grid barrier
   int ins_n[2];         // pairs an evaluation adds to the history (by parity)
+  int stage_bad;        // a state upload held a value that is not finite
+  int flat_valid;       // 1: the flat pair list (persistent Verlet step) matches the near lists
   double res_sweep[1];  // per-sweep residual slots follow (velocity_iters)
 };
 
@@ -175,19 +177,23 @@ struct Nsc {
 constexpr size_t kTeamBarBytes = 1024;
 // Contact bookkeeping of the persistent Verlet step (rg_verlet.cu).
 struct VerletTeam {
-  // two contact lists (before and after a detection): per rod the first of
-  // its contacts, per contact its second body and its history entry (-1: none)
-  int *off[2] = {nullptr, nullptr}, *pb[2] = {nullptr, nullptr}, *hidx[2] = {nullptr, nullptr};
+  // two contact lists (before and after a detection): per rod the first
+  // contact it is first body of (-1: none), per contact its bodies and its
+  // history entry (-1: none)
+  int *first[2] = {nullptr, nullptr}, *hidx[2] = {nullptr, nullptr};
+  int2* pk[2] = {nullptr, nullptr};
   int cb = 0;                            // the current one
   int *head = nullptr, *next = nullptr;  // per rod: list of the contacts it is second body of
   int* ins = nullptr;                    // contacts whose pair an evaluation adds
+  // the near lists (or, without them, the whole lists) as one list of pairs
+  // sorted by (i, j)
+  int2* flat = nullptr;
+  int flat_cap = 0;
   void* view_dev = nullptr;
   cudaError_t alloc(int n, int ccap);
   void free_();
 };
-// Largest system whose Verlet steps run in the persistent form, and the rods
-// a block of its team takes.
-constexpr int kVerletTeamRods = 600000, kVerletRodsPerBlock = 128;
+constexpr int kVerletRodsPerBlock = 128;  // rods a block of a persistent Verlet team takes
 // What the contact buffers hold: nothing current, the contacts of the current
 // positions with the body CSR (multi-kernel form), or with the persistent
 // form's bookkeeping.
@@ -254,16 +260,6 @@ struct rg_system {
 
   int coop_blocks = 0;        // co-resident blocks for the persistent kernels
   int team_blocks = 0;        // blocks of the NSC team (0: automatic)
-  cudaGraphExec_t graph = nullptr;
-  int graph_kind = -1;
-  // one velocity-Verlet step (soft / HM) captured as a CUDA graph; valid
-  // while the buffers it names are the current ones (buf_gen) and the
-  // history table starts in the same ping-pong buffer (vgraph_cur)
-  cudaGraphExec_t vgraph = nullptr;
-  long long vgraph_gen = -1;
-  int vgraph_cur = -1;
-  long long vgraph_kernels = 0;  // kernel nodes of the graph
-  long long buf_gen = 0;         // bumped by every (re)allocation of device buffers
 
   // pinned staging for host <-> device state copies (19 n doubles)
   double* h_stage = nullptr;

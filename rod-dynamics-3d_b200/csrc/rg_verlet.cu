@@ -1,5 +1,5 @@
 // rg_verlet.cu - the velocity-Verlet step (soft and Hertz-Mindlin models) as
-// one persistent kernel for small and medium systems.
+// one persistent kernel.
 //
 // The same step as the multi-kernel form (rg_api.cu verlet_step; App::
 // physicsStep, src/app/main.cpp:4529-4810): forces at t, half kick and drift,
@@ -14,7 +14,7 @@
 //    the pass after the hit counts are known; the forces at the next step's
 //    start reuse those contacts in place;
 //  * a body's contacts are found without a sorted incidence table: those where
-//    it is the first body are a contiguous range of the (a, b)-sorted list,
+//    it is the first body are a run of the (a, b)-sorted list,
 //    those where it is the second hang off it in a short linked list, walked
 //    in ascending order; together the contact order of the reference's sums;
 //  * the history entry of a persisting contact is found through the previous
@@ -24,12 +24,13 @@
 //    ends (or the table fills up), when they are removed.
 //
 // Bound: instruction and L2 latency of the five phases plus the barriers (1 to
-// 2 us each).  Measured, multi-kernel form -> this one, us per step: 1,000
-// rods 80 -> 38, 5,000 (soft) 104 -> 39, 20,000 103 -> 52, 100,000 130 -> 82,
-// 400,000 279 -> 238, 1,000,000 441 -> 507 (sparse contacts) and 641 -> 606
-// (80,000 contacts).  The line between them (kVerletTeamRods) lies where the
-// multi-kernel form, with more warps on an SM for the per-rod passes, draws
-// level.
+// 2 us each) up to some 50,000 rods, then the two passes over the body state.
+// Measured, multi-kernel form (one captured graph a step) -> this one, us per
+// step: 1,000 rods 80 -> 33, 5,000 (soft) 104 -> 38, 20,000 103 -> 41, 100,000
+// 130 -> 61, 400,000 279 -> 167, 1,000,000 441 -> 320 (5,000 contacts) and 641
+// -> 389 (80,000 contacts).  It is the faster one at every size, so the
+// multi-kernel form only serves the stage timers, single force evaluations
+// and detections.
 #include <cstring>
 #include <vector>
 
@@ -44,7 +45,7 @@ constexpr int kIns = 512;           // inserted pairs sorted on chip
 // Where one team stands in its system's call (the same in every block).
 struct VerletRun {
   int H, cur;      // history entries (dead ones included), current table
-  int C, cb;       // contacts, current contact-index buffer
+  int C, cb;       // contacts, current contact list
   long long fr;    // evaluation counter
   bool idx_ok;     // hidx[cb] names the contacts' table entries
   int lo, hi;      // this block's rods
@@ -230,9 +231,9 @@ __device__ inline void v_body_sum(const VerletView& W, const VerletRun& r, int i
     t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
     last = c;
   }
-  const int* off = W.off[r.cb];
-  const int e = off[i + 1];
-  for (int c = off[i]; c < e; ++c) {  // first body of
+  const int2* pk = W.pk[r.cb];
+  const int c0 = W.first[r.cb][i];
+  for (int c = c0; c >= 0 && c < r.C && pk[c].x == i; ++c) {  // first body of
     const double* g = W.cf + c;
     f.x = f.x + g[0]; f.y = f.y + g[cc]; f.z = f.z + g[2 * cc];
     t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
@@ -249,47 +250,24 @@ __device__ inline void v_publish_disp(const NscView& V, double m, double m2, Sme
   }
 }
 
-// Detection at the current segment records (every block past a barrier since
-// they and the displacement bounds were written), and evaluation r.fr on the
-// contacts found.
-template <int G>
-__device__ __forceinline__ int v_count(const VerletView& W, const VerletRun& r, const int* cnt, const int* nbr,
-                                       int prefilter) {
-  const NscView& V = W.v;
-  int mine = 0;
-  for (int base = r.lo; base < r.hi; base += blockDim.x / G) {
-    const int i = base + threadIdx.x / G;
-    const bool valid = i < r.hi;
-    const int c = narrow_count_lanes<G>(i, valid, V.seg, V.st.inv_mass, V.box, W.delta, cnt, nbr, V.maxnb, V.words,
-                                        V.mask, prefilter);
-    if (valid && (threadIdx.x & (G - 1)) == 0) {
-      V.hit_cnt[i] = c;
-      W.head[i] = -1;
-      mine += c;
-    }
-  }
-  return mine;
-}
-__device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, VerletRun& r, VerletSmem& S,
-                                           bool energy) {
+// The flat pair list: near lists from the lists where they are due (else the
+// lists themselves), then all rods' entries as (i, j) pairs in order.
+__device__ __noinline__ bool v_flatten(const Team& T, const VerletView& W, const VerletRun& r, VerletSmem& S, bool due) {
   const NscView& V = W.v;
   Ctl* ctl = V.ctl;
   const int n = V.st.n, rank = T.rank(), t = threadIdx.x;
-  const bool need = *(volatile int*)&ctl->rebuild ||
-                    (!V.all_pairs && *(volatile double*)&ctl->maxdisp >= 0.5 * V.skin * (1.0 - 1e-9));
+  const double* im = V.st.inv_mass;
   const bool near = W.near_cnt != nullptr;
-  const bool due = near && (need || !*(volatile int*)&ctl->near_valid ||
-                            *(volatile double*)&ctl->near_disp >= 0.5 * V.near_skin * (1.0 - 1e-9));
-  if (need && !rebuild_phase(T, V, S.s)) return false;
-  if (due) {
-    const double* im = V.st.inv_mass;
-    for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+  int mine = 0;
+  for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+    const int cnt = V.nbr_cnt[i];
+    int m = cnt;
+    if (near && due) {
       const Seg A = V.seg[i];
       const bool a_static = !(im[i] > 0.0);
-      const int cnt = V.nbr_cnt[i];
       const int* list = V.nbr + (size_t)i * V.maxnb;
       int* out = W.near_nbr + (size_t)i * V.maxnb;
-      int m = 0;
+      m = 0;
       for (int k = 0; k < cnt; ++k) {
         const int j = list[k];
         if (a_static && !(im[j] > 0.0)) continue;
@@ -301,21 +279,85 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
       W.near_cnt[i] = m;
       V.ref2[i] = A.cx; V.ref2[n + i] = A.cy; V.ref2[2 * n + i] = A.cz;
       V.ref2[3 * n + i] = A.ux; V.ref2[4 * n + i] = A.uy; V.ref2[5 * n + i] = A.uz;
+    } else if (near) {
+      m = W.near_cnt[i];
     }
-    if (!team_sync(T)) return false;
-    if (rank == 0 && t == 0) {  // every block has read them
+    mine += m;
+  }
+  const int bsum = block_reduce_sum_i(mine, S.s.red_i);
+  if (t == 0) V.blk[rank] = bsum;
+  if (!team_sync(T)) return false;
+  int prefix, total;
+  block_prefix(V.blk, T.nb, rank, prefix, total, S.s);
+  if (total > W.flat_cap) {
+    if (rank == 0 && t == 0) atomicOr(&ctl->err, ERR_NBR_CAP);
+    return false;
+  }
+  const int* cnts = near ? W.near_cnt : V.nbr_cnt;
+  const int* lists = near ? W.near_nbr : V.nbr;
+  int run = prefix;
+  for (int base = r.lo; base < r.hi; base += blockDim.x) {
+    const int i = base + t;
+    const int m = i < r.hi ? cnts[i] : 0;
+    int tot;
+    const int o = run + block_excl_scan(m, S.s.scan_w, tot);
+    const int* list = lists + (size_t)i * V.maxnb;
+    for (int k = 0; k < m; ++k) W.flat[o + k] = make_int2(i, list[k]);
+    run += tot;
+  }
+  if (rank == 0 && t == 0) {  // every block has read them
+    ctl->near_n = total;
+    ctl->flat_valid = 1;
+    if (near && due) {
       ctl->near_valid = 1;
       ctl->near_disp = 0.0;
       ctl->near_rebuilds += 1;
     }
   }
-  const int* cnt = near ? W.near_cnt : V.nbr_cnt;
-  const int* nbr = near ? W.near_nbr : V.nbr;
-  // lanes a rod: as many as one round of the block has (whole lists: four)
-  const int rods = r.hi - r.lo, threads = (int)blockDim.x, pre = near ? 0 : (V.all_pairs ? 2 : 1);
-  const int mine = 4 * rods <= threads || !near ? v_count<4>(W, r, cnt, nbr, pre)
-                   : 2 * rods <= threads        ? v_count<2>(W, r, cnt, nbr, pre)
-                                                : v_count<1>(W, r, cnt, nbr, pre);
+  return team_sync(T);
+}
+
+// Detection at the current segment records (every block past a barrier since
+// they and the displacement bounds were written), and evaluation r.fr on the
+// contacts found.  One thread tests one pair of the flat list (a thread per
+// rod over its near list left most lanes idle: a rod has 0.2 to 0.6 entries,
+// a warp's busiest one three or four).
+__device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, VerletRun& r, VerletSmem& S,
+                                           bool energy) {
+  const NscView& V = W.v;
+  Ctl* ctl = V.ctl;
+  const int rank = T.rank(), t = threadIdx.x;
+  const bool need = *(volatile int*)&ctl->rebuild ||
+                    (!V.all_pairs && *(volatile double*)&ctl->maxdisp >= 0.5 * V.skin * (1.0 - 1e-9));
+  const bool due = need || (W.near_cnt && (!*(volatile int*)&ctl->near_valid ||
+                                           *(volatile double*)&ctl->near_disp >= 0.5 * V.near_skin * (1.0 - 1e-9)));
+  const bool flat = due || !*(volatile int*)&ctl->flat_valid;
+  if (need && !rebuild_phase(T, V, S.s)) return false;
+  if (flat && !v_flatten(T, W, r, S, due)) return false;
+  // test: each block a 32-aligned range of pairs, one bit per pair
+  const int P = *(volatile int*)&ctl->near_n;
+  const int per = (((P + T.nb - 1) / T.nb) + 31) & ~31;
+  const int plo = min(rank * per, P), phi = min(plo + per, P);
+  unsigned* bits = reinterpret_cast<unsigned*>(V.mask);
+  const double* im = V.st.inv_mass;
+  int mine = 0;
+  for (int p0 = plo; p0 < phi; p0 += blockDim.x) {
+    const int p = p0 + t;
+    bool hit = false;
+    if (p < phi) {
+      const int2 pr = W.flat[p];
+      if (im[pr.x] > 0.0 || im[pr.y] > 0.0) {
+        const Seg A = V.seg[pr.x], B = V.seg[pr.y];
+        const Narrow nr = narrow_pair(A, B, V.box);
+        hit = contact_test(nr.d2, A.r + B.r, W.delta);
+      }
+    }
+    const unsigned word = __ballot_sync(0xffffffffu, hit);
+    if ((t & 31) == 0 && p < phi) {
+      bits[p >> 5] = word;
+      mine += __popc(word);
+    }
+  }
   const int bsum = block_reduce_sum_i(mine, S.s.red_i);
   if (t == 0) V.blk[rank] = bsum;
   if (!team_sync(T)) return false;
@@ -326,28 +368,20 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
     if (rank == 0 && t == 0) atomicOr(&ctl->err, ERR_CONTACT_CAP);
     return false;
   }
-  const int ob = r.cb, cb = 1 - r.cb;  // the contact lists before and now
-  int* off = W.off[cb];
+  // contacts in pair order: the hits' pairs to their slots first, then one
+  // thread per slot
+  const int ob = r.cb, cb = 1 - r.cb, oc = r.C;  // the contact lists before and now
   int run = prefix;
-  for (int base = r.lo; base < r.hi; base += blockDim.x) {
-    const int i = base + t;
-    const int c = i < r.hi ? V.hit_cnt[i] : 0;
+  const int wlo = plo >> 5, whi = plo < phi ? (phi + 31) >> 5 : wlo;
+  for (int base = wlo; base < whi; base += blockDim.x) {
+    const int w = base + t;
+    const unsigned word = w < whi ? bits[w] : 0u;  // (this block wrote it)
     int tot;
-    int o = run + block_excl_scan(c, S.s.scan_w, tot);
-    if (i < r.hi) off[i] = o;
-    if (c) {
-      const int* list = nbr + (size_t)i * V.maxnb;
-      for (int w = 0; w * 64 < cnt[i]; ++w)
-        for (unsigned long long m = __ldcg(&V.mask[(size_t)i * V.words + w]); m; m &= m - 1) {
-          V.con.a[o] = i;
-          V.con.b[o] = list[w * 64 + __ffsll((long long)m) - 1];
-          ++o;
-        }
-    }
+    int o = run + block_excl_scan(__popc(word), S.s.scan_w, tot);
+    for (unsigned m = word; m; m &= m - 1) W.pk[cb][o++] = W.flat[(w << 5) + __ffs((int)m) - 1];
     run += tot;
   }
   if (rank == 0 && t == 0) {
-    off[n] = total;
     ctl->contacts = total;
     ctl->contact_steps += total;
   }
@@ -356,19 +390,25 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
   __syncthreads();
   for (int c = prefix + t; c < run; c += blockDim.x) {
     // every load that needs no result comes before the first store
-    const int a = V.con.a[c], b = V.con.b[c];
+    const int2 pr = W.pk[cb][c];
+    const int a = pr.x, b = pr.y;
+    // the first contact of a: the slot before belongs to another rod (of a
+    // block's first slot the block before may hold more of the same run: the
+    // lowest slot wins below)
+    const bool head_of_a = c > prefix ? W.pk[cb][c - 1].x != a : true;
     const Seg A = V.seg[a], B = V.seg[b];
     const PairIn in = load_pair(V.st, a, b);
     int f = -1;
     bool known = false;
-    if (r.idx_ok) {
-      const int e = W.off[ob][a + 1];
-      for (int k = W.off[ob][a]; k < e; ++k)
-        if (W.pb[ob][k] == b) {
+    if (r.idx_ok)
+      for (int k = W.first[ob][a]; k >= 0 && k < oc; ++k) {
+        const int2 q = W.pk[ob][k];
+        if (q.x != a) break;
+        if (q.y == b) {
           f = W.hidx[ob][k];
           known = true;
         }
-    }
+      }
     if (!known && r.H > 0) f = v_find(W, r, a, b);
     long long frame = 0;
     const d3 old = v_old(W, r, f, frame);
@@ -377,7 +417,7 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
     const d3 diff = nr.pb - nr.pa;
     const VContact g{nr.pa, nr.pb, dist > 1e-10 ? diff / dist : mk3(1, 0, 0), nr.sh, dist, A.r + B.r};
     W.next[c] = atomicExch(&W.head[b], c);
-    W.pb[cb][c] = b;
+    if (head_of_a) atomicMin(reinterpret_cast<unsigned*>(&W.first[cb][a]), (unsigned)c);
     write_contact(V.con, c, a, b, g.surf, nr);
     v_eval(W, r, c, in, g, f, old, frame, energy);
   }
@@ -434,6 +474,8 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
     for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
       const Seg s = make_seg(st, i);
       V.seg[i] = s;
+      W.head[i] = -1;
+      W.first[1 - r.cb][i] = -1;
       if (out.ref) m = fmax(m, seg_disp(s, out.ref, n, i, V.box));
       if (out.ref2) m2 = fmax(m2, seg_disp(s, out.ref2, n, i, V.box));
     }
@@ -448,8 +490,8 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
     if (step == 0 && !W.fresh) {
       if (!v_detect_eval(T, W, r, S, false)) return false;
     } else {
-      const int c1 = W.off[r.cb][r.hi];
-      for (int c = W.off[r.cb][r.lo] + t; c < c1; c += blockDim.x) v_eval_again(W, r, c);
+      const int per = (r.C + T.nb - 1) / T.nb, c1 = min((rank + 1) * per, r.C);
+      for (int c = rank * per + t; c < c1; c += blockDim.x) v_eval_again(W, r, c);
       if (rank == 0 && t == 0) ctl->contact_steps += r.C;
     }
     if (!team_sync(T)) return false;
@@ -461,6 +503,8 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
       for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
         d3 f{0, 0, 0}, tq{0, 0, 0};
         if (st.inv_mass[i] > 0.0) v_body_sum(W, r, i, f, tq);
+        W.head[i] = -1;  // for the detection that follows
+        W.first[1 - r.cb][i] = -1;
         drift_rod(st, V.box, cfg, ax, wall, i, f, tq, out, invL, m, m2);
       }
       if (out.ref || out.ref2) v_publish_disp(V, m, m2, S.s);
@@ -558,8 +602,8 @@ VerletView make_verlet_view(rg_system* s) {
     W.hkey[k] = H.key[k];
     W.hval[k] = H.val[k];
     W.hframe[k] = H.frame[k];
-    W.off[k] = s->vteam.off[k];
-    W.pb[k] = s->vteam.pb[k];
+    W.first[k] = s->vteam.first[k];
+    W.pk[k] = s->vteam.pk[k];
     W.hidx[k] = s->vteam.hidx[k];
   }
   W.hcap = H.cap;
@@ -572,6 +616,8 @@ VerletView make_verlet_view(rg_system* s) {
   W.head = s->vteam.head;
   W.next = s->vteam.next;
   W.ins = s->vteam.ins;
+  W.flat = s->vteam.flat;
+  W.flat_cap = s->vteam.flat_cap;
   W.fresh = s->contacts_fresh == Fresh::kTeam ? 1 : 0;
   W.cb = s->vteam.cb;
   return W;
@@ -586,8 +632,7 @@ void verlet_launched(rg_system* s, int nsteps) {
 
 bool verlet_team_fits(const rg_system* s) {
   const int m = s->cfg.model;
-  return (m == RG_MODEL_HARMONIC || m == RG_MODEL_HERTZ_MINDLIN) && !s->prof_on && s->vteam.head &&
-         s->n <= kVerletTeamRods;
+  return (m == RG_MODEL_HARMONIC || m == RG_MODEL_HERTZ_MINDLIN) && !s->prof_on && s->vteam.head;
 }
 
 void verlet_launch(const VerletView* views, const TeamDesc* teams, int nteams, const int* members, int grid, int nsteps,
@@ -624,27 +669,32 @@ void verlet_run_launch(rg_system* s, int nsteps) {
   verlet_launched(s, nsteps);
 }
 
-// One allocation behind all arrays (each a multiple of 16 bytes).
+// One allocation behind the arrays (each a multiple of 16 bytes); the flat
+// list belongs to the detector's lists.
 cudaError_t VerletTeam::alloc(int n, int ccap) {
-  const size_t rods = ((size_t)n + 4) / 4 * 4, cons = ((size_t)ccap + 3) / 4 * 4;
+  const size_t rods = ((size_t)n + 3) / 4 * 4, cons = ((size_t)ccap + 3) / 4 * 4;
   const size_t view = (sizeof(VerletView) + 15) / 16 * 16;
-  const cudaError_t e = cudaMalloc(&view_dev, view + sizeof(int) * (3 * rods + 6 * cons));
+  const cudaError_t e = cudaMalloc(&view_dev, view + sizeof(int) * (3 * rods + 8 * cons));
   if (e) return e;
   int* p = reinterpret_cast<int*>(static_cast<char*>(view_dev) + view);
   for (int k = 0; k < 2; ++k) {
-    off[k] = p;
-    pb[k] = p + rods;
-    hidx[k] = p + rods + cons;
-    p += rods + 2 * cons;
+    pk[k] = reinterpret_cast<int2*>(p);
+    hidx[k] = p + 2 * cons;
+    first[k] = p + 3 * cons;
+    p += 3 * cons + rods;
   }
-  head = p;
-  next = p + rods;
-  ins = next + cons;
+  next = p;
+  ins = p + cons;
+  head = p + 2 * cons;
   return cudaSuccess;
 }
 void VerletTeam::free_() {
   cudaFree(view_dev);
+  int2* const f = flat;
+  const int fc = flat_cap;
   *this = VerletTeam();
+  flat = f;
+  flat_cap = fc;
 }
 
 }  // namespace rg

@@ -225,7 +225,9 @@ struct VerletView {
   int hcap, hcur;
   int *touched, *touched_off, *kept, *kept_off;
   double* newval;
-  int *off[2], *pb[2], *hidx[2], *head, *next, *ins;  // VerletTeam
+  int *first[2], *hidx[2], *head, *next, *ins;  // VerletTeam
+  int2 *pk[2], *flat;
+  int flat_cap;
   int fresh, cb;  // 1: contacts, indices and lists of buffer cb are current
 };
 VerletView make_verlet_view(rg_system* s);
