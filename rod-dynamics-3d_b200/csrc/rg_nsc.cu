@@ -628,6 +628,7 @@ struct SmallSmem {
   unsigned char dyn[kSmallB];        // 1: dynamic body
   // this block's contacts in colour-major slots: contact, colour, body slots
   unsigned short order[kSmallC], pa[kSmallC], pb[kSmallC];
+  unsigned short comp[kSmallC];      // component of the slot's contact (split solves)
   unsigned char pcol[kSmallC];
   unsigned char cached[kSmallC];     // 1: the slot's contact is in the warm cache
   int cnt[kMaxColors + 1], coff[kMaxColors + 1], cur[kMaxColors + 1];
@@ -797,6 +798,7 @@ __device__ __noinline__ Share small_split(const Team& T, int C, int ncol) {
       S.pcol[c] = 0;
       S.pa[c] = X.la[c];
       S.pb[c] = X.lb[c];
+      S.comp[c] = 0;
     }
     if (t == 0) {
       S.nbody = S.nloc;
@@ -907,6 +909,7 @@ __device__ __noinline__ Share small_split(const Team& T, int C, int ncol) {
     S.pcol[p] = (unsigned char)k;
     S.pa[p] = (unsigned short)X.bl[X.la[c]];
     S.pb[p] = (unsigned short)X.bl[X.lb[c]];
+    S.comp[p] = split ? (unsigned short)X.lab[c] : 0;
   }
   __syncthreads();
   return sh;
@@ -1146,12 +1149,19 @@ __device__ __forceinline__ int sweep_share(const Sweep w, int C, Row& h, Update 
   const bool wall = S.pa[q0] == S.pb[q0];
   double* vs = &S.vel[6 * (side ? S.pb[q0] : S.pa[q0])];
   const int nv = 6 * S.nbody;
+  // One warp: a component that a sweep left unchanged stays so and its lanes
+  // rest; a colour without other contacts costs nothing (in the sweeps of a
+  // set that will not converge, most components are done early: a step of
+  // 50000 rods 358 -> 346 us, of a set with more such sweeps 403 -> 384).
+  const unsigned same = ONE ? __match_any_sync(0xffffffffu, pair < C ? (int)S.comp[pair] : -1) : 0u;
+  bool rest = false;
   int i = 0;
   while (i < w.n) {
     double loc = 0.0;
     for (int k = 0; k < w.colors; ++k) {
-      const bool mine = col == k;
+      const bool mine = col == k && !rest;
       const unsigned act = __ballot_sync(0xffffffffu, mine);
+      if (ONE && act == 0u) continue;
       if (mine) loc = update(h, vs, side, wall, act);
       if (k + 1 < w.colors) sweep_sync<ONE>();
     }
@@ -1163,7 +1173,10 @@ __device__ __forceinline__ int sweep_share(const Sweep w, int C, Row& h, Update 
       if ((t & 31) == 0) ls[t >> 5] = m;
     }
     ++i;
-    if (ONE) __syncwarp();  // (the vote below orders nothing)
+    if (ONE) {
+      __syncwarp();  // (the votes below order nothing)
+      rest = (__ballot_sync(0xffffffffu, loc != 0.0) & same) == 0u;
+    }
     // one vote: goes on while a change reaches the limit (or, in a chunk,
     // while anything changes)
     const int more = w.stop >= 0.0 ? loc >= w.stop : loc != 0.0;
