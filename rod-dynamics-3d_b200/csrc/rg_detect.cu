@@ -14,6 +14,7 @@
 // list stays exact until some rod has moved (translation plus end-point swing)
 // more than skin/2 since the build; a device-side check triggers the rebuild.
 // Neighbour cells are staged through shared memory tile by tile.
+#include <algorithm>
 #include <cstdio>
 
 #include "rg_detect_dev.cuh"
@@ -336,7 +337,8 @@ __global__ void k_zero_cells(int* cnt, int* fill, int ncells, int* nbr_cnt, int 
   }
 }
 
-// One block per home cell (see build_cell).
+// One block per home cell (see build_cell_pairs); in all-pairs boxes one
+// warp per rod.
 __global__ void __launch_bounds__(kTile) k_build_lists(const Seg* seg, int n, const GridDev* gdev, Box box,
                                                        const int* cell_start, const int* cell_rods,
                                                        double margin, double skin, double cut_center,
@@ -349,23 +351,28 @@ __global__ void __launch_bounds__(kTile) k_build_lists(const Seg* seg, int n, co
   constexpr int kQ = 4 * kTile;  // candidate queues of the compacted build
   __shared__ unsigned q1[kQ], q2[kQ];
   int overflow = 0;
-  double invL[3] = {1.0, 1.0, 1.0};
-  for (int k = 0; k < 3; ++k)
-    if (box.L[k] > 0.0) invL[k] = 1.0 / box.L[k];
-  for (int cell = blockIdx.x; cell < g.ncells; cell += gridDim.x)
-    build_cell_pairs(seg, g, box, invL, cell_start, cell_rods, margin, skin, all_pairs, nbr_cnt, nbr, maxnb,
-                     cell, sm, q1, q2, kQ, overflow);
+  if (all_pairs) {
+    list_all_pairs(n, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), (int)((gridDim.x * blockDim.x) >> 5),
+                   nbr_cnt, nbr, maxnb, overflow);
+  } else {
+    double invL[3] = {1.0, 1.0, 1.0};
+    for (int k = 0; k < 3; ++k)
+      if (box.L[k] > 0.0) invL[k] = 1.0 / box.L[k];
+    for (int cell = blockIdx.x; cell < g.ncells; cell += gridDim.x)
+      build_cell_pairs(seg, g, box, invL, cell_start, cell_rods, margin, skin, nbr_cnt, nbr, maxnb, cell, sm,
+                       q1, q2, kQ, overflow);
+  }
   if (overflow) atomicOr(&ctl->err, ERR_NBR_CAP);
-  (void)n;
   (void)cut_center;
 }
 
-__global__ void k_save_ref(const Seg* seg, int n, double* ref, int* nbr, int* nbr_cnt, int maxnb, Ctl* ctl) {
+__global__ void k_save_ref(const Seg* seg, int n, double* ref, int* nbr, int* nbr_cnt, int maxnb, int all_pairs,
+                           Ctl* ctl) {
   griddep_wait();
   if (ctl->err || !ctl->rebuild) return;
   int overflow = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    sort_list(nbr, nbr_cnt, maxnb, i, overflow);
+    if (!all_pairs) sort_list(nbr, nbr_cnt, maxnb, i, overflow);
     Seg s = seg[i];
     ref[i] = s.cx; ref[n + i] = s.cy; ref[2 * n + i] = s.cz;
     ref[3 * n + i] = s.ux; ref[4 * n + i] = s.uy; ref[5 * n + i] = s.uz;
@@ -655,11 +662,13 @@ void detect_launch(rg_system* s, double delta, bool check_rebuild, bool seg_read
   RGL launch_dep(k_cell_count_dyn, g, bs, st, d.seg, n, &dd->grid, s->box.pbc, d.cell_of, d.cell_cnt, ctl);
   s->scan.run(d.cell_cnt, d.cell_start, &dd->ncells, &ctl->err, st);
   RGL launch_dep(k_cell_fill, g, bs, st, n, d.cell_of, d.cell_start, d.cell_fill, d.cell_rods, ctl);
-  int gb = d.ncells < s->sm_count * 8 ? d.ncells : s->sm_count * 8;
+  // a block per home cell, or a warp per rod
+  const int gb = std::min(d.all_pairs ? grid_for(n * 32, kTile) : d.ncells, s->sm_count * 8);
   RGL launch_dep(k_build_lists, gb, kTile, st, d.seg, n, &dd->grid, s->box, d.cell_start, d.cell_rods,
                                        d.margin, d.skin, d.cut_center, d.all_pairs ? 1 : 0,
                                        d.nbr_cnt, d.nbr, d.maxnb, ctl);
-  RGL launch_dep(k_save_ref, g, bs, st, d.seg, n, d.ref, d.nbr, d.nbr_cnt, d.maxnb, ctl);
+  RGL launch_dep(k_save_ref, g, bs, st, d.seg, n, d.ref, d.nbr, d.nbr_cnt, d.maxnb,
+                 d.all_pairs ? 1 : 0, ctl);
   // --- near lists (every kernel below returns at once unless they are due) ---
   const int* lcnt = d.nbr_cnt;
   const int* lnbr = d.nbr;

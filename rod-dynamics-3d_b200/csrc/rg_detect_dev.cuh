@@ -138,15 +138,14 @@ __device__ inline bool seg_far(const Seg& A, const Seg& B, d3 d, double lim) {
 // conservative test as build_cell.
 __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const Box& box, const double* invL,
                                         const int* cell_start, const int* cell_rods, double margin,
-                                        double skin, int all_pairs, int* nbr_cnt, int* nbr, int maxnb,
-                                        int cell, BuildSmem& sm, unsigned* q1, unsigned* q2, int qcap,
-                                        int& overflow) {
+                                        double skin, int* nbr_cnt, int* nbr, int maxnb, int cell,
+                                        BuildSmem& sm, unsigned* q1, unsigned* q2, int qcap, int& overflow) {
   int cx = cell % g.n[0], cy = (cell / g.n[0]) % g.n[1], cz = cell / (g.n[0] * g.n[1]);
   // Half shell: the home cell (pairs j > i) and the 13 cells ahead of it
   // (every pair), each unordered pair met once and listed under its lower
   // index.  Needs distinct neighbour cells: three or more cells along every
-  // periodic axis, and not the all-pairs scan.
-  const bool half = !all_pairs && !(box.pbc && (g.n[0] < 3 || g.n[1] < 3 || g.n[2] < 3));
+  // periodic axis.
+  const bool half = !(box.pbc && (g.n[0] < 3 || g.n[1] < 3 || g.n[2] < 3));
   if (threadIdx.x == 0 && half) {
     int cnt = 0;
     const int c3[3] = {cx, cy, cz};
@@ -171,7 +170,7 @@ __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const 
     int lo[3], hi[3];
     int c3[3] = {cx, cy, cz};
     for (int k = 0; k < 3; ++k) {
-      if (box.pbc && (g.n[k] < 3 || all_pairs)) {
+      if (box.pbc && g.n[k] < 3) {
         lo[k] = 0; hi[k] = g.n[k] - 1;
       } else {
         lo[k] = c3[k] - 1; hi[k] = c3[k] + 1;
@@ -242,18 +241,6 @@ __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const 
           sm.tile.put(threadIdx.x, seg[j]);
         }
         __syncthreads();
-        if (all_pairs) {
-          // tiny periodic boxes: every pair is listed
-          if (!mine) continue;
-          for (int u = sub; u < m; u += G) {
-            const int j = sm.tidx[u];
-            if (j <= i) continue;
-            int pos = atomicAdd(&nbr_cnt[i], 1);
-            if (pos < maxnb) nbr[(size_t)i * maxnb + pos] = j;
-            else overflow = 1;
-          }
-          continue;
-        }
         // Three block-wide stages per round, each over compacted work, so a
         // warp's lanes run the same test: centre test of every candidate ->
         // queue q1; axial/line prefilter of q1 -> queue q2; exact distance
@@ -342,17 +329,15 @@ __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const 
 // Rod-parallel list build (one thread per home rod, no block barriers):
 // the candidates of rod i are the rods of its cell's neighbourhood, read
 // from the cell arrays; accepted j > i are appended to i's own list (sorted
-// afterwards by sort_list).  Same acceptance as build_cell_pairs.  Suits
-// sparse cells, where staging a tile per neighbouring cell costs a memory
-// round trip and a barrier for a handful of pairs.
+// afterwards by sort_list).  Same acceptance as build_cell_pairs.
 __device__ inline void build_rod_list(int i, const Seg* seg, const GridDev& g, const Box& box, const double* invL,
                                       const int* cell_of, const int* cell_start, const int* cell_rods, double margin,
-                                      double skin, int all_pairs, int* nbr_cnt, int* nbr, int maxnb, int& overflow) {
+                                      double skin, int* nbr_cnt, int* nbr, int maxnb, int& overflow) {
   const int cell = cell_of[i];
   const int c3[3] = {cell % g.n[0], (cell / g.n[0]) % g.n[1], cell / (g.n[0] * g.n[1])};
   int lo[3], hi[3];
   for (int k = 0; k < 3; ++k) {
-    if (box.pbc && (g.n[k] < 3 || all_pairs)) {
+    if (box.pbc && g.n[k] < 3) {
       lo[k] = 0; hi[k] = g.n[k] - 1;
     } else {
       lo[k] = c3[k] - 1; hi[k] = c3[k] + 1;
@@ -376,21 +361,38 @@ __device__ inline void build_rod_list(int i, const Seg* seg, const GridDev& g, c
           const int j = cell_rods[q];
           if (j <= i) continue;
           const Seg B = seg[j];
-          if (!all_pairs) {
-            const d3 d = centre_offset(A, B, box, invL);
-            const double cc = A.h + B.h + A.r + B.r + margin + skin;
-            if (dot(d, d) > cc * cc * (1.0 + 1e-9)) continue;
-            const double lim = A.r + B.r + margin + skin;
-            if (seg_far(A, B, d, lim)) continue;
-            const Narrow nr = narrow_pair(A, B, box);
-            if (!(nr.d2 < lim * lim)) continue;
-          }
+          const d3 d = centre_offset(A, B, box, invL);
+          const double cc = A.h + B.h + A.r + B.r + margin + skin;
+          if (dot(d, d) > cc * cc * (1.0 + 1e-9)) continue;
+          const double lim = A.r + B.r + margin + skin;
+          if (seg_far(A, B, d, lim)) continue;
+          const Narrow nr = narrow_pair(A, B, box);
+          if (!(nr.d2 < lim * lim)) continue;
           if (cnt < maxnb) L[cnt] = j;
           else overflow = 1;
           ++cnt;
         }
       }
   nbr_cnt[i] = cnt;
+}
+
+// All-pairs lists (periodic boxes too small for image-free cells): rod i lists
+// every j > i, written in order by one warp per rod, nothing left to sort.
+// Appended in cell order and sorted by one thread per rod afterwards, the
+// sort's moves grew with the square of a list: 1000 rods of aspect 40 took
+// 73 ms, written in order (and near lists drawn from them) 0.8, on 8 blocks.
+__device__ inline void list_all_pairs(int n, int warp, int nwarps, int* nbr_cnt, int* nbr, int maxnb,
+                                      int& overflow) {
+  const int lane = threadIdx.x & 31;
+  for (int i = warp; i < n; i += nwarps) {
+    int m = n - 1 - i;
+    if (m > maxnb) {
+      overflow = 1;
+      m = maxnb;
+    }
+    for (int k = lane; k < m; k += 32) nbr[(size_t)i * maxnb + k] = i + 1 + k;
+    if (lane == 0) nbr_cnt[i] = m;
+  }
 }
 
 // Sorts rod i's neighbour list ascending (insertion sort; lists are short).

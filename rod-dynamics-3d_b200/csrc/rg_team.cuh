@@ -174,8 +174,8 @@ __device__ inline bool team_excl_scan(const Team& T, const int* in, int* out, in
 // ---------------------------------------------------------------------------
 // Detection inside the persistent kernel.
 // ---------------------------------------------------------------------------
-static __device__ __noinline__ bool rebuild_phase(const Team& T, const NscView& V, SmemNsc& sm) {
-  Ctl* ctl = V.ctl;
+// Cell lists and the candidates within margin + skin of every rod (unordered).
+static __device__ bool build_lists(const Team& T, const NscView& V, SmemNsc& sm, int& overflow) {
   const int n = V.st.n;
   const int tid = T.tid(), TS = T.size(), rank = T.rank();
   if (!V.box.pbc) {
@@ -204,7 +204,6 @@ static __device__ __noinline__ bool rebuild_phase(const Team& T, const NscView& 
     }
     g.ncells = vg->ncells;
   }
-  unsigned long long t_start = (ctl->prof_phases && rank == 0 && threadIdx.x == 0) ? gtimer() : 0;
   for (int c = tid; c <= g.ncells; c += TS) {
     V.cell_cnt[c] = 0;
     V.cell_fill[c] = 0;
@@ -227,26 +226,42 @@ static __device__ __noinline__ bool rebuild_phase(const Team& T, const NscView& 
     V.cell_rods[V.cell_start[c] + atomicAdd(&V.cell_fill[c], 1)] = i;
   }
   if (!team_sync(T)) return false;
-  int overflow = 0;
   double invL[3] = {1.0, 1.0, 1.0};
   for (int k = 0; k < 3; ++k)
     if (V.box.L[k] > 0.0) invL[k] = 1.0 / V.box.L[k];
-  if (n < 48 * g.ncells) {
-    // sparse cells: one thread per home rod
+  // One thread per home rod where every block has thousands of rods of its
+  // own and a rod few candidates, else the block splits the pairs of one home
+  // cell at a time: a thread alone with its rod's candidates is a serial chain
+  // (1000 rods of aspect 10 on 8 blocks: 954 us by rod, 241 by cell; 5000 of
+  // aspect 10 on 40: 1425 and 275; 20000 of aspect 5 on 148: 743 and 221;
+  // 400000 of aspect 20, 46 rods a cell, on 148: 10.8 and 5.3 ms).  The two
+  // meet at 200000 rods of aspect 5 (1.60 and 1.66 ms); at a million of
+  // aspect 5 or 3, some 10 rods a cell, staging a tile for a handful of pairs
+  // costs more: 6.7 and 5.8 ms by rod, 8.3 and 10.2 by cell.
+  if (n < 16 * g.ncells && n > 2048 * T.nb) {
     for (int i = tid; i < n; i += TS)
       build_rod_list(i, V.seg, g, V.box, invL, V.cell_of, V.cell_start, V.cell_rods, V.margin, V.skin,
-                     V.all_pairs, V.nbr_cnt, V.nbr, V.maxnb, overflow);
+                     V.nbr_cnt, V.nbr, V.maxnb, overflow);
   } else {
-    // crowded cells: the block splits the pairs of one home cell at a time
     for (int cell = rank; cell < g.ncells; cell += T.nb)
-      build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin, V.all_pairs,
+      build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin,
                        V.nbr_cnt, V.nbr, V.maxnb, cell, *reinterpret_cast<BuildSmem*>(team_dyn_smem),
                        reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff),
                        reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff) + kBuildQ, kBuildQ, overflow);
   }
-  if (!team_sync(T)) return false;
+  return team_sync(T);
+}
+
+static __device__ __noinline__ bool rebuild_phase(const Team& T, const NscView& V, SmemNsc& sm) {
+  Ctl* ctl = V.ctl;
+  const int n = V.st.n;
+  const int tid = T.tid(), TS = T.size(), rank = T.rank();
+  unsigned long long t_start = (ctl->prof_phases && rank == 0 && threadIdx.x == 0) ? gtimer() : 0;
+  int overflow = 0;
+  if (V.all_pairs) list_all_pairs(n, tid >> 5, TS >> 5, V.nbr_cnt, V.nbr, V.maxnb, overflow);
+  else if (!build_lists(T, V, sm, overflow)) return false;
   for (int i = tid; i < n; i += TS) {
-    sort_list(V.nbr, V.nbr_cnt, V.maxnb, i, overflow);
+    if (!V.all_pairs) sort_list(V.nbr, V.nbr_cnt, V.maxnb, i, overflow);
     Seg s = V.seg[i];
     V.ref[i] = s.cx; V.ref[n + i] = s.cy; V.ref[2 * n + i] = s.cz;
     V.ref[3 * n + i] = s.ux; V.ref[4 * n + i] = s.uy; V.ref[5 * n + i] = s.uz;
