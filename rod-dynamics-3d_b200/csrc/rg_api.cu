@@ -1035,10 +1035,16 @@ int rg_compute_forces(rg_system* s, double* f, double* tau, double* pe) {
     Ctl* h = s->h_ctl;
     std::memcpy(h, sn.ctl.data(), s->ctl_bytes);
     h->err = 0;
+    h->ins_n[0] = h->ins_n[1] = 0;
     RG_TRY(cudaMemcpyAsync(s->d_ctl, h, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream), "ctl");
-    clear_forces_launch(s);
     s->contacts_fresh = Fresh::kNo;
-    force_eval_launch(s);
+    if (verlet_team_fits(s)) {
+      verlet_run_launch(s, 0);  // one launch (the multi-kernel evaluation: 24)
+    } else {
+      clear_forces_launch(s);
+      force_eval_launch(s);
+      s->contacts_fresh = Fresh::kCsr;
+    }
     RG_TRY(cudaGetLastError(), "force launch");
     RG_TRY(cudaMemcpyAsync(h, s->d_ctl, s->ctl_bytes, cudaMemcpyDeviceToHost, s->stream), "ctl");
     RG_TRY(cudaStreamSynchronize(s->stream), "forces");
@@ -1053,7 +1059,6 @@ int rg_compute_forces(rg_system* s, double* f, double* tau, double* pe) {
     RG_TRY(take_snapshot(s, sn), "snapshot");
     reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
   }
-  s->contacts_fresh = Fresh::kCsr;
   if (pe) *pe = s->h_ctl->pe;
   return rg_get_state(s, nullptr, nullptr, nullptr, nullptr, f, tau);
 }

@@ -444,7 +444,7 @@ __device__ inline void v_energy(const VerletView& W, int C, SmemNsc& sm) {
   __syncthreads();
 }
 
-// nsteps steps of one system by its team.
+// nsteps steps of one system by its team (0: one force evaluation).
 __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nsteps, VerletSmem& S) {
   const NscView& V = W.v;
   const State& st = V.st;
@@ -483,6 +483,22 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
   }
   // (every block has read the control words before the first one changes any)
   if (!team_sync(T)) return false;
+  if (nsteps == 0) {  // one force evaluation at the current state, kept in f and tau
+    ++r.fr;
+    if (!v_detect_eval(T, W, r, S, true)) return false;
+    if (!team_sync(T)) return false;
+    const int added = *(volatile int*)&ctl->ins_n[r.fr & 1];
+    for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+      d3 f{0, 0, 0}, tq{0, 0, 0};
+      v_body_sum(W, r, i, f, tq);
+      if (wall && st.inv_mass[i] > 0.0) soft_wall_apply(cfg, ax, st.r[i], st.x.ld(i), st.v.ld(i), f);
+      st.f.st(i, f);
+      st.tau.st(i, tq);
+    }
+    if (rank == 0) v_energy(W, r.C, S.s);
+    if (added && !v_insert(T, W, r, S, added)) return false;
+    if (!team_sync(T)) return false;
+  }
   for (int step = 0; step < nsteps; ++step) {
     const bool last = step == nsteps - 1;
     // forces at t: with the first detection, or on the contacts in place
@@ -657,7 +673,11 @@ void verlet_launch(const VerletView* views, const TeamDesc* teams, int nteams, c
 }
 
 void verlet_run_launch(rg_system* s, int nsteps) {
-  int nb = s->team_blocks > 0 ? s->team_blocks : (s->n + kVerletRodsPerBlock - 1) / kVerletRodsPerBlock;
+  // (a force evaluation alone crosses few barriers, so a new state's list
+  // build decides: four times the blocks; 1000 rods, first pass 435 -> 300 us,
+  // later ones the same)
+  const int per = nsteps > 0 ? kVerletRodsPerBlock : kVerletRodsPerBlock / 4;
+  int nb = s->team_blocks > 0 ? s->team_blocks : (s->n + per - 1) / per;
   if (nb > s->sm_count) nb = s->sm_count;
   const VerletView W = make_verlet_view(s);
   const TeamDesc td{0, nb, 0, 1, s->nsc.bar, nullptr};
