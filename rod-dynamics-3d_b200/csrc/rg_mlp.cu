@@ -21,22 +21,35 @@
 namespace rg {
 
 // ---------------------------------------------------------------------------
-// Training: one fused kernel per minibatch.  A block of kTrainWarps warps
-// takes tiles of kTrainRows rows (16 per warp) and runs, for its rows, the
-// forward pass (pre-activations Z kept in shared memory, activations in
-// registers: the accumulator fragment of a layer is the A fragment of the
-// next), the loss, the backward pass (dH = dZ W with W read transposed from
-// shared memory, dZ = dH * silu'(Z)) and the block's share of the weight
-// gradients dW = dZ^T H as block-level mma.sync products over the tile's
-// rows (H recomputed from Z).  Each block writes its partial gradient (and
-// loss) to its own slice of a partial buffer, summing over its tiles in a
-// fixed order; one reduction kernel then adds the slices in block order
-// (deterministic) and applies Adam and the BF16 weight copies.
+// Training: one fused kernel per minibatch.  A block takes tiles of kTrainRows
+// rows and runs, for its rows, the forward pass (pre-activations Z kept in
+// shared memory), the loss, the backward pass (dH = dZ W with W read
+// transposed from shared memory, dZ = dH * silu'(Z)) and the block's share of
+// the weight gradients dW = dZ^T H as block-level mma.sync products over the
+// tile's rows.  A row group of 16 rows belongs to kTrainCols warps, each with
+// its share of a layer's output columns; the BF16 activations pass between
+// them through the dZ buffers, which are free during the forward pass.  Each
+// block writes its partial gradient (and loss) to its own slice of a partial
+// buffer, summing over its tiles in a fixed order; one reduction kernel then
+// adds the slices in block order (deterministic) and applies Adam and the BF16
+// weight copies.
+//
+// Bound by the instructions of a minibatch's 64 blocks (a tile's chain of
+// products and its activations; the tensor pipe is idle most of the time).
+// One warp a row group recomputed silu(Z) for every m-tile of a weight
+// gradient and gathered transposed fragments by 16-bit loads: 157 us for 4096
+// rows from a cold L2.  Now silu is taken once more, in place of Z, fragments
+// come by ldmatrix, and four warps share a row group: 33 us; 65536 records, 4
+// epochs: 7.43 -> 4.29 ms (two warps a row group 4.7).
 // ---------------------------------------------------------------------------
-constexpr int kTrainWarps = 4;
+constexpr int kTrainGroups = 4;                   // row groups of 16 rows
+constexpr int kTrainCols = 4;                     // warps a row group
+constexpr int kTrainWarps = kTrainGroups * kTrainCols;
 constexpr int kTrainThreads = 32 * kTrainWarps;
-constexpr int kTrainRows = 16 * kTrainWarps;      // 64 rows per tile
-constexpr int kZLd = kMlpH + 8;                   // FP32 pre-activation rows (136)
+constexpr int kTrainRows = 16 * kTrainGroups;     // 64 rows per tile
+constexpr int kTrainNt = 16 / kTrainCols;         // n-tiles (8 columns) a warp
+constexpr int kZLd = kMlpH + 4;                   // FP32 pre-activation rows (132)
+constexpr int kHLd = 2 * kZLd;                    // BF16 activations in the place of Z
 constexpr int kXLd = kW1Pad + 8;                  // BF16 input rows (24)
 constexpr int kDyLd = 16;                         // BF16 output-gradient rows
 constexpr int kGradParams = kOffInMean;           // trained parameters
@@ -51,9 +64,9 @@ constexpr int kTsZ = kTsX + 2 * kTrainRows * kXLd;                     // Z1, Z2
 constexpr int kTsDzA = kTsZ + 3 * 4 * kTrainRows * kZLd;
 constexpr int kTsDzB = kTsDzA + 2 * kTrainRows * kWhLd;
 constexpr int kTsDy = kTsDzB + 2 * kTrainRows * kWhLd;
-constexpr int kTsBias = kTsDy + 2 * kTrainRows * kDyLd;                // [warp][b1|b2|b3|b4(8)]
-constexpr int kTsLoss = kTsBias + 4 * kTrainWarps * (3 * kMlpH + 8);
-constexpr int kTrainSmem = kTsLoss + 16 * kTrainWarps;
+constexpr int kTsBias = kTsDy + 2 * kTrainRows * kDyLd;                // [row group][b1|b2|b3|b4(8)]
+constexpr int kTsLoss = kTsBias + 4 * kTrainGroups * (3 * kMlpH + 8);
+constexpr int kTrainSmem = kTsLoss + 16 * kTrainGroups;
 static_assert(kTrainSmem <= 227 * 1024, "training kernel shared memory");
 static_assert(kTsSmall % 16 == 0 && kTsX % 16 == 0 && kTsZ % 16 == 0 && kTsDzA % 16 == 0 && kTsDzB % 16 == 0 &&
                   kTsDy % 16 == 0 && kTsBias % 16 == 0,
@@ -62,12 +75,12 @@ static_assert(kTsSmall % 16 == 0 && kTsX % 16 == 0 && kTsZ % 16 == 0 && kTsDzA %
 struct TrainSmem {
   __nv_bfloat16 *w2, *w3;  // [128][kWhLd]
   MlpStage st;             // W1 [128][kW1Ld], W4 [8][kWhLd], biases and scales
-  __nv_bfloat16* x;        // [64][kXLd] normalised inputs (columns 8..15 zero)
-  float* z[3];             // [64][kZLd] pre-activations of layers 1..3
-  __nv_bfloat16 *dza, *dzb;  // [64][kWhLd] BF16 dZ of two layers
+  __nv_bfloat16* x;        // [64][kXLd] normalised inputs (columns 0..7)
+  float* z[3];             // [64][kZLd] pre-activations of layers 1..3; then [64][kHLd] BF16 activations
+  __nv_bfloat16 *dza, *dzb;  // [64][kWhLd] BF16 dZ of two layers (forward: activations)
   __nv_bfloat16* dy;       // [64][kDyLd] BF16 dY (columns 3..15 zero)
-  float* bias;             // [warp][3 * 128 + 8] bias-gradient partial sums
-  float* loss;             // [warp]
+  float* bias;             // [row group][3 * 128 + 8] bias-gradient partial sums
+  float* loss;             // [row group]
 };
 __device__ inline TrainSmem train_smem(unsigned char* b) {
   TrainSmem s;
@@ -89,48 +102,47 @@ __device__ inline unsigned short bf16_bits(__nv_bfloat16 v) { return *reinterpre
 __device__ inline unsigned pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
   return (unsigned)bf16_bits(lo) | ((unsigned)bf16_bits(hi) << 16);
 }
-// B fragment of W^T for the backward product dH = dZ W (W row-major
-// [out][in] with leading dimension ldw): k = out (k-tile kt), n = in
-// (n-tile nt); elements of a register come from two rows of W.
-__device__ inline void load_bt(const __nv_bfloat16* W, int ldw, int nt, int kt, int lane, unsigned& b0,
-                               unsigned& b1) {
-  const int g = lane >> 2, t = lane & 3;
-  const int n = nt * 8 + g, k = kt * 16 + 2 * t;
-  b0 = pack2(W[(size_t)k * ldw + n], W[(size_t)(k + 1) * ldw + n]);
-  b1 = pack2(W[(size_t)(k + 8) * ldw + n], W[(size_t)(k + 9) * ldw + n]);
+// Four (two) 8 x 8 BF16 matrices from shared memory, lane l giving the address
+// of row l % 8 of matrix l / 8; trans: the transposed matrices' fragments.
+__device__ inline void ldm4(const __nv_bfloat16* row, unsigned (&f)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3])
+               : "r"((unsigned)__cvta_generic_to_shared(row)) : "memory");
+}
+__device__ inline void ldm4t(const __nv_bfloat16* row, unsigned (&f)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3])
+               : "r"((unsigned)__cvta_generic_to_shared(row)) : "memory");
+}
+__device__ inline void ldm2t(const __nv_bfloat16* row, unsigned& f0, unsigned& f1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
+               : "=r"(f0), "=r"(f1)
+               : "r"((unsigned)__cvta_generic_to_shared(row)) : "memory");
+}
+// Barrier of the warps of one row group.
+__device__ inline void group_sync(int rg) {
+  asm volatile("bar.sync %0, %1;" ::"r"(rg + 1), "r"(32 * kTrainCols) : "memory");
 }
 __device__ inline float silu_grad(float z) {
   const float s = 1.0f / (1.0f + __expf(-z));
   return s * (1.0f + z * (1.0f - s));
 }
-// Accumulator fragments (16 n-tiles) -> A fragments of the next product.
-__device__ inline void acc_to_a(const float (&c)[16][4], unsigned (&a)[8][4], bool act) {
-#pragma unroll
-  for (int kk = 0; kk < 8; ++kk) {
-    const float* p = c[2 * kk];
-    const float* q = c[2 * kk + 1];
-    if (act) {
-      a[kk][0] = pack_bf16(silu(p[0]), silu(p[1]));
-      a[kk][1] = pack_bf16(silu(p[2]), silu(p[3]));
-      a[kk][2] = pack_bf16(silu(q[0]), silu(q[1]));
-      a[kk][3] = pack_bf16(silu(q[2]), silu(q[3]));
-    } else {
-      a[kk][0] = pack_bf16(p[0], p[1]);
-      a[kk][1] = pack_bf16(p[2], p[3]);
-      a[kk][2] = pack_bf16(q[0], q[1]);
-      a[kk][3] = pack_bf16(q[2], q[3]);
-    }
-  }
-}
-// Stores a warp's 16 x 128 FP32 accumulator block at rows lr0.. of Z.
-__device__ inline void store_z(float* z, int lr0, const float (&c)[16][4], int lane) {
+// A warp's accumulator block (16 rows from lr0, columns from c0) as FP32 rows
+// of Z, and its BF16 activations as rows of h.
+__device__ inline void store_zh(float* z, __nv_bfloat16* h, int lr0, int c0, const float (&c)[kTrainNt][4], int lane) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
-    const int col = nt * 8 + 2 * t;
-    *reinterpret_cast<float2*>(&z[(size_t)(lr0 + g) * kZLd + col]) = make_float2(c[nt][0], c[nt][1]);
-    *reinterpret_cast<float2*>(&z[(size_t)(lr0 + g + 8) * kZLd + col]) = make_float2(c[nt][2], c[nt][3]);
+  for (int nt = 0; nt < kTrainNt; ++nt) {
+    const int col = c0 + nt * 8 + 2 * t;
+    *reinterpret_cast<float2*>(&z[(lr0 + g) * kZLd + col]) = make_float2(c[nt][0], c[nt][1]);
+    *reinterpret_cast<float2*>(&z[(lr0 + g + 8) * kZLd + col]) = make_float2(c[nt][2], c[nt][3]);
+    *reinterpret_cast<unsigned*>(&h[(lr0 + g) * kWhLd + col]) = pack_bf16(silu(c[nt][0]), silu(c[nt][1]));
+    *reinterpret_cast<unsigned*>(&h[(lr0 + g + 8) * kWhLd + col]) = pack_bf16(silu(c[nt][2]), silu(c[nt][3]));
   }
+}
+// A fragment of rows lr0.. of x (BF16 [64][kWhLd]), k-tile kt.
+__device__ inline void load_a(const __nv_bfloat16* x, int lr0, int kt, int lane, unsigned (&a)[4]) {
+  ldm4(x + (lr0 + (lane & 15)) * kWhLd + kt * 16 + (lane >> 4) * 8, a);
 }
 
 __device__ inline float warp_sum_f(float v) {
@@ -142,48 +154,42 @@ __device__ inline float warp_sum_f(float v) {
 __device__ inline void part_put(float* p, int i, float v, bool first) { p[i] = first ? v : p[i] + v; }
 
 // Block-level weight gradient dW[o][i] = Σ_r dZ[r][o] H[r][i] over the
-// tile's 64 rows: output rows o in m-tiles [0, mtiles) (warp w takes m-tiles
-// w, w + 4, ...), input columns [0, 8 * NTN).  dZ: BF16 rows of leading
-// dimension ldz.  H: the BF16 copy of silu(Z) (Z FP32 [64][kZLd]) or, when
-// zs is null, the BF16 inputs xs [64][kXLd].  Rows o < nrows and columns
-// i < ncols go to part[off + o * ncols + i].
+// tile's 64 rows: output rows o in m-tiles [0, mtiles), input columns in
+// ngroups groups of NTN n-tiles; the warps take the (m-tile, group) products
+// in turn.  dZ, H: BF16 rows of leading dimensions ldz and ldh.  Rows
+// o < nrows and columns i < ncols go to part[off + o * ncols + i].
 template <int NTN>
-__device__ inline void block_dw(const __nv_bfloat16* dz, int ldz, int mtiles, int nrows, const float* zs,
-                                const __nv_bfloat16* xs, int ncols, float* part, int off, bool first, int warp,
+__device__ inline void block_dw(const __nv_bfloat16* dz, int ldz, int mtiles, int nrows, const __nv_bfloat16* h,
+                                int ldh, int ngroups, int ncols, float* part, int off, bool first, int warp,
                                 int lane) {
   const int g = lane >> 2, t = lane & 3;
-  for (int mt = warp; mt < mtiles; mt += kTrainWarps) {
-    const int m0 = mt * 16;
+  for (int u = warp; u < mtiles * ngroups; u += kTrainWarps) {
+    const int m0 = (u / ngroups) * 16, n0 = (u % ngroups) * NTN * 8;
     float c[NTN][4];
 #pragma unroll
     for (int j = 0; j < NTN; ++j) c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.0f;
 #pragma unroll
     for (int ks = 0; ks < kTrainRows / 16; ++ks) {
-      const int r = ks * 16 + 2 * t;
-      const __nv_bfloat16* d0 = dz + (size_t)r * ldz + m0 + g;
-      const unsigned a0 = pack2(d0[0], d0[ldz]);
-      const unsigned a1 = pack2(d0[8], d0[ldz + 8]);
-      const unsigned a2 = pack2(d0[8 * ldz], d0[9 * ldz]);
-      const unsigned a3 = pack2(d0[8 * ldz + 8], d0[9 * ldz + 8]);
-#pragma unroll
-      for (int j = 0; j < NTN; ++j) {
-        const int n = j * 8 + g;
+      unsigned a[4];
+      ldm4t(dz + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * ldz + m0 + ((lane >> 3) & 1) * 8, a);
+      const __nv_bfloat16* hr = h + (ks * 16 + (lane & 15)) * ldh + n0;
+      if constexpr (NTN == 1) {
         unsigned b0, b1;
-        if (zs) {
-          const float* z0 = zs + (size_t)r * kZLd + n;
-          b0 = pack_bf16(silu(z0[0]), silu(z0[kZLd]));
-          b1 = pack_bf16(silu(z0[8 * kZLd]), silu(z0[9 * kZLd]));
-        } else {
-          const __nv_bfloat16* x0 = xs + (size_t)r * kXLd + n;
-          b0 = pack2(x0[0], x0[kXLd]);
-          b1 = pack2(x0[8 * kXLd], x0[9 * kXLd]);
+        ldm2t(hr, b0, b1);
+        mma_bf16(c[0], a[0], a[1], a[2], a[3], b0, b1);
+      } else {
+#pragma unroll
+        for (int j = 0; j < NTN; j += 2) {
+          unsigned b[4];
+          ldm4t(hr + j * 8 + (lane >> 4) * 8, b);
+          mma_bf16(c[j], a[0], a[1], a[2], a[3], b[0], b[1]);
+          mma_bf16(c[j + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
         }
-        mma_bf16(c[j], a0, a1, a2, a3, b0, b1);
       }
     }
 #pragma unroll
     for (int j = 0; j < NTN; ++j) {
-      const int col = j * 8 + 2 * t;
+      const int col = n0 + j * 8 + 2 * t;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int o = m0 + g + (e >= 2 ? 8 : 0), i = col + (e & 1);
@@ -193,13 +199,12 @@ __device__ inline void block_dw(const __nv_bfloat16* dz, int ldz, int mtiles, in
   }
 }
 
-// Column sums over a warp's 16 rows of a 16 x 128 FP32 fragment block,
-// added to sums[0..127] ('=' on the block's first tile); lanes with g = 0
-// write.
-__device__ inline void warp_colsum_acc(const float (&c)[16][4], float* sums, int lane, bool first) {
+// Column sums over a warp's 16 rows of its FP32 fragment block, added to
+// sums[c0..] ('=' on the block's first tile); lanes with g = 0 write.
+__device__ inline void warp_colsum_acc(const float (&c)[kTrainNt][4], float* sums, int c0, int lane, bool first) {
   const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
+  for (int nt = 0; nt < kTrainNt; ++nt) {
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       float v = c[nt][cc] + c[nt][2 + cc];
@@ -207,68 +212,81 @@ __device__ inline void warp_colsum_acc(const float (&c)[16][4], float* sums, int
       v += __shfl_xor_sync(0xffffffffu, v, 8);
       v += __shfl_xor_sync(0xffffffffu, v, 16);
       if (g == 0) {
-        float* s = &sums[nt * 8 + 2 * t + cc];
+        float* s = &sums[c0 + nt * 8 + 2 * t + cc];
         *s = first ? v : *s + v;
       }
     }
   }
 }
 
-// dZ = dH * silu'(Z) in place on the accumulator block (Z rows lr0..), and
-// its BF16 copy into dzs.
-__device__ inline void dz_from_dh(float (&c)[16][4], const float* z, __nv_bfloat16* dzs, int lr0, int lane) {
-  const int g = lane >> 2, t = lane & 3;
+// dZ = dH * silu'(Z) in place on the accumulator block (Z rows lr0..), its
+// BF16 copy into dzs, and, once the whole row group has read its Z, the BF16
+// activations silu(Z) in Z's place.
+__device__ inline void dz_from_dh(float (&c)[kTrainNt][4], float* z, __nv_bfloat16* dzs, int rg, int c0, int lane) {
+  const int g = lane >> 2, t = lane & 3, lr0 = 16 * rg;
+  unsigned h[kTrainNt][2];
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
-    const int col = nt * 8 + 2 * t;
-    const float2 z0 = *reinterpret_cast<const float2*>(&z[(size_t)(lr0 + g) * kZLd + col]);
-    const float2 z1 = *reinterpret_cast<const float2*>(&z[(size_t)(lr0 + g + 8) * kZLd + col]);
+  for (int nt = 0; nt < kTrainNt; ++nt) {
+    const int col = c0 + nt * 8 + 2 * t;
+    const float2 z0 = *reinterpret_cast<const float2*>(&z[(lr0 + g) * kZLd + col]);
+    const float2 z1 = *reinterpret_cast<const float2*>(&z[(lr0 + g + 8) * kZLd + col]);
     c[nt][0] *= silu_grad(z0.x);
     c[nt][1] *= silu_grad(z0.y);
     c[nt][2] *= silu_grad(z1.x);
     c[nt][3] *= silu_grad(z1.y);
-    *reinterpret_cast<unsigned*>(&dzs[(size_t)(lr0 + g) * kWhLd + col]) = pack_bf16(c[nt][0], c[nt][1]);
-    *reinterpret_cast<unsigned*>(&dzs[(size_t)(lr0 + g + 8) * kWhLd + col]) = pack_bf16(c[nt][2], c[nt][3]);
+    h[nt][0] = pack_bf16(silu(z0.x), silu(z0.y));
+    h[nt][1] = pack_bf16(silu(z1.x), silu(z1.y));
+    *reinterpret_cast<unsigned*>(&dzs[(lr0 + g) * kWhLd + col]) = pack_bf16(c[nt][0], c[nt][1]);
+    *reinterpret_cast<unsigned*>(&dzs[(lr0 + g + 8) * kWhLd + col]) = pack_bf16(c[nt][2], c[nt][3]);
+  }
+  group_sync(rg);
+  __nv_bfloat16* hz = reinterpret_cast<__nv_bfloat16*>(z);
+#pragma unroll
+  for (int nt = 0; nt < kTrainNt; ++nt) {
+    const int col = c0 + nt * 8 + 2 * t;
+    *reinterpret_cast<unsigned*>(&hz[(lr0 + g) * kHLd + col]) = h[nt][0];
+    *reinterpret_cast<unsigned*>(&hz[(lr0 + g + 8) * kHLd + col]) = h[nt][1];
   }
 }
-// dH = dZ W for a warp's 16 rows: dZ A fragments from dzs (BF16 rows lr0..),
-// W staged [out][kWhLd].
-__device__ inline void dh_product(const __nv_bfloat16* dzs, int lr0, const __nv_bfloat16* W, float (&c)[16][4],
-                                  int lane) {
-  const int g = lane >> 2, t = lane & 3;
+// dH = dZ W for a warp's 16 rows and columns c0..: dZ A fragments from dzs
+// (BF16 rows lr0..), W staged [out][kWhLd].
+__device__ inline void dh_product(const __nv_bfloat16* dzs, int lr0, const __nv_bfloat16* W, int c0,
+                                  float (&c)[kTrainNt][4], int lane) {
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
+  for (int nt = 0; nt < kTrainNt; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
 #pragma unroll
   for (int kt = 0; kt < 8; ++kt) {
-    const __nv_bfloat16* r0 = dzs + (size_t)(lr0 + g) * kWhLd + kt * 16 + 2 * t;
-    const __nv_bfloat16* r1 = r0 + 8 * kWhLd;
-    const unsigned a0 = *reinterpret_cast<const unsigned*>(r0), a1 = *reinterpret_cast<const unsigned*>(r1);
-    const unsigned a2 = *reinterpret_cast<const unsigned*>(r0 + 8), a3 = *reinterpret_cast<const unsigned*>(r1 + 8);
+    unsigned a[4];
+    load_a(dzs, lr0, kt, lane, a);
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt) {
-      unsigned b0, b1;
-      load_bt(W, kWhLd, nt, kt, lane, b0, b1);
-      mma_bf16(c[nt], a0, a1, a2, a3, b0, b1);
+    for (int nt = 0; nt < kTrainNt; nt += 2) {
+      unsigned b[4];  // k = out, n = in: the transposed fragments of two n-tiles
+      ldm4t(W + (kt * 16 + (lane & 15)) * kWhLd + c0 + nt * 8 + (lane >> 4) * 8, b);
+      mma_bf16(c[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
+      mma_bf16(c[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
     }
   }
 }
-// Forward through one hidden layer from A fragments a (16 x 128) with W
-// staged [out][kWhLd]: c = a W^T + bias (FP32).
-__device__ inline void fwd_product(const unsigned (&a)[8][4], const __nv_bfloat16* W, const float* bias,
-                                   float (&c)[16][4], int lane) {
+// Forward through one hidden layer from BF16 rows h (lr0..), columns c0..,
+// with W staged [out][kWhLd]: c = h W^T + bias (FP32).
+__device__ inline void fwd_product(const __nv_bfloat16* h, int lr0, const __nv_bfloat16* W, const float* bias, int c0,
+                                   float (&c)[kTrainNt][4], int lane) {
   const int t = lane & 3;
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
-    const float bl = bias[nt * 8 + 2 * t], bh = bias[nt * 8 + 2 * t + 1];
+  for (int nt = 0; nt < kTrainNt; ++nt) {
+    const float bl = bias[c0 + nt * 8 + 2 * t], bh = bias[c0 + nt * 8 + 2 * t + 1];
     c[nt][0] = bl; c[nt][1] = bh; c[nt][2] = bl; c[nt][3] = bh;
   }
 #pragma unroll
   for (int kt = 0; kt < 8; ++kt) {
+    unsigned a[4];
+    load_a(h, lr0, kt, lane, a);
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt) {
-      unsigned b0, b1;
-      load_b(W, kWhLd, nt, kt, lane, b0, b1);
-      mma_bf16(c[nt], a[kt][0], a[kt][1], a[kt][2], a[kt][3], b0, b1);
+    for (int nt = 0; nt < kTrainNt; nt += 2) {
+      unsigned b[4];  // two n-tiles
+      ldm4(W + (c0 + nt * 8 + (lane & 7) + (lane >> 4) * 8) * kWhLd + kt * 16 + ((lane >> 3) & 1) * 8, b);
+      mma_bf16(c[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
+      mma_bf16(c[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
     }
   }
 }
@@ -293,13 +311,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   float* mypart = part + (size_t)blockIdx.x * kGradParams;
   const int ntiles = (n + kTrainRows - 1) / kTrainRows;
   const float inv_n3 = 1.0f / (float)(n * kMlpOut);
-  const int lr0 = warp * 16;
-  float* bsum = S.bias + warp * (3 * kMlpH + 8);
+  const int rg = warp & (kTrainGroups - 1), lr0 = 16 * rg;           // row group
+  const int cg = warp / kTrainGroups, c0 = cg * kTrainNt * 8;        // column group
+  float* bsum = S.bias + rg * (3 * kMlpH + 8);
   float lsum = 0.0f;
   bool first = true;
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, first = false) {
     const int row0 = tile * kTrainRows;
-    // ---- forward (per warp, rows lr0..lr0+15 of the tile) ----
+    // ---- forward (rows lr0..lr0+15 of the tile, columns c0..) ----
     unsigned x0, x1;
     {
       float v[4];
@@ -312,31 +331,31 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
           const int k = 2 * t + cc;
           v[rr * 2 + cc] = r < n ? (feat[(size_t)rid * kMlpIn + k] - q.in_mean[k]) * q.in_scale[k] : 0.0f;
         }
-        *reinterpret_cast<unsigned*>(&S.x[(size_t)lr * kXLd + 2 * t]) = pack_bf16(v[rr * 2], v[rr * 2 + 1]);
-        *reinterpret_cast<unsigned*>(&S.x[(size_t)lr * kXLd + 8 + 2 * t]) = 0u;
+        if (cg == 0) *reinterpret_cast<unsigned*>(&S.x[(size_t)lr * kXLd + 2 * t]) = pack_bf16(v[rr * 2], v[rr * 2 + 1]);
       }
       x0 = pack_bf16(v[0], v[1]);
       x1 = pack_bf16(v[2], v[3]);
     }
-    unsigned a[8][4];
-    float c[16][4];
+    float c[kTrainNt][4];
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt) {
-      const float bl = q.b1[nt * 8 + 2 * t], bh = q.b1[nt * 8 + 2 * t + 1];
+    for (int nt = 0; nt < kTrainNt; ++nt) {
+      const int col = c0 + nt * 8 + 2 * t;
+      const float bl = q.b1[col], bh = q.b1[col + 1];
       c[nt][0] = bl; c[nt][1] = bh; c[nt][2] = bl; c[nt][3] = bh;
       unsigned b0, b1;
-      load_b(S.st.w1, kW1Ld, nt, 0, lane, b0, b1);
+      load_b(S.st.w1, kW1Ld, cg * kTrainNt + nt, 0, lane, b0, b1);
       mma_bf16(c[nt], x0, x1, 0u, 0u, b0, b1);
     }
-    store_z(S.z[0], lr0, c, lane);
-    acc_to_a(c, a, true);
-    fwd_product(a, S.w2, q.b2, c, lane);
-    store_z(S.z[1], lr0, c, lane);
-    acc_to_a(c, a, true);
-    fwd_product(a, S.w3, q.b3, c, lane);
-    store_z(S.z[2], lr0, c, lane);
-    acc_to_a(c, a, true);
-    // output layer, loss and dY (outputs 2t, 2t + 1 of rows g, g + 8)
+    store_zh(S.z[0], S.dza, lr0, c0, c, lane);
+    group_sync(rg);
+    fwd_product(S.dza, lr0, S.w2, q.b2, c0, c, lane);
+    store_zh(S.z[1], S.dzb, lr0, c0, c, lane);
+    group_sync(rg);  // (and no warp of the group reads dza any more)
+    fwd_product(S.dzb, lr0, S.w3, q.b3, c0, c, lane);
+    store_zh(S.z[2], S.dza, lr0, c0, c, lane);
+    group_sync(rg);
+    // output layer, loss and dY (outputs 2t, 2t + 1 of rows g, g + 8), by every
+    // warp of the row group; the first one keeps them
     float dy[4];
     {
       float y[4];
@@ -344,9 +363,10 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       y[0] = bl; y[1] = bh; y[2] = bl; y[3] = bh;
 #pragma unroll
       for (int kt = 0; kt < 8; ++kt) {
-        unsigned b0, b1;
+        unsigned a[4], b0, b1;
+        load_a(S.dza, lr0, kt, lane, a);
         load_b(S.st.w4, kWhLd, 0, kt, lane, b0, b1);
-        mma_bf16(y, a[kt][0], a[kt][1], a[kt][2], a[kt][3], b0, b1);
+        mma_bf16(y, a[0], a[1], a[2], a[3], b0, b1);
       }
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
@@ -359,13 +379,15 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
           if (o < kMlpOut && r < n) {
             const float tn = (tgt[(size_t)rid * kMlpOut + o] - feat[(size_t)rid * kMlpIn + 4 + o]) / q.out_scale[o];
             const float diff = y[rr * 2 + cc] - tn;
-            lsum += diff * diff;
+            if (cg == 0) lsum += diff * diff;
             d = 2.0f * diff * inv_n3;
           }
           dy[rr * 2 + cc] = d;
         }
-        *reinterpret_cast<unsigned*>(&S.dy[(size_t)lr * kDyLd + 2 * t]) = pack_bf16(dy[rr * 2], dy[rr * 2 + 1]);
-        *reinterpret_cast<unsigned*>(&S.dy[(size_t)lr * kDyLd + 8 + 2 * t]) = 0u;
+        if (cg == 0) {
+          *reinterpret_cast<unsigned*>(&S.dy[(size_t)lr * kDyLd + 2 * t]) = pack_bf16(dy[rr * 2], dy[rr * 2 + 1]);
+          *reinterpret_cast<unsigned*>(&S.dy[(size_t)lr * kDyLd + 8 + 2 * t]) = 0u;
+        }
       }
     }
     // ---- backward through the output layer: db4, dH3 = dY W4 ----
@@ -376,57 +398,60 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         v += __shfl_xor_sync(0xffffffffu, v, 4);
         v += __shfl_xor_sync(0xffffffffu, v, 8);
         v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if (g == 0) {
+        if (g == 0 && cg == 0) {
           float* s = &bsum[3 * kMlpH + 2 * t + cc];
           *s = first ? v : *s + v;
         }
       }
       const unsigned ya0 = pack_bf16(dy[0], dy[1]), ya1 = pack_bf16(dy[2], dy[3]);
 #pragma unroll
-      for (int nt = 0; nt < 16; ++nt) {
+      for (int nt = 0; nt < kTrainNt; ++nt) {
         c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
-        const int nn = nt * 8 + g;
+        const int nn = c0 + nt * 8 + g;
         const unsigned b0 = pack2(S.st.w4[(size_t)(2 * t) * kWhLd + nn], S.st.w4[(size_t)(2 * t + 1) * kWhLd + nn]);
         mma_bf16(c[nt], ya0, ya1, 0u, 0u, b0, 0u);
       }
     }
+    group_sync(rg);  // every warp of the group has read H3 in dza
     // layer 3: dZ3 -> dza, db3; dH2 = dZ3 W3
-    dz_from_dh(c, S.z[2], S.dza, lr0, lane);
-    warp_colsum_acc(c, bsum + 2 * kMlpH, lane, first);
-    __syncwarp();
-    dh_product(S.dza, lr0, S.w3, c, lane);
+    dz_from_dh(c, S.z[2], S.dza, rg, c0, lane);
+    warp_colsum_acc(c, bsum + 2 * kMlpH, c0, lane, first);
+    dh_product(S.dza, lr0, S.w3, c0, c, lane);
     // layer 2: dZ2 -> dzb, db2
-    dz_from_dh(c, S.z[1], S.dzb, lr0, lane);
-    warp_colsum_acc(c, bsum + kMlpH, lane, first);
-    __syncthreads();  // every warp's dZ3, dZ2 and dY are in shared memory
-    block_dw<16>(S.dza, kWhLd, kMlpH / 16, kMlpH, S.z[1], nullptr, kMlpH, mypart, kOffW3, first, warp, lane);
-    block_dw<16>(S.dy, kDyLd, 1, kMlpOut, S.z[2], nullptr, kMlpH, mypart, kOffW4, first, warp, lane);
+    dz_from_dh(c, S.z[1], S.dzb, rg, c0, lane);
+    warp_colsum_acc(c, bsum + kMlpH, c0, lane, first);
+    __syncthreads();  // every warp's dZ3, dZ2, dY, H3 and H2 are in shared memory
+    const __nv_bfloat16* h1 = reinterpret_cast<const __nv_bfloat16*>(S.z[0]);
+    const __nv_bfloat16* h2 = reinterpret_cast<const __nv_bfloat16*>(S.z[1]);
+    const __nv_bfloat16* h3 = reinterpret_cast<const __nv_bfloat16*>(S.z[2]);
+    block_dw<8>(S.dza, kWhLd, kMlpH / 16, kMlpH, h2, kHLd, 2, kMlpH, mypart, kOffW3, first, warp, lane);
+    block_dw<1>(S.dy, kDyLd, 1, kMlpOut, h3, kHLd, 16, kMlpH, mypart, kOffW4, first, warp, lane);
     __syncthreads();  // dza is free again
     // layer 1: dH1 = dZ2 W2, dZ1 -> dza, db1
-    dh_product(S.dzb, lr0, S.w2, c, lane);
-    dz_from_dh(c, S.z[0], S.dza, lr0, lane);
-    warp_colsum_acc(c, bsum, lane, first);
+    dh_product(S.dzb, lr0, S.w2, c0, c, lane);
+    dz_from_dh(c, S.z[0], S.dza, rg, c0, lane);
+    warp_colsum_acc(c, bsum, c0, lane, first);
     __syncthreads();
-    block_dw<16>(S.dzb, kWhLd, kMlpH / 16, kMlpH, S.z[0], nullptr, kMlpH, mypart, kOffW2, first, warp, lane);
-    block_dw<2>(S.dza, kWhLd, kMlpH / 16, kMlpH, nullptr, S.x, kMlpIn, mypart, kOffW1, first, warp, lane);
+    block_dw<8>(S.dzb, kWhLd, kMlpH / 16, kMlpH, h1, kHLd, 2, kMlpH, mypart, kOffW2, first, warp, lane);
+    block_dw<1>(S.dza, kWhLd, kMlpH / 16, kMlpH, S.x, kXLd, 1, kMlpIn, mypart, kOffW1, first, warp, lane);
     __syncthreads();  // shared tiles are reused by the next tile
   }
-  // bias gradients and loss: sum the warps' partial sums in warp order
+  // bias gradients and loss: sum the row groups' partial sums in order
   lsum = warp_sum_f(lsum);
-  if (lane == 0) S.loss[warp] = lsum;
+  if (lane == 0 && cg == 0) S.loss[rg] = lsum;
   __syncthreads();
   const bool any = blockIdx.x < ntiles;
   for (int i = threadIdx.x; i < 3 * kMlpH + kMlpOut; i += blockDim.x) {
     float v = 0.0f;
     if (any)
-      for (int w = 0; w < kTrainWarps; ++w) v += S.bias[w * (3 * kMlpH + 8) + i];
+      for (int w = 0; w < kTrainGroups; ++w) v += S.bias[w * (3 * kMlpH + 8) + i];
     const int off = i < kMlpH ? kOffB1 + i : i < 2 * kMlpH ? kOffB2 + i - kMlpH
                   : i < 3 * kMlpH ? kOffB3 + i - 2 * kMlpH : kOffB4 + i - 3 * kMlpH;
     mypart[off] = v;
   }
   if (threadIdx.x == 0) {
     float l = 0.0f;
-    for (int w = 0; w < kTrainWarps; ++w) l += S.loss[w];
+    for (int w = 0; w < kTrainGroups; ++w) l += S.loss[w];
     loss_part[blockIdx.x] = any ? l : 0.0f;
   }
   if (!any) {  // a block without a tile contributes zero weight gradients
@@ -441,6 +466,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 // g_i = Σ_b part[b][i] in block order (deterministic), i < kGradParams.
 __device__ inline float grad_sum(const float* part, int nblk, int i) {
   float g = 0.0f;
+#pragma unroll 16
   for (int b = 0; b < nblk; ++b) g += part[(size_t)b * kGradParams + i];
   return g;
 }
