@@ -32,7 +32,8 @@ def build(ref=True):
     """Compiles the oracle (and the reference's CPU and CUDA sources, when
     its tree is present)."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-    if ref and os.path.isdir(REF_TREE):
+    # (an empty folder of that name is not a checkout)
+    if ref and os.path.isfile(os.path.join(REF_TREE, "src", "physics", "rigid_body.cpp")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", "refcuda", f"REF={REF_TREE}"], check=True)
 
 
