@@ -27,10 +27,9 @@
 // 2 us each) up to some 50,000 rods, then the two passes over the body state.
 // Measured, multi-kernel form (one captured graph a step) -> this one, us per
 // step: 1,000 rods 80 -> 33, 5,000 (soft) 104 -> 38, 20,000 103 -> 41, 100,000
-// 130 -> 61, 400,000 279 -> 167, 1,000,000 441 -> 320 (5,000 contacts) and 641
-// -> 389 (80,000 contacts).  It is the faster one at every size, so the
-// multi-kernel form only serves the stage timers, single force evaluations
-// and detections.
+// 130 -> 61, 400,000 279 -> 163, 1,000,000 441 -> 299 (5,000 contacts) and 641
+// -> 360 (80,000 contacts).  It is the faster one at every size, so the
+// multi-kernel form only serves the stage timers and contact queries.
 #include <cstring>
 #include <vector>
 
@@ -240,6 +239,33 @@ __device__ inline void v_body_sum(const VerletView& W, const VerletRun& r, int i
   }
 }
 
+// Rod i's records on their way to L2: a thread's next rod, while the present
+// one is worked on.  With thousands of rods a block the state is streamed from
+// memory each phase, and 16 warps (128 registers a thread) do not cover its
+// latency: a million rods 350 -> 332 us a step, 325 with the next pairs'
+// segments in the detection too; up to 20000 rods (one turn a thread) the
+// same.  Loading the next values into registers spilled: 365.
+__device__ inline void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ inline void v_prefetch(const VerletView& W, const VerletRun& r, int i, bool drift, const DriftOut& o) {
+  const State& st = W.v.st;
+  const int n = st.n;
+  prefetch_l2(W.head + i);
+  prefetch_l2(W.first[r.cb] + i);
+  prefetch_l2(st.inv_mass + i);
+  prefetch_l2(st.mass + i);
+  auto p3 = [&](const auto& a) { prefetch_l2(a.x + i); prefetch_l2(a.y + i); prefetch_l2(a.z + i); };
+  p3(st.v); p3(st.w); p3(st.I);
+  prefetch_l2(st.q.w + i); p3(st.q);
+  if (!drift) return;
+  p3(st.x);
+  prefetch_l2(st.h + i);
+  prefetch_l2(st.r + i);
+  for (int k = 0; k < 6; ++k) {
+    if (o.ref) prefetch_l2(o.ref + (size_t)k * n + i);
+    if (o.ref2) prefetch_l2(o.ref2 + (size_t)k * n + i);
+  }
+}
+
 // The largest displacement bounds of the block's rods.
 __device__ inline void v_publish_disp(const NscView& V, double m, double m2, SmemNsc& sm) {
   m = block_reduce_max(m, sm.red_d);
@@ -341,11 +367,20 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
   unsigned* bits = reinterpret_cast<unsigned*>(V.mask);
   const double* im = V.st.inv_mass;
   int mine = 0;
+  const int ahead = blockDim.x;  // a thread's next pair, its segments on their way to L2
+  int2 pr{0, 0}, next{0, 0};
+  if (plo + t < phi) pr = W.flat[plo + t];
+  if (plo + t + ahead < phi) next = W.flat[plo + t + ahead];
   for (int p0 = plo; p0 < phi; p0 += blockDim.x) {
     const int p = p0 + t;
     bool hit = false;
+    int2 after{0, 0};
+    if (p + ahead < phi) {
+      prefetch_l2(V.seg + next.x);
+      prefetch_l2(V.seg + next.y);
+      if (p + 2 * ahead < phi) after = W.flat[p + 2 * ahead];
+    }
     if (p < phi) {
-      const int2 pr = W.flat[p];
       if (im[pr.x] > 0.0 || im[pr.y] > 0.0) {
         const Seg A = V.seg[pr.x], B = V.seg[pr.y];
         const Narrow nr = narrow_pair(A, B, V.box);
@@ -357,6 +392,8 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
       bits[p >> 5] = word;
       mine += __popc(word);
     }
+    pr = next;
+    next = after;
   }
   const int bsum = block_reduce_sum_i(mine, S.s.red_i);
   if (t == 0) V.blk[rank] = bsum;
@@ -517,6 +554,7 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
       if (rank == 0 && t == 0) ctl->ins_n[(r.fr + 1) & 1] = 0;
       double m = 0.0, m2 = 0.0;
       for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+        if (i + (int)blockDim.x < r.hi) v_prefetch(W, r, i + blockDim.x, true, out);
         d3 f{0, 0, 0}, tq{0, 0, 0};
         if (st.inv_mass[i] > 0.0) v_body_sum(W, r, i, f, tq);
         W.head[i] = -1;  // for the detection that follows
@@ -537,6 +575,7 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
       if (rank == 0 && t == 0) ctl->ins_n[(r.fr + 1) & 1] = 0;
       int bad = 0;
       for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
+        if (i + (int)blockDim.x < r.hi) v_prefetch(W, r, i + blockDim.x, false, out);
         d3 f{0, 0, 0}, tq{0, 0, 0};
         v_body_sum(W, r, i, f, tq);
         bad |= kick_rod(st, cfg, ax, wall, i, f, tq, el, ea);

@@ -46,6 +46,7 @@ SOFT = dict(model="harmonic", dt=1e-4, soft_damping=0.3, soft_friction_mode="cun
     (580, 0.05, 0.08, 0.9, 0, {}),                      # every pair listed, near lists drawn from them
     (300, 0.1, 0.05, 0.9, 1, dict(pbc_enabled=0)),      # open box, one block
     (1500, 0.1, 0.10, 0.95, 3, dict(skin=0.02)),        # 500 rods a block, lists rebuilt in the call
+    (1300, 0.1, 0.10, 0.95, 1, {}),                     # several rods and pairs a thread
     (1500, 0.1, 0.10, 0.95, 0, dict(near_skin_pct=-1)),  # full lists instead of near lists
     (4000, 0.1, 0.12, 0.7, 0, {}),                      # more new pairs at once than are sorted on chip
 ])
