@@ -113,7 +113,7 @@ typedef struct rg_config {
   /* Neighbour-list broad phase (project-specific, no reference field). */
   double skin;                   /* Verlet skin; <= 0: max(d/2, L/10), means */
   int32_t max_neighbors;         /* initial per-rod list capacity; <= 0 auto */
-  int32_t team_blocks;           /* blocks of the persistent NSC team; 0 auto */
+  int32_t team_blocks;           /* blocks of the persistent team; 0 auto */
   int32_t nsc_mlp_scope;         /* learned start for: 0 contacts new since
                                     the last step (not in the warm cache),
                                     1 every contact                          */
@@ -361,7 +361,8 @@ int rg_mlp_infer(rg_system* sys, const float* features, float* out, size_t n);
 
 /* ---- batched independent systems ---------------------------------------- */
 /* A batch runs many independent periodic systems of uneven size in one
- * device step (one launch sequence, CUDA-graph captured).  Each member has
+ * device step (one launch for the NSC members, CUDA-graph captured, and one
+ * for the others).  Each member has
  * its own rg_config (box, model, dt, μ, ...).  Bodies of member k occupy
  * global indices [offset_k, offset_k + n_k). */
 typedef struct rg_batch rg_batch;
