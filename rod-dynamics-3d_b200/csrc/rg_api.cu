@@ -713,6 +713,17 @@ void launch_steps(rg_system* s, int nsteps) {
   }
   // the multi-kernel form, whose launches the stage timers bracket
   for (int k = 0; k < nsteps; ++k) verlet_step(s, k == nsteps - 1);
+  s->fresh_after = s->contacts_fresh;
+  s->contacts_fresh = Fresh::kNo;
+}
+
+void call_begin(rg_system* s) {
+  s->fresh_after = s->contacts_fresh;
+  s->vteam.cb_after = s->vteam.cb;
+}
+void call_done(rg_system* s) {
+  s->contacts_fresh = s->fresh_after;
+  s->vteam.cb = s->vteam.cb_after;
 }
 
 // Grows the buffer named by the error bits.  Returns false if nothing grew.
@@ -800,6 +811,7 @@ cudaError_t reset_call_ctl(rg_system* s, const Snapshot& sn) {
 int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   *retry = false;
   if (!err) return RG_OK;
+  s->contacts_fresh = Fresh::kNo;
   // Every failure puts back the state, history and warm cache the call
   // started from, so the handle stays usable after an error status.
   cudaError_t e = restore_snapshot(s, sn);
@@ -807,7 +819,6 @@ int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   if (err & (ERR_TIMEOUT | ERR_NONFINITE | ERR_COLOR)) {
     std::memcpy(s->h_ctl, sn.ctl.data(), s->ctl_bytes);
     reinterpret_cast<Ctl*>(s->h_ctl)->rebuild = 1;
-    s->contacts_fresh = Fresh::kNo;
     e = cudaMemcpyAsync(s->d_ctl, s->h_ctl, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream);
     if (!e) e = cudaStreamSynchronize(s->stream);
     if (e) return cuda_fail(s, e, "restore control words");
@@ -819,7 +830,6 @@ int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   e = take_snapshot(s, sn);
   if (e) return cuda_fail(s, e, "snapshot");
   reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
-  s->contacts_fresh = Fresh::kNo;
   *retry = true;
   return RG_OK;
 }
@@ -866,6 +876,7 @@ int rg_step(rg_system* s, int nsteps, rg_step_stats* stats) {
     int ev0 = prof_event(s), ev1 = prof_event(s);
     const long long l0 = g_launches;
     cudaEventRecord(s->ev_pool[ev0], s->stream);
+    call_begin(s);
     launch_steps(s, nsteps);
     cudaEventRecord(s->ev_pool[ev1], s->stream);
     cudaError_t e = cudaGetLastError();
@@ -878,6 +889,7 @@ int rg_step(rg_system* s, int nsteps, rg_step_stats* stats) {
     s->last_call_ms = call_ms;
     s->last_call_launches = g_launches - l0;
     if (!h->err) {
+      call_done(s);
       prof_resolve(s);
       break;
     }
@@ -896,6 +908,7 @@ int rg_detect(rg_system* s, double delta, int32_t* pairs, double* geom, double* 
   if (!s || !n) return RG_ERR_ARG;
   if (!s->bodies_set || !s->state_set) return fail(s, RG_ERR_STATE, "set bodies and state first");
   if (delta > s->det.margin) return fail(s, RG_ERR_ARG, "delta exceeds the neighbour-list margin of this model");
+  s->contacts_fresh = Fresh::kNo;  // the force path must detect again, also after a query that fails
   for (int attempt = 0; attempt < 8; ++attempt) {
     Ctl* h = s->h_ctl;
     RG_TRY(cudaMemsetAsync(&s->d_ctl->err, 0, sizeof(int), s->stream), "ctl");
@@ -910,7 +923,6 @@ int rg_detect(rg_system* s, double delta, int32_t* pairs, double* geom, double* 
     if (!grow(s, h->err)) return fail(s, RG_ERR_CAPACITY, "could not grow device buffers");
     force_rebuild(s);
   }
-  s->contacts_fresh = Fresh::kNo;  // the force path must rebuild its CSR
   const int C = s->h_ctl->contacts;
   if (C < 0 || C > s->ccap) return fail(s, RG_ERR_CAPACITY, "contact count exceeds the contact buffer");
   *n = (size_t)C;
@@ -1038,26 +1050,25 @@ int rg_compute_forces(rg_system* s, double* f, double* tau, double* pe) {
     h->ins_n[0] = h->ins_n[1] = 0;
     RG_TRY(cudaMemcpyAsync(s->d_ctl, h, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream), "ctl");
     s->contacts_fresh = Fresh::kNo;
+    call_begin(s);
     if (verlet_team_fits(s)) {
       verlet_run_launch(s, 0);  // one launch (the multi-kernel evaluation: 24)
     } else {
       clear_forces_launch(s);
       force_eval_launch(s);
-      s->contacts_fresh = Fresh::kCsr;
+      s->fresh_after = Fresh::kCsr;
     }
     RG_TRY(cudaGetLastError(), "force launch");
     RG_TRY(cudaMemcpyAsync(h, s->d_ctl, s->ctl_bytes, cudaMemcpyDeviceToHost, s->stream), "ctl");
     RG_TRY(cudaStreamSynchronize(s->stream), "forces");
-    if (!h->err) break;
-    if (h->err & ERR_TIMEOUT) return fail(s, RG_ERR_TIMEOUT, "a device-side wait timed out in force evaluation");
-    if (h->err & ERR_NONFINITE) return fail(s, RG_ERR_NONFINITE, "non-finite body state");
-    if (h->err & ERR_COLOR) return fail(s, RG_ERR_CAPACITY, "force evaluation failed");
+    if (!h->err) {
+      call_done(s);
+      break;
+    }
+    bool retry = false;
+    const int rc = resolve_call(s, sn, h->err, &retry);  // the evaluation updates the history in place
+    if (rc != RG_OK) return rc;
     if (attempt == 7) return fail(s, RG_ERR_CAPACITY, "capacity retries exhausted");
-    int err = h->err;
-    RG_TRY(restore_snapshot(s, sn), "restore");
-    if (!grow(s, err)) return fail(s, RG_ERR_CAPACITY, "could not grow device buffers");
-    RG_TRY(take_snapshot(s, sn), "snapshot");
-    reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
   }
   if (pe) *pe = s->h_ctl->pe;
   return rg_get_state(s, nullptr, nullptr, nullptr, nullptr, f, tau);

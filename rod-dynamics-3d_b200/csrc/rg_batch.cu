@@ -651,6 +651,7 @@ int batch_call(rg_batch* b, int nsteps, rg_step_stats* per, bool restore_after =
     }
     const long long l0 = g_launches;
     cudaEventRecord(b->ev0, b->stream);
+    for (int k : todo) call_begin(b->sys[k]);
     cudaError_t e = launch_nsc(b, (int)teams.size(), grid, nsteps, full);
     if (e) return bfail(b, RG_ERR_CUDA, std::string("persistent launch: ") + cudaGetErrorString(e));
     if ((e = launch_verlet(b, todo, nsteps)))
@@ -688,7 +689,10 @@ int batch_call(rg_batch* b, int nsteps, rg_step_stats* per, bool restore_after =
           over.push_back(t - sv - b->par[k] / nb);
         }
       }
-      if (!err) continue;
+      if (!err) {
+        call_done(s);
+        continue;
+      }
       bool retry = false;
       int rc = resolve_call(s, sn[k], err, &retry);
       if (rc != RG_OK) return bfail(b, rc, "member " + std::to_string(k) + ": " + s->err_text);

@@ -182,7 +182,7 @@ struct VerletTeam {
   // history entry (-1: none)
   int *first[2] = {nullptr, nullptr}, *hidx[2] = {nullptr, nullptr};
   int2* pk[2] = {nullptr, nullptr};
-  int cb = 0;                            // the current one
+  int cb = 0, cb_after = 0;              // the current one; the one a running call ends on
   int *head = nullptr, *next = nullptr;  // per rod: list of the contacts it is second body of
   int* ins = nullptr;                    // contacts whose pair an evaluation adds
   // the near lists (or, without them, the whole lists) as one list of pairs
@@ -213,6 +213,9 @@ struct rg_system {
   std::string err_text;
   bool bodies_set = false, state_set = false;
   rg::Fresh contacts_fresh = rg::Fresh::kNo;  // contacts match the current positions
+  // what a running call leaves, taken over by call_done: nothing is current
+  // while launched work has not been seen to end without an error
+  rg::Fresh fresh_after = rg::Fresh::kNo;
 
   double* d_state = nullptr;  // 19 n
   double* d_props = nullptr;  // 11 n
@@ -423,6 +426,8 @@ void finish_snapshot(rg_system* s, Snapshot& sn);  // after the stream synchroni
 cudaError_t restore_snapshot(rg_system* s, const Snapshot& sn);
 cudaError_t reset_call_ctl(rg_system* s, const Snapshot& sn);
 int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry);
+void call_begin(rg_system* s);  // before a call's launches
+void call_done(rg_system* s);   // after them, with an error word of zero
 void launch_steps(rg_system* s, int nsteps);
 void fill_stats(rg_system* s, int nsteps, rg_step_stats* stats, bool ke_launched = false);
 double kinetic_energy(rg_system* s);

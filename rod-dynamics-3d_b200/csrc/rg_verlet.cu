@@ -678,11 +678,15 @@ VerletView make_verlet_view(rg_system* s) {
   return W;
 }
 
-// Bookkeeping of a launch of nsteps steps: the contacts it leaves.
+// Bookkeeping of a launch of nsteps steps: the contacts it leaves when it ends
+// without an error.  Until then (a barrier that timed out, a launch that never
+// ran) they are not to be relied on: the lists hold whatever the kernel had
+// reached, and indices read from them could lie outside the tables.
 void verlet_launched(rg_system* s, int nsteps) {
   const int detections = nsteps + (s->contacts_fresh == Fresh::kTeam ? 0 : 1);
-  s->vteam.cb = (s->vteam.cb + detections) & 1;
-  s->contacts_fresh = Fresh::kTeam;
+  s->vteam.cb_after = (s->vteam.cb + detections) & 1;
+  s->fresh_after = Fresh::kTeam;
+  s->contacts_fresh = Fresh::kNo;
 }
 
 bool verlet_team_fits(const rg_system* s) {

@@ -1,0 +1,96 @@
+"""The library's host side when a call of the CUDA runtime fails or a kernel
+reports an error, on the CPU: the library runs in a child process over a
+stand-in runtime (fake_cudart.cpp), whose kernels do nothing and whose failures
+are set by the test.
+"""
+import os
+import subprocess
+import sys
+
+import pytest
+
+import rodgpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+SETUP = """
+import ctypes
+import numpy as np
+import rodgpu
+
+fake = ctypes.CDLL({fake!r})
+fake.fake_launches.restype = ctypes.c_longlong
+fake.fake_uploads.restype = ctypes.c_size_t
+fake.fake_uploads.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+ERR = dict(contacts=1, lists=2, history=8, timeout=16)
+N = 50
+rng = np.random.default_rng(1)
+X, Q, Z = rng.uniform(-1, 1, (N, 3)), np.tile([1.0, 0, 0, 0], (N, 1)), np.zeros((N, 3))
+
+
+def system(model):
+    s = rodgpu.System(rodgpu.default_config(n_bodies=N, model=model, dt=1e-4))
+    s.set_bodies(np.full(N, 0.05), np.full(N, 0.5), np.ones(N), np.ones((N, 3)))
+    s.set_state(X, Q, Z, Z)
+    return s
+
+
+def uploads():
+    buf = ctypes.create_string_buffer(1 << 20)
+    n = fake.fake_uploads(buf, len(buf))
+    assert n <= len(buf)
+    return buf.raw[:n]
+
+
+def code(call, *a):
+    try:
+        call(*a)
+    except rodgpu.RgError as e:
+        return rodgpu.STATUS[e.code]
+    return "ok"
+
+"""
+
+
+@pytest.fixture(scope="module")
+def run_child(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I/usr/local/cuda/include", "-o", out,
+                    os.path.join(HERE, "fake_cudart.cpp")], check=True)
+
+    def run(body):
+        env = dict(os.environ, LD_PRELOAD=out, PYTHONPATH=rodgpu.PKG)
+        r = subprocess.run([sys.executable, "-c", SETUP.format(fake=out) + body], env=env, capture_output=True,
+                           text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return run
+
+
+@pytest.mark.parametrize("model", ["hertz-mindlin", "harmonic"])
+@pytest.mark.parametrize("call", ["s.step, 4", "s.compute_forces"])
+@pytest.mark.parametrize("failure", ["fake.fake_fail_launches(1)", "fake.fake_next_error(ERR['timeout'])"])
+def test_contacts_of_a_failed_call_are_not_used(run_child, model, call, failure):
+    # What the next step uploads (control words, then the kernel's view with
+    # the flag that says which contacts are current) is what a step after a
+    # new state uploads, byte for byte: the failed call left nothing.
+    run_child(f"""
+s = system({model!r})
+s.detect(0.0)        # names the error word
+s.set_state(X, Q, Z, Z)
+uploads()
+s.step(3)
+first = uploads()
+s.step(2)
+assert uploads() != first          # contacts of the call before are used
+s.set_state(X, Q, Z, Z)
+uploads()
+s.step(3)
+assert uploads() == first
+s.set_state(X, Q, Z, Z)
+{failure}
+assert code({call}) in ("CUDA error", "device wait timed out")
+uploads()
+s.step(3)
+assert uploads() == first
+""")
