@@ -805,9 +805,19 @@ cudaError_t reset_call_ctl(rg_system* s, const Snapshot& sn) {
   return cudaMemcpyAsync(s->d_ctl, h, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream);
 }
 
+// Control words of the snapshot, lists to be rebuilt, onto the device.
+static int upload_ctl(rg_system* s, Snapshot& sn) {
+  reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
+  std::memcpy(s->h_ctl, sn.ctl.data(), s->ctl_bytes);
+  cudaError_t e = cudaMemcpyAsync(s->d_ctl, s->h_ctl, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream);
+  if (!e) e = cudaStreamSynchronize(s->stream);
+  return e ? cuda_fail(s, e, "restore control words") : RG_OK;
+}
+
 // Turns the error bits of a finished call into a status.  Capacity errors
 // restore the snapshot, grow the buffers and ask for a retry (RG_OK with
-// *retry set).
+// *retry set; the handle is sound without one, too: a batch may have to
+// return another member's error instead).
 int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   *retry = false;
   if (!err) return RG_OK;
@@ -816,20 +826,15 @@ int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   // started from, so the handle stays usable after an error status.
   cudaError_t e = restore_snapshot(s, sn);
   if (e) return cuda_fail(s, e, "restore");
-  if (err & (ERR_TIMEOUT | ERR_NONFINITE | ERR_COLOR)) {
-    std::memcpy(s->h_ctl, sn.ctl.data(), s->ctl_bytes);
-    reinterpret_cast<Ctl*>(s->h_ctl)->rebuild = 1;
-    e = cudaMemcpyAsync(s->d_ctl, s->h_ctl, s->ctl_bytes, cudaMemcpyHostToDevice, s->stream);
-    if (!e) e = cudaStreamSynchronize(s->stream);
-    if (e) return cuda_fail(s, e, "restore control words");
-  }
+  int rc;
+  if ((err & (ERR_TIMEOUT | ERR_NONFINITE | ERR_COLOR)) && (rc = upload_ctl(s, sn)) != RG_OK) return rc;
   if (err & ERR_TIMEOUT) return fail(s, RG_ERR_TIMEOUT, "a device-side barrier timed out");
   if (err & ERR_NONFINITE) return fail(s, RG_ERR_NONFINITE, "non-finite body state");
   if (err & ERR_COLOR) return fail(s, RG_ERR_CAPACITY, "contact graph needs more than 64 colours");
   if (!grow(s, err)) return fail(s, RG_ERR_CAPACITY, "could not grow device buffers");
   e = take_snapshot(s, sn);
   if (e) return cuda_fail(s, e, "snapshot");
-  reinterpret_cast<Ctl*>(sn.ctl.data())->rebuild = 1;
+  if ((rc = upload_ctl(s, sn)) != RG_OK) return rc;
   *retry = true;
   return RG_OK;
 }

@@ -667,6 +667,10 @@ int batch_call(rg_batch* b, int nsteps, rg_step_stats* per, bool restore_after =
     const long long launches = g_launches - l0;
     std::vector<int> again;
     std::vector<double> over;  // team overhead samples of multi-block members
+    // every member with an error is put back (and given its larger buffers)
+    // before the first status that no replay can cure is returned
+    int fatal = RG_OK;
+    std::string why;
     for (int k : todo) {
       rg_system* s = b->sys[k];
       s->last_call_ms = ms;
@@ -695,9 +699,14 @@ int batch_call(rg_batch* b, int nsteps, rg_step_stats* per, bool restore_after =
       }
       bool retry = false;
       int rc = resolve_call(s, sn[k], err, &retry);
-      if (rc != RG_OK) return bfail(b, rc, "member " + std::to_string(k) + ": " + s->err_text);
-      again.push_back(k);
+      if (rc == RG_OK) {
+        again.push_back(k);
+      } else if (fatal == RG_OK) {
+        fatal = rc;
+        why = "member " + std::to_string(k) + ": " + s->err_text;
+      }
     }
+    if (fatal != RG_OK) return bfail(b, fatal, why);
     if (!over.empty()) {
       std::nth_element(over.begin(), over.begin() + over.size() / 2, over.end());
       const double m = std::min(1.0, std::max(0.0, over[over.size() / 2]));
