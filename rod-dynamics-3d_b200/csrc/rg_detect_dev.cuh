@@ -140,6 +140,8 @@ __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const 
                                         const int* cell_start, const int* cell_rods, double margin,
                                         double skin, int* nbr_cnt, int* nbr, int maxnb, int cell,
                                         BuildSmem& sm, unsigned* q1, unsigned* q2, int qcap, int& overflow) {
+  const int hs = cell_start[cell], he = cell_start[cell + 1];
+  if (hs == he) return;  // no home rod (every thread reads the same)
   int cx = cell % g.n[0], cy = (cell / g.n[0]) % g.n[1], cz = cell / (g.n[0] * g.n[1]);
   // Half shell: the home cell (pairs j > i) and the 13 cells ahead of it
   // (every pair), each unordered pair met once and listed under its lower
@@ -202,7 +204,6 @@ __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const 
     for (int c = 0; c < nn; ++c) sm.npre[c + 1] += sm.npre[c];
   }
   // (read after the barrier at the top of the home-tile loop)
-  const int hs = cell_start[cell], he = cell_start[cell + 1];
   for (int h0 = hs; h0 < he; h0 += kTile) {
     const int H = he - h0 < kTile ? he - h0 : kTile;
     // G threads per home rod, each scanning every G-th rod of a tile: no

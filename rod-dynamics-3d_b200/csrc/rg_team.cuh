@@ -221,33 +221,56 @@ static __device__ bool build_lists(const Team& T, const NscView& V, SmemNsc& sm,
   }
   if (!team_sync(T)) return false;
   if (!team_excl_scan(T, V.cell_cnt, V.cell_start, g.ncells, V.blk, sm)) return false;
+  int others = 0;  // rods that share a rod's cell, summed over the rods
   for (int i = tid; i < n; i += TS) {
     int c = V.cell_of[i];
-    V.cell_rods[V.cell_start[c] + atomicAdd(&V.cell_fill[c], 1)] = i;
+    const int first = V.cell_start[c];
+    V.cell_rods[first + atomicAdd(&V.cell_fill[c], 1)] = i;
+    others += min(V.cell_start[c + 1] - first - 1, 255);
   }
+  others = block_reduce_sum_i(others, sm.red_i);
+  if (threadIdx.x == 0) V.blk[rank] = (int)(65536.0 * others / n);
   if (!team_sync(T)) return false;
+  int before, total;
+  block_prefix(V.blk, T.nb, rank, before, total, sm);
+  const double rho = total / 65536.0;
   double invL[3] = {1.0, 1.0, 1.0};
   for (int k = 0; k < 3; ++k)
     if (V.box.L[k] > 0.0) invL[k] = 1.0 / V.box.L[k];
-  // One thread per home rod where every block has thousands of rods of its
-  // own and a rod few candidates, else the block splits the pairs of one home
-  // cell at a time: a thread alone with its rod's candidates is a serial chain
-  // (1000 rods of aspect 10 on 8 blocks: 954 us by rod, 241 by cell; 5000 of
-  // aspect 10 on 40: 1425 and 275; 20000 of aspect 5 on 148: 743 and 221;
-  // 400000 of aspect 20, 46 rods a cell, on 148: 10.8 and 5.3 ms).  The two
-  // meet at 200000 rods of aspect 5 (1.60 and 1.66 ms); at a million of
-  // aspect 5 or 3, some 10 rods a cell, staging a tile for a handful of pairs
-  // costs more: 6.7 and 5.8 ms by rod, 8.3 and 10.2 by cell.
-  if (n < 16 * g.ncells && n > 2048 * T.nb) {
+  // One thread per home rod, or the block splits the pairs of one home cell at
+  // a time.  A thread alone with its rod's candidates is a serial chain, some
+  // 50 + 60 rho us a turn of the threads with rho other rods in the average
+  // rod's cell; a cell that holds rods costs a block some 13 us (barriers and
+  // the staging of its neighbourhood) until there are rods enough to fill the
+  // tiles, so a block with n / nb rods, rho a cell, takes 13 n / (nb rho).
+  // They meet at n / nb = rho (4 + 5 rho), and where threads have several
+  // turns near rho = 12.  Measured, by rod and by cell, us: 1000 rods on 8
+  // blocks, rho 0.03 54 and 2132 (32768 cells), 1 115 and 818, 4 242 and 351,
+  // 8 552 and 144; 20000 on 148, rho 1 137 and 1168, 4 288 and 460, 8 506 and
+  // 237; 20000 on 40, rho 8 502 and 774, 16 945 and 662; a million on 148, rho
+  // 1 1384 and 49811, 8 5154 and 11045, 16 8723 and 7469.
+  if (rho < 12.0 && n > rho * (4.0 + 5.0 * rho) * T.nb) {
     for (int i = tid; i < n; i += TS)
       build_rod_list(i, V.seg, g, V.box, invL, V.cell_of, V.cell_start, V.cell_rods, V.margin, V.skin,
                      V.nbr_cnt, V.nbr, V.maxnb, overflow);
   } else {
-    for (int cell = rank; cell < g.ncells; cell += T.nb)
-      build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin,
-                       V.nbr_cnt, V.nbr, V.maxnb, cell, *reinterpret_cast<BuildSmem*>(team_dyn_smem),
-                       reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff),
-                       reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff) + kBuildQ, kBuildQ, overflow);
+    // a block's cells, those without rods passed over a word of cells at a
+    // time (one after the other, 0.5 us each)
+    const int lane = threadIdx.x & 31, nwarp = (int)(blockDim.x >> 5);
+    for (int first = rank; first < g.ncells; first += (int)blockDim.x * T.nb) {
+      const int c = first + (int)threadIdx.x * T.nb;
+      const unsigned any = __ballot_sync(0xffffffffu, c < g.ncells && V.cell_start[c + 1] > V.cell_start[c]);
+      if (lane == 0) sm.pre[threadIdx.x >> 5] = (int)any;
+      __syncthreads();
+      for (int w = 0; w < nwarp; ++w)
+        for (unsigned m = (unsigned)sm.pre[w]; m; m &= m - 1)
+          build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin, V.nbr_cnt, V.nbr,
+                           V.maxnb, first + (32 * w + __ffs((int)m) - 1) * T.nb,
+                           *reinterpret_cast<BuildSmem*>(team_dyn_smem),
+                           reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff),
+                           reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff) + kBuildQ, kBuildQ, overflow);
+      __syncthreads();
+    }
   }
   return team_sync(T);
 }
