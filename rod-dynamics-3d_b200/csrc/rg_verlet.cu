@@ -15,8 +15,8 @@
 //    start reuse those contacts in place;
 //  * a body's contacts are found without a sorted incidence table: those where
 //    it is the first body are a run of the (a, b)-sorted list,
-//    those where it is the second hang off it in a short linked list, walked
-//    in ascending order; together the contact order of the reference's sums;
+//    those where it is the second hang off it in a linked list, walked in
+//    ascending order; together the contact order of the reference's sums;
 //  * the history entry of a persisting contact is found through the previous
 //    contact list (same first body, a handful of candidates) and rewritten in
 //    place; the sorted table is merged only in evaluations that add a pair,
@@ -215,28 +215,94 @@ __device__ __noinline__ bool v_insert(const Team& T, const VerletView& W, Verlet
   return true;
 }
 
+// Sorts a list of contacts ascending and returns its new head: turned over (a
+// warp's contacts then mostly ascend, having been pushed in lane order), then
+// pairs of ascending runs merged until one is left.
+__device__ __noinline__ int v_sort_list(int* next, int head) {
+  int rev = -1;
+  while (head >= 0) {
+    const int k = next[head];
+    next[head] = rev;
+    rev = head;
+    head = k;
+  }
+  head = rev;
+  auto run_end = [&](int p, int& rest) {  // last of the run at p; what follows it
+    while ((rest = next[p]) > p) p = rest;
+    return p;
+  };
+  for (;;) {
+    int p = head, tail = -1, runs = 0;
+    auto append = [&](int k) {
+      if (tail < 0) head = k;
+      else next[tail] = k;
+      tail = k;
+    };
+    while (p >= 0) {
+      int q, rest;
+      const int pe = run_end(p, q);
+      next[pe] = -1;
+      ++runs;
+      if (q < 0) {
+        append(p);
+        break;
+      }
+      const int qe = run_end(q, rest);
+      next[qe] = -1;
+      while (p >= 0 && q >= 0) {
+        const int k = min(p, q);
+        append(k);  // (k's own link is read before the next append sets it)
+        if (k == p) p = next[p];
+        else q = next[q];
+      }
+      append(p >= 0 ? p : q);
+      tail = p >= 0 ? pe : qe;
+      p = rest;
+    }
+    if (runs <= 1) return head;
+  }
+}
+
 // Sums of body i's contact addends in contact order.
 __device__ inline void v_body_sum(const VerletView& W, const VerletRun& r, int i, d3& f, d3& t) {
   const size_t cc = (size_t)W.v.ccap;
-  const int* next = W.next;
-  const int h0 = W.head[i];
-  for (int last = -1; h0 >= 0;) {  // second body of: ascending walk of the list
-    int c = 0x7fffffff;
-    for (int k = h0; k >= 0; k = next[k])
-      if (k > last && k < c) c = k;
-    if (c == 0x7fffffff) break;
-    const double* g = W.cf + 6 * cc + c;
+  int* next = W.next;
+  int h0 = W.head[i];
+  auto add = [&](const double* g) {
     f.x = f.x + g[0]; f.y = f.y + g[cc]; f.z = f.z + g[2 * cc];
     t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
-    last = c;
+  };
+  const double* fb = W.cf + 6 * cc;
+  if (h0 >= 0) {  // second body of: the list, in ascending order
+    int low = h0, len = 1;
+    bool sorted = true;
+    for (int p = h0, k = next[h0]; k >= 0; p = k, k = next[k], ++len) {
+      sorted = sorted && k > p;
+      low = min(low, k);
+    }
+    // A walk of the list for each of its contacts suits the usual two or
+    // three; a long one (a large body under many small ones) is sorted in
+    // place, once a detection: a rod under 1000 others, some 6000 contacts in
+    // all, 23 -> 1.1 ms a step.
+    if (!sorted && len > 8) {
+      W.head[i] = h0 = v_sort_list(next, h0);
+      sorted = true;
+    }
+    if (sorted) {
+      for (int k = h0; k >= 0; k = next[k]) add(fb + k);
+    } else {
+      for (int c = low; c < 0x7fffffff;) {
+        add(fb + c);
+        int up = 0x7fffffff;
+        for (int k = h0; k >= 0; k = next[k])
+          if (k > c && k < up) up = k;
+        c = up;
+      }
+    }
   }
   const int2* pk = W.pk[r.cb];
   const int c0 = W.first[r.cb][i];
-  for (int c = c0; c >= 0 && c < r.C && pk[c].x == i; ++c) {  // first body of
-    const double* g = W.cf + c;
-    f.x = f.x + g[0]; f.y = f.y + g[cc]; f.z = f.z + g[2 * cc];
-    t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
-  }
+  for (int c = c0; c >= 0 && c < r.C && pk[c].x == i; ++c) add(W.cf + c);  // first body of
 }
 
 // Rod i's records on their way to L2: a thread's next rod, while the present
@@ -437,15 +503,18 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
     const PairIn in = load_pair(V.st, a, b);
     int f = -1;
     bool known = false;
-    if (r.idx_ok)
-      for (int k = W.first[ob][a]; k >= 0 && k < oc; ++k) {
+    if (r.idx_ok) {  // among a's contacts before, in order (a long run: by search below)
+      const int k0 = W.first[ob][a];
+      for (int k = k0; k >= 0 && k < min(oc, k0 + 8); ++k) {
         const int2 q = W.pk[ob][k];
-        if (q.x != a) break;
+        if (q.x != a || q.y > b) break;
         if (q.y == b) {
           f = W.hidx[ob][k];
           known = true;
+          break;
         }
       }
+    }
     if (!known && r.H > 0) f = v_find(W, r, a, b);
     long long frame = 0;
     const d3 old = v_old(W, r, f, frame);
