@@ -488,7 +488,8 @@ int rg_create(const rg_config* cfg, rg_system** out) {
     return RG_ERR_ARG;
   }
   cudaError_t e;
-  if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) ||
+  if ((e = nsc_allow_smem()) || (e = verlet_allow_smem()) ||
+      (e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) ||
       (e = cudaMalloc(&s->d_state, sizeof(double) * 19 * (size_t)s->n)) ||
       (e = cudaMalloc(&s->d_props, sizeof(double) * 11 * (size_t)s->n)) ||
       (e = cudaMemset(s->d_state, 0, sizeof(double) * 19 * (size_t)s->n)) ||

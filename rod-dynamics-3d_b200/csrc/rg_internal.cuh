@@ -379,6 +379,10 @@ void wrap_launch(rg_system* s);
 void nsc_run_launch(rg_system* s, int nsteps);
 int nsc_team_blocks(const rg_system* s);
 int nsc_blocks_per_sm();
+// The persistent kernels' dynamic shared memory, allowed on the current device
+// (the limit belongs to the device: every rg_create asks).
+cudaError_t nsc_allow_smem();
+cudaError_t verlet_allow_smem();
 size_t nsc_view_bytes();
 size_t nsc_team_bytes();
 // rg_verlet.cu

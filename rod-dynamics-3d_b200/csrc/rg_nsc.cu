@@ -2236,19 +2236,14 @@ void nsc_run_launch(rg_system* s, int nsteps) {
   int nteams = 1;
   const int* members = nullptr;
   void* args[] = {&views, &teams, &nteams, &members, &nsteps};
-  nsc_set_smem();
   ProfScope p(s, ST_OTHER);
   launch_coop((const void*)k_nsc_run, nb, kBlock, args, s->stream, sizeof(SmallSmem));
   s->contacts_fresh = Fresh::kNo;
 }
 
-void nsc_set_smem() {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute((const void*)k_nsc_run, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(SmallSmem));
-    attr_set = true;
-  }
+cudaError_t nsc_allow_smem() {
+  return cudaFuncSetAttribute((const void*)k_nsc_run, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)sizeof(SmallSmem));
 }
 
 // nsteps steps of many systems as one persistent cooperative launch: teams
@@ -2256,28 +2251,22 @@ void nsc_set_smem() {
 // systems members[first_k .. first_k + count_k) of views.
 void nsc_batch_launch(const NscView* views, const TeamDesc* teams, int nteams, const int* members, int grid,
                       int nsteps, cudaStream_t st) {
-  nsc_set_smem();
   void* args[] = {&views, &teams, &nteams, &members, &nsteps};
   launch_coop((const void*)k_nsc_run, grid, kBlock, args, st, sizeof(SmallSmem));
 }
 
 int nsc_block_threads() { return kBlock; }
 
-// Co-resident blocks of the persistent kernel per SM (its registers and
-// shared memory decide; the cooperative launch needs them all resident).
+// Co-resident blocks of the persistent kernel per SM of the current device
+// (its registers and shared memory decide; the cooperative launch needs them
+// all resident).
 int nsc_blocks_per_sm() {
-  static int per_sm = -1;
-  if (per_sm < 0) {
-    nsc_set_smem();
-    int k = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_nsc_run, kBlock, sizeof(SmallSmem)) != cudaSuccess ||
-        k < 1) {
-      cudaGetLastError();
-      k = 1;
-    }
-    per_sm = k;
+  int k = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_nsc_run, kBlock, sizeof(SmallSmem)) != cudaSuccess || k < 1) {
+    cudaGetLastError();
+    k = 1;
   }
-  return per_sm;
+  return k;
 }
 size_t nsc_block_smem() { return sizeof(SmallSmem) + sizeof(SmemNsc); }
 

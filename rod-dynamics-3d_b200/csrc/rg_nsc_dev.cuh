@@ -547,7 +547,6 @@ struct TeamDesc {
   long long* t_ns;    // optional: the team's device time for the launch
 };
 
-void nsc_set_smem();
 void nsc_batch_launch(const NscView* views, const TeamDesc* teams, int nteams, const int* members, int grid,
                       int nsteps, cudaStream_t st);
 int nsc_block_threads();

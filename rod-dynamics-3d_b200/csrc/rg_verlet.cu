@@ -763,13 +763,12 @@ bool verlet_team_fits(const rg_system* s) {
   return (m == RG_MODEL_HARMONIC || m == RG_MODEL_HERTZ_MINDLIN) && !s->prof_on && s->vteam.head;
 }
 
+cudaError_t verlet_allow_smem() {
+  return cudaFuncSetAttribute((const void*)k_verlet_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmem);
+}
+
 void verlet_launch(const VerletView* views, const TeamDesc* teams, int nteams, const int* members, int grid, int nsteps,
                    cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute((const void*)k_verlet_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmem);
-    attr_set = true;
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kVBlock);

@@ -94,3 +94,18 @@ uploads()
 s.step(3)
 assert uploads() == first
 """)
+
+
+@pytest.mark.parametrize("model", ["nsc", "hertz-mindlin", "harmonic"])
+def test_every_device_allows_the_shared_memory_of_the_step(run_child, model):
+    # the limit on dynamic shared memory belongs to a device, not to the process
+    run_child(f"""
+for device in (0, 1, 0):
+    fake.fake_set_device(device)
+    s = system({model!r})
+    s.step(2)
+    if {model!r} != "nsc":
+        s.compute_forces()
+    s.close()
+assert fake.fake_smem_refused() == 0
+""")
