@@ -1928,9 +1928,11 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, unsigned&
   const bool small = C <= kSmallC;
   if (small) {
     // colouring, rows, PSOR and warm cache on chip
-    const unsigned long long ts = (rank == 0 && threadIdx.x == 0) ? gtimer() : 0ull;
+    // (serial time of the batch's cost model: what one block does alone)
+    const bool alone = solo(C, V.rec_cap > 0) && rank == 0 && threadIdx.x == 0;
+    const unsigned long long ts = alone ? gtimer() : 0ull;
     if (!small_solve(T, V, C, Cp, chunk, pc)) return false;
-    if (rank == 0 && threadIdx.x == 0) ctl->serial_ns += (long long)(gtimer() - ts);
+    if (alone) ctl->serial_ns += (long long)(gtimer() - ts);
     pc.mark(10);
     if (!team_sync(T)) return false;
     pc.mark(11);
@@ -2082,9 +2084,10 @@ __device__ bool nsc_step(const Team& T, const NscView& V, SmemNsc& sm, unsigned&
     if (C2 < 0) return false;
     pc.mark(6);
     if (C2 <= kSmallC) {
-      const unsigned long long ts = (rank == 0 && threadIdx.x == 0) ? gtimer() : 0ull;
+      const bool alone = solo(C2, false) && rank == 0 && threadIdx.x == 0;
+      const unsigned long long ts = alone ? gtimer() : 0ull;
       if (!small_project(T, V, C2, chunk)) return false;
-      if (rank == 0 && threadIdx.x == 0) ctl->serial_ns += (long long)(gtimer() - ts);
+      if (alone) ctl->serial_ns += (long long)(gtimer() - ts);
       if (!team_sync(T)) return false;
     } else {
       if (!color_phase(T, V, C2, sm)) return false;
