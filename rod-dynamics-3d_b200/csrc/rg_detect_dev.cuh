@@ -69,6 +69,11 @@ struct SegTile {
   }
 };
 
+// Whether the two forms of a team's list build are functions of their own.
+#ifndef RG_BUILD_INLINE
+#define RG_BUILD_INLINE inline
+#endif
+
 struct BuildSmem {
   SegTile tile;
   int tidx[kTile];
@@ -331,9 +336,10 @@ __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const 
 // the candidates of rod i are the rods of its cell's neighbourhood, read
 // from the cell arrays; accepted j > i are appended to i's own list (sorted
 // afterwards by sort_list).  Same acceptance as build_cell_pairs.
-__device__ inline void build_rod_list(int i, const Seg* seg, const GridDev& g, const Box& box, const double* invL,
-                                      const int* cell_of, const int* cell_start, const int* cell_rods, double margin,
-                                      double skin, int* nbr_cnt, int* nbr, int maxnb, int& overflow) {
+static __device__ RG_BUILD_INLINE void build_rod_list(int i, const Seg* seg, const GridDev& g, const Box& box,
+                                                      const double* invL, const int* cell_of, const int* cell_start,
+                                                      const int* cell_rods, double margin, double skin, int* nbr_cnt,
+                                                      int* nbr, int maxnb, int& overflow) {
   const int cell = cell_of[i];
   const int c3[3] = {cell % g.n[0], (cell / g.n[0]) % g.n[1], cell / (g.n[0] * g.n[1])};
   int lo[3], hi[3];

@@ -174,6 +174,26 @@ __device__ inline bool team_excl_scan(const Team& T, const int* in, int* out, in
 // ---------------------------------------------------------------------------
 // Detection inside the persistent kernel.
 // ---------------------------------------------------------------------------
+// The pairs of a team's cells, each block its share; those without rods are
+// passed over a word of cells at a time (one after the other, 0.5 us each).
+static __device__ RG_BUILD_INLINE void build_cells(const Team& T, const NscView& V, const GridDev& g,
+                                                   const double* invL, SmemNsc& sm, int& overflow) {
+  const int rank = T.rank(), lane = threadIdx.x & 31, nwarp = (int)(blockDim.x >> 5);
+  for (int first = rank; first < g.ncells; first += (int)blockDim.x * T.nb) {
+    const int c = first + (int)threadIdx.x * T.nb;
+    const unsigned any = __ballot_sync(0xffffffffu, c < g.ncells && V.cell_start[c + 1] > V.cell_start[c]);
+    if (lane == 0) sm.pre[threadIdx.x >> 5] = (int)any;
+    __syncthreads();
+    for (int w = 0; w < nwarp; ++w)
+      for (unsigned m = (unsigned)sm.pre[w]; m; m &= m - 1)
+        build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin, V.nbr_cnt, V.nbr, V.maxnb,
+                         first + (32 * w + __ffs((int)m) - 1) * T.nb, *reinterpret_cast<BuildSmem*>(team_dyn_smem),
+                         reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff),
+                         reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff) + kBuildQ, kBuildQ, overflow);
+    __syncthreads();
+  }
+}
+
 // Cell lists and the candidates within margin + skin of every rod (unordered).
 static __device__ bool build_lists(const Team& T, const NscView& V, SmemNsc& sm, int& overflow) {
   const int n = V.st.n;
@@ -254,23 +274,7 @@ static __device__ bool build_lists(const Team& T, const NscView& V, SmemNsc& sm,
       build_rod_list(i, V.seg, g, V.box, invL, V.cell_of, V.cell_start, V.cell_rods, V.margin, V.skin,
                      V.nbr_cnt, V.nbr, V.maxnb, overflow);
   } else {
-    // a block's cells, those without rods passed over a word of cells at a
-    // time (one after the other, 0.5 us each)
-    const int lane = threadIdx.x & 31, nwarp = (int)(blockDim.x >> 5);
-    for (int first = rank; first < g.ncells; first += (int)blockDim.x * T.nb) {
-      const int c = first + (int)threadIdx.x * T.nb;
-      const unsigned any = __ballot_sync(0xffffffffu, c < g.ncells && V.cell_start[c + 1] > V.cell_start[c]);
-      if (lane == 0) sm.pre[threadIdx.x >> 5] = (int)any;
-      __syncthreads();
-      for (int w = 0; w < nwarp; ++w)
-        for (unsigned m = (unsigned)sm.pre[w]; m; m &= m - 1)
-          build_cell_pairs(V.seg, g, V.box, invL, V.cell_start, V.cell_rods, V.margin, V.skin, V.nbr_cnt, V.nbr,
-                           V.maxnb, first + (32 * w + __ffs((int)m) - 1) * T.nb,
-                           *reinterpret_cast<BuildSmem*>(team_dyn_smem),
-                           reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff),
-                           reinterpret_cast<unsigned*>(team_dyn_smem + kBuildQOff) + kBuildQ, kBuildQ, overflow);
-      __syncthreads();
-    }
+    build_cells(T, V, g, invL, sm, overflow);
   }
   return team_sync(T);
 }

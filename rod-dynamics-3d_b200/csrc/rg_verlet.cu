@@ -33,6 +33,10 @@
 #include <cstring>
 #include <vector>
 
+// Functions of their own here: inlined into the list rebuild, the registers
+// that they take from its callers made every step 1 % slower (the PSOR kernel:
+// the other way round).
+#define RG_BUILD_INLINE __noinline__
 #include "rg_team.cuh"
 #include "rg_verlet_dev.cuh"
 
@@ -215,10 +219,11 @@ __device__ __noinline__ bool v_insert(const Team& T, const VerletView& W, Verlet
   return true;
 }
 
-// Sorts a list of contacts ascending and returns its new head: turned over (a
-// warp's contacts then mostly ascend, having been pushed in lane order), then
-// pairs of ascending runs merged until one is left.
-__device__ __noinline__ int v_sort_list(int* next, int head) {
+// Sorts the list of contacts whose head is at *at: turned over (a warp's
+// contacts then mostly ascend, having been pushed in lane order), then pairs of
+// ascending runs merged until one is left.
+__device__ __noinline__ void v_sort_list(int* next, int* at) {
+  int head = *at;
   int rev = -1;
   while (head >= 0) {
     const int k = next[head];
@@ -259,50 +264,52 @@ __device__ __noinline__ int v_sort_list(int* next, int head) {
       tail = p >= 0 ? pe : qe;
       p = rest;
     }
-    if (runs <= 1) return head;
+    if (runs <= 1) break;
   }
+  *at = head;
 }
 
-// Sums of body i's contact addends in contact order.
-__device__ inline void v_body_sum(const VerletView& W, const VerletRun& r, int i, d3& f, d3& t) {
+// Sums of body i's contact addends in contact order.  A walk of the list of the
+// contacts that it is second body of, for each of them, suits the usual two or
+// three; a longer list (a large body under many small ones) has to be sorted:
+// false where it is not, and the caller sorts it and comes again, once a
+// detection.  A rod under 1000 others, some 6000 contacts in all: 23 -> 1.1 ms
+// a step.  (The call stays outside the callers' loops: inside, its registers
+// slowed all steps by 1 to 2 %.)
+constexpr int kShortList = 8;
+__device__ inline bool v_body_sum(const VerletView& W, const VerletRun& r, int i, d3& f, d3& t) {
   const size_t cc = (size_t)W.v.ccap;
-  int* next = W.next;
-  int h0 = W.head[i];
+  const int* next = W.next;
+  const int h0 = W.head[i];
   auto add = [&](const double* g) {
     f.x = f.x + g[0]; f.y = f.y + g[cc]; f.z = f.z + g[2 * cc];
     t.x = t.x + g[3 * cc]; t.y = t.y + g[4 * cc]; t.z = t.z + g[5 * cc];
   };
   const double* fb = W.cf + 6 * cc;
-  if (h0 >= 0) {  // second body of: the list, in ascending order
-    int low = h0, len = 1;
-    bool sorted = true;
-    for (int p = h0, k = next[h0]; k >= 0; p = k, k = next[k], ++len) {
-      sorted = sorted && k > p;
-      low = min(low, k);
-    }
-    // A walk of the list for each of its contacts suits the usual two or
-    // three; a long one (a large body under many small ones) is sorted in
-    // place, once a detection: a rod under 1000 others, some 6000 contacts in
-    // all, 23 -> 1.1 ms a step.
-    if (!sorted && len > 8) {
-      W.head[i] = h0 = v_sort_list(next, h0);
-      sorted = true;
-    }
-    if (sorted) {
-      for (int k = h0; k >= 0; k = next[k]) add(fb + k);
-    } else {
-      for (int c = low; c < 0x7fffffff;) {
-        add(fb + c);
-        int up = 0x7fffffff;
-        for (int k = h0; k >= 0; k = next[k])
-          if (k > c && k < up) up = k;
-        c = up;
+  // second body of: each walk of the list finds the contact after `last`
+  for (int last = -1, more = h0 >= 0 ? 2 : 0; more > 1;) {
+    int c = 0x7fffffff;
+    more = 0;
+    for (int k = h0; k >= 0; k = next[k])
+      if (k > last) {
+        ++more;
+        if (k < c) c = k;
       }
+    if (more > kShortList) {
+      int p = -1;
+      for (int k = h0; k >= 0; p = k, k = next[k]) {
+        if (k < p) return false;
+        add(fb + k);
+      }
+      break;
     }
+    add(fb + c);
+    last = c;
   }
   const int2* pk = W.pk[r.cb];
   const int c0 = W.first[r.cb][i];
   for (int c = c0; c >= 0 && c < r.C && pk[c].x == i; ++c) add(W.cf + c);  // first body of
+  return true;
 }
 
 // Rod i's records on their way to L2: a thread's next rod, while the present
@@ -503,15 +510,14 @@ __device__ __noinline__ bool v_detect_eval(const Team& T, const VerletView& W, V
     const PairIn in = load_pair(V.st, a, b);
     int f = -1;
     bool known = false;
-    if (r.idx_ok) {  // among a's contacts before, in order (a long run: by search below)
-      const int k0 = W.first[ob][a];
-      for (int k = k0; k >= 0 && k < min(oc, k0 + 8); ++k) {
+    if (r.idx_ok) {  // among a's first contacts before (of a longer run: by search)
+      const int k0 = W.first[ob][a], lim = min(oc, k0 + 8);
+      for (int k = k0; k >= 0 && k < lim; ++k) {
         const int2 q = W.pk[ob][k];
-        if (q.x != a || q.y > b) break;
+        if (q.x != a) break;
         if (q.y == b) {
           f = W.hidx[ob][k];
           known = true;
-          break;
         }
       }
     }
@@ -594,12 +600,17 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
     if (!v_detect_eval(T, W, r, S, true)) return false;
     if (!team_sync(T)) return false;
     const int added = *(volatile int*)&ctl->ins_n[r.fr & 1];
-    for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
-      d3 f{0, 0, 0}, tq{0, 0, 0};
-      v_body_sum(W, r, i, f, tq);
-      if (wall && st.inv_mass[i] > 0.0) soft_wall_apply(cfg, ax, st.r[i], st.x.ld(i), st.v.ld(i), f);
-      st.f.st(i, f);
-      st.tau.st(i, tq);
+    for (int i = r.lo + t; i < r.hi;) {
+      bool sort = false;
+      for (; i < r.hi; i += blockDim.x) {
+        d3 f{0, 0, 0}, tq{0, 0, 0};
+        sort = !v_body_sum(W, r, i, f, tq);
+        if (sort) break;
+        if (wall && st.inv_mass[i] > 0.0) soft_wall_apply(cfg, ax, st.r[i], st.x.ld(i), st.v.ld(i), f);
+        st.f.st(i, f);
+        st.tau.st(i, tq);
+      }
+      if (sort) v_sort_list(W.next, W.head + i);
     }
     if (rank == 0) v_energy(W, r.C, S.s);
     if (added && !v_insert(T, W, r, S, added)) return false;
@@ -622,13 +633,18 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
       const int added = *(volatile int*)&ctl->ins_n[r.fr & 1];
       if (rank == 0 && t == 0) ctl->ins_n[(r.fr + 1) & 1] = 0;
       double m = 0.0, m2 = 0.0;
-      for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
-        if (i + (int)blockDim.x < r.hi) v_prefetch(W, r, i + blockDim.x, true, out);
-        d3 f{0, 0, 0}, tq{0, 0, 0};
-        if (st.inv_mass[i] > 0.0) v_body_sum(W, r, i, f, tq);
-        W.head[i] = -1;  // for the detection that follows
-        W.first[1 - r.cb][i] = -1;
-        drift_rod(st, V.box, cfg, ax, wall, i, f, tq, out, invL, m, m2);
+      for (int i = r.lo + t; i < r.hi;) {
+        bool sort = false;
+        for (; i < r.hi; i += blockDim.x) {
+          if (i + (int)blockDim.x < r.hi) v_prefetch(W, r, i + blockDim.x, true, out);
+          d3 f{0, 0, 0}, tq{0, 0, 0};
+          if (st.inv_mass[i] > 0.0) sort = !v_body_sum(W, r, i, f, tq);
+          if (sort) break;
+          W.head[i] = -1;  // for the detection that follows
+          W.first[1 - r.cb][i] = -1;
+          drift_rod(st, V.box, cfg, ax, wall, i, f, tq, out, invL, m, m2);
+        }
+        if (sort) v_sort_list(W.next, W.head + i);
       }
       if (out.ref || out.ref2) v_publish_disp(V, m, m2, S.s);
       if (added && !v_insert(T, W, r, S, added)) return false;
@@ -643,15 +659,20 @@ __device__ __noinline__ bool v_run(const Team& T, const VerletView& W, int nstep
       const int added = *(volatile int*)&ctl->ins_n[r.fr & 1];
       if (rank == 0 && t == 0) ctl->ins_n[(r.fr + 1) & 1] = 0;
       int bad = 0;
-      for (int i = r.lo + t; i < r.hi; i += blockDim.x) {
-        if (i + (int)blockDim.x < r.hi) v_prefetch(W, r, i + blockDim.x, false, out);
-        d3 f{0, 0, 0}, tq{0, 0, 0};
-        v_body_sum(W, r, i, f, tq);
-        bad |= kick_rod(st, cfg, ax, wall, i, f, tq, el, ea);
-        if (last) {  // the forces that the call's last kick used
-          st.f.st(i, f);
-          st.tau.st(i, tq);
+      for (int i = r.lo + t; i < r.hi;) {
+        bool sort = false;
+        for (; i < r.hi; i += blockDim.x) {
+          if (i + (int)blockDim.x < r.hi) v_prefetch(W, r, i + blockDim.x, false, out);
+          d3 f{0, 0, 0}, tq{0, 0, 0};
+          sort = !v_body_sum(W, r, i, f, tq);
+          if (sort) break;
+          bad |= kick_rod(st, cfg, ax, wall, i, f, tq, el, ea);
+          if (last) {  // the forces that the call's last kick used
+            st.f.st(i, f);
+            st.tau.st(i, tq);
+          }
         }
+        if (sort) v_sort_list(W.next, W.head + i);
       }
       if (bad) atomicOr(&ctl->err, ERR_NONFINITE);
       if (last && rank == 0) v_energy(W, r.C, S.s);
