@@ -565,6 +565,7 @@ int rg_set_bodies(rg_system* s, const double* radius, const double* half_height,
   RG_TRY(cudaMemcpy(s->d_props, p.data(), sizeof(double) * p.size(), cudaMemcpyHostToDevice), "upload bodies");
   free_contact_buffers(s);
   detector_free(s);
+  s->vteam.flat_cap = 0;
   cudaError_t e = detector_alloc(s);
   if (e == cudaErrorInvalidValue)
     return fail(s, RG_ERR_ARG, "periodic box smaller than twice the contact range with more than 4096 bodies");
@@ -781,6 +782,10 @@ bool grow(rg_system* s, int err) {
       s->scan.free_();
       s->scan.alloc(s->det.ncells + 1);
     }
+    grew = true;
+  }
+  if (err & ERR_FLAT_CAP) {
+    if (flat_grow(s)) return false;
     grew = true;
   }
   return grew;

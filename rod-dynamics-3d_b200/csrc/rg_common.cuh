@@ -23,7 +23,8 @@ enum : int {
   ERR_TIMEOUT = 16,      // a bounded grid barrier gave up
   ERR_CELL = 32,         // cell grid capacity
   ERR_NONFINITE = 64,    // non-finite state
-  ERR_RECORD_CAP = 128   // MLP record buffer full (recording stops, not fatal)
+  ERR_RECORD_CAP = 128,  // MLP record buffer full (recording stops, not fatal)
+  ERR_FLAT_CAP = 256     // flat pair list overflow (persistent Verlet step)
 };
 
 constexpr int kMaxColors = 64;

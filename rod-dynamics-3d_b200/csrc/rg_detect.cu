@@ -511,6 +511,22 @@ __global__ void k_grid_ncells(DetDev* dd, const Ctl* ctl) {
 // Near lists are on unless near_skin_pct is negative (full lists).
 static bool check_near_lists(const rg_config& c) { return c.near_skin_pct >= 0; }
 
+// The flat pair list's largest length, and its buffer of cap pairs (never
+// shorter than a call has found necessary).
+static long long flat_most(const rg_system* s) {
+  const long long n = s->n, most = s->det.all_pairs ? n * n / 2 + 1 : n * s->det.maxnb;
+  return std::min(most, 2000000000ll);
+}
+static cudaError_t flat_alloc(rg_system* s, long long cap) {
+  VerletTeam& v = s->vteam;
+  cudaFree(v.flat);
+  v.flat = nullptr;
+  v.flat_cap = (int)std::min(std::max(cap, (long long)v.flat_cap), flat_most(s));
+  return cudaMalloc(&v.flat, sizeof(int2) * (size_t)v.flat_cap);
+}
+// Four times the pairs after ERR_FLAT_CAP (a replay of the call each time).
+cudaError_t flat_grow(rg_system* s) { return flat_alloc(s, 4ll * s->vteam.flat_cap); }
+
 cudaError_t detector_alloc(rg_system* s) {
   Detector& d = s->det;
   const int n = s->n;
@@ -591,13 +607,11 @@ cudaError_t detector_alloc(rg_system* s) {
     if ((e = cudaMalloc(&d.ref2, sizeof(double) * 6 * (size_t)n))) return e;
   }
   if (c.model == RG_MODEL_HARMONIC || c.model == RG_MODEL_HERTZ_MINDLIN) {
-    // near lists hold a few pairs a rod; a list that does not fit grows with
-    // the neighbour lists (ERR_NBR_CAP)
-    const long long all = d.all_pairs ? (long long)n * n / 2 + 1 : (long long)n * d.maxnb;
+    // The flat pair list holds a few pairs a rod and grows by itself
+    // (flat_grow), except where it is known to hold every pair.
     const long long few = (long long)n * (d.maxnb / 8 > 1 ? d.maxnb / 8 : 1);
-    const long long cap = d.near_cnt && few < all ? few : all;
-    s->vteam.flat_cap = (int)(cap < 2000000000ll ? cap : 2000000000ll);
-    if ((e = cudaMalloc(&s->vteam.flat, sizeof(int2) * (size_t)s->vteam.flat_cap))) return e;
+    const bool all = d.all_pairs && !d.near_cnt;
+    if ((e = flat_alloc(s, all ? flat_most(s) : few))) return e;
   }
   if (c.model == RG_MODEL_NSC) {
     d.near_skin = near_skin;

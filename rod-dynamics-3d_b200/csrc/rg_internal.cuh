@@ -351,6 +351,7 @@ inline void prof_resolve(rg_system* s) {
 // rg_detect.cu
 cudaError_t detector_alloc(rg_system* s);
 void detector_free(rg_system* s);
+cudaError_t flat_grow(rg_system* s);  // a longer flat pair list (VerletTeam)
 // seg_ready: the segment records and the displacement check of the current
 // positions were written by the drift kernel (reduce_drift_launch)
 // body_csr: the narrow phase also zeroes and counts the body CSR (csr_launch

@@ -389,7 +389,7 @@ __device__ __noinline__ bool v_flatten(const Team& T, const VerletView& W, const
   int prefix, total;
   block_prefix(V.blk, T.nb, rank, prefix, total, S.s);
   if (total > W.flat_cap) {
-    if (rank == 0 && t == 0) atomicOr(&ctl->err, ERR_NBR_CAP);
+    if (rank == 0 && t == 0) atomicOr(&ctl->err, ERR_FLAT_CAP);
     return false;
   }
   const int* cnts = near ? W.near_cnt : V.nbr_cnt;
