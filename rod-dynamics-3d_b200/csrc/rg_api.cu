@@ -207,6 +207,8 @@ cudaError_t snapshot_alloc(rg_system* s) {
   const History& H = s->hist;
   if (s->snap_hcap != H.cap) {
     cudaFree(s->snap_hkey); cudaFree(s->snap_hval); cudaFree(s->snap_hframe);
+    s->snap_hkey = nullptr; s->snap_hval = nullptr; s->snap_hframe = nullptr;
+    s->snap_hcap = 0;
     if ((e = cudaMalloc(&s->snap_hkey, sizeof(unsigned long long) * H.cap))) return e;
     if ((e = cudaMalloc(&s->snap_hval, sizeof(double) * 3 * (size_t)H.cap))) return e;
     if ((e = cudaMalloc(&s->snap_hframe, sizeof(long long) * H.cap))) return e;
@@ -216,6 +218,8 @@ cudaError_t snapshot_alloc(rg_system* s) {
   const size_t wl_bytes = sizeof(double) * 3 * (size_t)N.wcap + sizeof(int) * (size_t)N.wcap;
   if (s->snap_wcap != N.wcap) {
     cudaFree(s->snap_wkey); cudaFree(s->snap_wlam);
+    s->snap_wkey = nullptr; s->snap_wlam = nullptr;
+    s->snap_wcap = 0;
     if ((e = cudaMalloc(&s->snap_wkey, sizeof(unsigned long long) * N.wcap))) return e;
     if ((e = cudaMalloc(&s->snap_wlam, wl_bytes))) return e;
     s->snap_wcap = N.wcap;
@@ -780,7 +784,7 @@ bool grow(rg_system* s, int err) {
     if (detector_alloc(s)) return false;
     if (s->det.ncells + 1 > s->scan.cap) {
       s->scan.free_();
-      s->scan.alloc(s->det.ncells + 1);
+      if (s->scan.alloc(s->det.ncells + 1)) return false;
     }
     grew = true;
   }
@@ -789,6 +793,14 @@ bool grow(rg_system* s, int err) {
     grew = true;
   }
   return grew;
+}
+
+// grow() frees before it allocates: a handle whose buffers could not be
+// allocated takes no further call until its bodies are set again.
+static int fail_grow(rg_system* s) {
+  s->bodies_set = false;
+  cudaGetLastError();
+  return fail(s, RG_ERR_CAPACITY, "could not grow device buffers (set the bodies again)");
 }
 
 // Per-call counters start from the snapshot's control words.
@@ -837,10 +849,10 @@ int resolve_call(rg_system* s, Snapshot& sn, int err, bool* retry) {
   if (err & ERR_TIMEOUT) return fail(s, RG_ERR_TIMEOUT, "a device-side barrier timed out");
   if (err & ERR_NONFINITE) return fail(s, RG_ERR_NONFINITE, "non-finite body state");
   if (err & ERR_COLOR) return fail(s, RG_ERR_CAPACITY, "contact graph needs more than 64 colours");
-  if (!grow(s, err)) return fail(s, RG_ERR_CAPACITY, "could not grow device buffers");
+  if (!grow(s, err)) return fail_grow(s);
+  force_rebuild(s);  // (before anything can fail: new lists hold nothing)
   e = take_snapshot(s, sn);
   if (e) return cuda_fail(s, e, "snapshot");
-  if ((rc = upload_ctl(s, sn)) != RG_OK) return rc;
   *retry = true;
   return RG_OK;
 }
@@ -931,7 +943,7 @@ int rg_detect(rg_system* s, double delta, int32_t* pairs, double* geom, double* 
     if (h->err & ERR_TIMEOUT) return fail(s, RG_ERR_TIMEOUT, "a device-side wait timed out in detection");
     if (h->err & ERR_NONFINITE) return fail(s, RG_ERR_NONFINITE, "non-finite body state");
     if (attempt == 7) return fail(s, RG_ERR_CAPACITY, "capacity retries exhausted");
-    if (!grow(s, h->err)) return fail(s, RG_ERR_CAPACITY, "could not grow device buffers");
+    if (!grow(s, h->err)) return fail_grow(s);
     force_rebuild(s);
   }
   const int C = s->h_ctl->contacts;

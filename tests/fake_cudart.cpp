@@ -15,7 +15,7 @@
 namespace {
 int g_device = 0;
 int g_fail_launches = 0;  // kernels to refuse
-bool g_fail_malloc = false;
+int g_mallocs_left = -1;  // device allocations until one fails, and all after it (-1: none fails)
 int g_err_bits = 0;       // written by the next cooperative kernel ...
 int* g_err_word = nullptr;  // ... to the int cleared last by an asynchronous memset
 cudaError_t g_last = cudaSuccess;
@@ -55,7 +55,7 @@ extern "C" {
 // ---- control -------------------------------------------------------------------
 void fake_set_device(int d) { g_device = d; }
 void fake_fail_launches(int n) { g_fail_launches = n; }
-void fake_fail_malloc(int on) { g_fail_malloc = on != 0; }
+void fake_fail_malloc_after(int n) { g_mallocs_left = n; }
 void fake_next_error(int bits) { g_err_bits = bits; }
 long long fake_launches() { return g_launches; }
 int fake_smem_refused() { return g_smem_refused; }
@@ -104,7 +104,8 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 148; retu
 cudaError_t cudaGetLastError() { const cudaError_t e = g_last; g_last = cudaSuccess; return e; }
 const char* cudaGetErrorString(cudaError_t) { return "an error of the stand-in runtime"; }
 cudaError_t cudaMalloc(void** p, size_t n) {
-  if (g_fail_malloc) return g_last = cudaErrorMemoryAllocation;
+  if (g_mallocs_left == 0) return g_last = cudaErrorMemoryAllocation;
+  if (g_mallocs_left > 0) --g_mallocs_left;
   *p = std::calloc(1, n ? n : 1);
   return cudaSuccess;
 }

@@ -109,3 +109,36 @@ for device in (0, 1, 0):
     s.close()
 assert fake.fake_smem_refused() == 0
 """)
+
+
+@pytest.mark.parametrize("model,bit", [("hertz-mindlin", "contacts"), ("harmonic", "lists"), ("nsc", "contacts")])
+def test_a_handle_without_buffers_asks_for_its_bodies(run_child, model, bit):
+    # the larger buffers cannot be allocated: no kernel may run on the handle
+    # until its bodies are set again
+    run_child(f"""
+seen = 0
+for left in range(0, 60):
+    s = system({model!r})
+    s.detect(0.0)
+    s.step(1)
+    fake.fake_next_error(ERR[{bit!r}])
+    fake.fake_fail_malloc_after(left)
+    first = code(s.step, 1)
+    fake.fake_fail_malloc_after(-1)
+    if first == "ok":
+        s.close()
+        break
+    n = fake.fake_launches()
+    if first == "capacity exceeded":
+        seen += 1
+        assert code(s.step, 1) == code(s.detect, 0.0) == "call out of order"
+        if {model!r} != "nsc":
+            assert code(s.compute_forces) == "call out of order"
+        assert fake.fake_launches() == n
+        s.set_bodies(np.full(N, 0.05), np.full(N, 0.5), np.ones(N), np.ones((N, 3)))
+    else:  # the buffers are there, the snapshot's are not
+        assert first == "CUDA error", first
+    assert code(s.step, 1) == "ok" and fake.fake_launches() > n
+    s.close()
+assert seen > 1
+""")
