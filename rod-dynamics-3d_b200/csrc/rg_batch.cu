@@ -165,6 +165,7 @@ __global__ void k_bulk_gather(const BulkMember* m, int nm, long long T, double* 
 namespace {
 
 int bfail(rg_batch* b, int code, const std::string& msg) {
+  if (code == RG_ERR_CUDA) cudaGetLastError();  // reported now, not by the next call
   b->err = msg;
   return code;
 }
@@ -493,7 +494,9 @@ cudaError_t launch_verlet(rg_batch* b, const std::vector<int>& todo, int nsteps)
   }
   if (which.empty()) return cudaGetLastError();
   cudaError_t e;
-  if (!b->d_vviews) {
+  if (!b->d_vbars) {  // (the last one: all are there, or all are asked for again)
+    cudaFree(b->d_vviews); cudaFree(b->d_vmembers); cudaFree(b->d_vteams);
+    b->d_vviews = nullptr; b->d_vmembers = nullptr; b->d_vteams = nullptr;
     const int bars = std::max(b->n, b->sys[0]->sm_count);
     if ((e = cudaMalloc(&b->d_vviews, sizeof(VerletView) * b->n)) || (e = cudaMalloc(&b->d_vmembers, sizeof(int) * b->n)) ||
         (e = cudaMalloc(&b->d_vteams, sizeof(TeamDesc) * bars)) || (e = cudaMalloc(&b->d_vbars, kTeamBarBytes * bars)))

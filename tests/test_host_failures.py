@@ -142,3 +142,31 @@ for left in range(0, 60):
     s.close()
 assert seen > 1
 """)
+
+
+def test_a_batch_asks_again_for_what_its_first_step_did_not_get(run_child):
+    # the tables of the Verlet members' launch are allocated by the first
+    # step; a step that got only some of them leaves the others to the next
+    run_child("""
+cut = 0
+for left in range(0, 200):
+    b = rodgpu.Batch([rodgpu.default_config(n_bodies=N, model=m, dt=1e-4) for m in ("hertz-mindlin", "harmonic")])
+    for k in range(2):
+        b.set_bodies(k, np.full(N, 0.05), np.full(N, 0.5), np.ones(N), np.ones((N, 3)))
+        b.set_state(k, X, Q, Z, Z)
+    fake.fake_fail_malloc_after(left)
+    try:
+        b.step(1)
+        done = True
+    except rodgpu.RgError as e:
+        done = False
+        if "Verlet launch" in str(e):
+            cut += 1
+            fake.fake_fail_malloc_after(-1)
+            assert code(b.step, 1) == "ok"
+    fake.fake_fail_malloc_after(-1)
+    b.close()
+    if done:
+        break
+assert cut == 4, cut
+""")
