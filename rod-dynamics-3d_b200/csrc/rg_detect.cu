@@ -341,9 +341,8 @@ __global__ void k_zero_cells(int* cnt, int* fill, int ncells, int* nbr_cnt, int 
 // warp per rod.
 __global__ void __launch_bounds__(kTile) k_build_lists(const Seg* seg, int n, const GridDev* gdev, Box box,
                                                        const int* cell_start, const int* cell_rods,
-                                                       double margin, double skin, double cut_center,
-                                                       int all_pairs, int* nbr_cnt, int* nbr,
-                                                       int maxnb, Ctl* ctl) {
+                                                       double margin, double skin, int all_pairs, int* nbr_cnt,
+                                                       int* nbr, int maxnb, Ctl* ctl) {
   griddep_wait();
   if (ctl->err || !ctl->rebuild) return;
   const GridDev g = *gdev;
@@ -363,7 +362,6 @@ __global__ void __launch_bounds__(kTile) k_build_lists(const Seg* seg, int n, co
                        q1, q2, kQ, overflow);
   }
   if (overflow) atomicOr(&ctl->err, ERR_NBR_CAP);
-  (void)cut_center;
 }
 
 __global__ void k_save_ref(const Seg* seg, int n, double* ref, int* nbr, int* nbr_cnt, int maxnb, int all_pairs,
@@ -679,7 +677,7 @@ void detect_launch(rg_system* s, double delta, bool check_rebuild, bool seg_read
   // a block per home cell, or a warp per rod
   const int gb = std::min(d.all_pairs ? grid_for(n * 32, kTile) : d.ncells, s->sm_count * 8);
   RGL launch_dep(k_build_lists, gb, kTile, st, d.seg, n, &dd->grid, s->box, d.cell_start, d.cell_rods,
-                                       d.margin, d.skin, d.cut_center, d.all_pairs ? 1 : 0,
+                                       d.margin, d.skin, d.all_pairs ? 1 : 0,
                                        d.nbr_cnt, d.nbr, d.maxnb, ctl);
   RGL launch_dep(k_save_ref, g, bs, st, d.seg, n, d.ref, d.nbr, d.nbr_cnt, d.maxnb,
                  d.all_pairs ? 1 : 0, ctl);

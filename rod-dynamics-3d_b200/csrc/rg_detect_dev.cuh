@@ -86,20 +86,6 @@ struct BuildSmem {
   int qn[2];       // queue fills (see build_cell_pairs)
 };
 
-__device__ inline int list_insert(int* list, int cnt, int cap, int j, int& overflow) {
-  if (cnt >= cap) {
-    overflow = 1;
-    return cnt;
-  }
-  int k = cnt;
-  while (k > 0 && list[k - 1] > j) {
-    list[k] = list[k - 1];
-    --k;
-  }
-  list[k] = j;
-  return cnt + 1;
-}
-
 // Conservative minimum-image centre offset B - A without divisions (for list
 // building only; the exact narrow phase uses min_image_shift).
 __device__ inline d3 centre_offset(const Seg& A, const Seg& B, const Box& box, const double* invL) {
@@ -139,8 +125,8 @@ __device__ inline bool seg_far(const Seg& A, const Seg& B, d3 d, double lim) {
 // home rods and each neighbour cell are staged in shared memory and the
 // block's threads split the (home rod, neighbour rod) pairs.  Accepted j > i
 // are appended with an atomic per-rod counter (nbr_cnt zeroed beforehand);
-// sort_lists() orders every list afterwards.  Acceptance is the same
-// conservative test as build_cell.
+// sort_list orders every list afterwards.  A conservative centre test, then
+// seg_far, then the exact distance decide.
 __device__ inline void build_cell_pairs(const Seg* seg, const GridDev& g, const Box& box, const double* invL,
                                         const int* cell_start, const int* cell_rods, double margin,
                                         double skin, int* nbr_cnt, int* nbr, int maxnb, int cell,

@@ -2258,8 +2258,6 @@ void nsc_batch_launch(const NscView* views, const TeamDesc* teams, int nteams, c
   launch_coop((const void*)k_nsc_run, grid, kBlock, args, st, sizeof(SmallSmem));
 }
 
-int nsc_block_threads() { return kBlock; }
-
 // Co-resident blocks of the persistent kernel per SM of the current device
 // (its registers and shared memory decide; the cooperative launch needs them
 // all resident).
@@ -2271,8 +2269,6 @@ int nsc_blocks_per_sm() {
   }
   return k;
 }
-size_t nsc_block_smem() { return sizeof(SmallSmem) + sizeof(SmemNsc); }
-
 size_t nsc_view_bytes() { return sizeof(NscView); }
 size_t nsc_team_bytes() { return sizeof(TeamDesc); }
 

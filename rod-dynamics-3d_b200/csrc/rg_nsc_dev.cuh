@@ -549,8 +549,6 @@ struct TeamDesc {
 
 void nsc_batch_launch(const NscView* views, const TeamDesc* teams, int nteams, const int* members, int grid,
                       int nsteps, cudaStream_t st);
-int nsc_block_threads();
-size_t nsc_block_smem();
 NscView make_view(rg_system* s);
 
 }  // namespace rg
