@@ -113,7 +113,11 @@ typedef struct rg_config {
   /* Neighbour-list broad phase (project-specific, no reference field). */
   double skin;                   /* Verlet skin; <= 0: max(d/2, L/10), means */
   int32_t max_neighbors;         /* initial per-rod list capacity; <= 0 auto */
-  int32_t team_blocks;           /* blocks of the persistent team; 0 auto */
+  int32_t team_blocks;           /* blocks of the persistent team; 0 auto (up
+                                    to one per SM).  A call holds them until
+                                    it ends: handles stepped from several
+                                    threads run side by side when their teams
+                                    fit the GPU together, else in turn        */
   int32_t nsc_mlp_scope;         /* learned start for: 0 contacts new since
                                     the last step (not in the warm cache),
                                     1 every contact                          */
@@ -260,14 +264,18 @@ int rg_compute_forces(rg_system* sys, double* f, double* tau, double* pe);
 int rg_get_history(const rg_system* sys, int32_t* pairs, double* value,
                    int64_t* last_frame, size_t cap, size_t* n);
 
-/* Enables (1) or disables (0) the stage timers; resets the accumulators. */
+/* Enables (1) or disables (0) the stage timers; resets the accumulators.
+ * Soft and Hertz-Mindlin steps run as plain launches, which the timers bracket,
+ * while they are on: the same results, but not the kernel whose time
+ * rg_step_stats.device_ms gives without them. */
 int rg_set_profiling(rg_system* sys, int enable);
 /* Accumulated milliseconds and launch counts per stage since enabling. */
 int rg_get_profile(const rg_system* sys, double* ms, int64_t* launches);
 /* Phase times of the persistent NSC step since enabling (ms, n <= 12):
  * 0 free flight, 1 detection, 2 colouring, 3 manifold rows, 4 PSOR,
  * 5 position update, 6 projection detection, 7 projection colouring,
- * 8 projection sweeps. */
+ * 8 projection sweeps, 9 list builds (part of 1 and 6), 10 body slots of the
+ * on-chip solve and its results, 11 the wait after it. */
 int rg_get_phase_times(const rg_system* sys, double* ms, int n);
 
 /* ---- seeded packings generated on the device ------------------------------ */
