@@ -174,6 +174,27 @@ __device__ inline bool team_excl_scan(const Team& T, const int* in, int* out, in
 // ---------------------------------------------------------------------------
 // Detection inside the persistent kernel.
 // ---------------------------------------------------------------------------
+// Rods in the 27 cells about cell c, a row of three at a time (the wrap along x
+// left out: an estimate).
+static __device__ inline int cells_around(const GridDev& g, const Box& box, const int* cell_start, int c) {
+  const int cx = c % g.n[0], cy = (c / g.n[0]) % g.n[1], cz = c / (g.n[0] * g.n[1]);
+  const int x0 = max(cx - 1, 0), x1 = min(cx + 2, g.n[0]);
+  int sum = 0;
+  for (int dz = -1; dz <= 1; ++dz)
+    for (int dy = -1; dy <= 1; ++dy) {
+      int y = cy + dy, z = cz + dz;
+      if (box.pbc) {
+        y = (y + g.n[1]) % g.n[1];
+        z = (z + g.n[2]) % g.n[2];
+      } else if (y < 0 || z < 0 || y >= g.n[1] || z >= g.n[2]) {
+        continue;
+      }
+      const int row = (z * g.n[1] + y) * g.n[0];
+      sum += cell_start[row + x1] - cell_start[row + x0];
+    }
+  return sum;
+}
+
 // The pairs of a team's cells, each block its share; those without rods are
 // passed over a word of cells at a time (one after the other, 0.5 us each).
 static __device__ RG_BUILD_INLINE void build_cells(const Team& T, const NscView& V, const GridDev& g,
@@ -229,6 +250,7 @@ static __device__ bool build_lists(const Team& T, const NscView& V, SmemNsc& sm,
     V.cell_fill[c] = 0;
   }
   for (int i = tid; i < n; i += TS) V.nbr_cnt[i] = 0;
+  if (rank == 0 && threadIdx.x < 2) V.bounds[threadIdx.x] = 0ull;  // (an open box's grid has been made from them)
   if (!team_sync(T)) return false;
   for (int i = tid; i < n; i += TS) {
     Seg s = V.seg[i];
@@ -241,35 +263,47 @@ static __device__ bool build_lists(const Team& T, const NscView& V, SmemNsc& sm,
   }
   if (!team_sync(T)) return false;
   if (!team_excl_scan(T, V.cell_cnt, V.cell_start, g.ncells, V.blk, sm)) return false;
-  int others = 0;  // rods that share a rod's cell, summed over the rods
+  // (and how crowded the cells are: the other rods in a rod's cell and in its
+  // neighbourhood, over every rod of a small system, every 16th of a large one)
+  const int step = n > 16384 ? 16 : 1;
+  int own = 0, near = 0;
   for (int i = tid; i < n; i += TS) {
     int c = V.cell_of[i];
     const int first = V.cell_start[c];
     V.cell_rods[first + atomicAdd(&V.cell_fill[c], 1)] = i;
-    others += min(V.cell_start[c + 1] - first - 1, 255);
+    if (i % step) continue;
+    own += min(V.cell_start[c + 1] - first - 1, 4095);
+    near += min(cells_around(g, V.box, V.cell_start, c) - 1, 4095);
   }
-  others = block_reduce_sum_i(others, sm.red_i);
-  if (threadIdx.x == 0) V.blk[rank] = (int)(65536.0 * others / n);
+  own = block_reduce_sum_i(own, sm.red_i);
+  near = block_reduce_sum_i(near, sm.red_i);
+  if (threadIdx.x == 0) {
+    atomicAdd(&V.bounds[0], (unsigned long long)own);
+    atomicAdd(&V.bounds[1], (unsigned long long)near);
+  }
   if (!team_sync(T)) return false;
-  int before, total;
-  block_prefix(V.blk, T.nb, rank, before, total, sm);
-  const double rho = total / 65536.0;
+  const int seen = (n + step - 1) / step;
+  const double K = (double)*(volatile unsigned long long*)&V.bounds[1] / seen;
+  const double shared = 1.0 + (double)*(volatile unsigned long long*)&V.bounds[0] / seen;
   double invL[3] = {1.0, 1.0, 1.0};
   for (int k = 0; k < 3; ++k)
     if (V.box.L[k] > 0.0) invL[k] = 1.0 / V.box.L[k];
   // One thread per home rod, or the block splits the pairs of one home cell at
-  // a time.  A thread alone with its rod's candidates is a serial chain, some
-  // 50 + 60 rho us a turn of the threads with rho other rods in the average
-  // rod's cell; a cell that holds rods costs a block some 13 us (barriers and
-  // the staging of its neighbourhood) until there are rods enough to fill the
-  // tiles, so a block with n / nb rods, rho a cell, takes 13 n / (nb rho).
-  // They meet at n / nb = rho (4 + 5 rho), and where threads have several
-  // turns near rho = 12.  Measured, by rod and by cell, us: 1000 rods on 8
-  // blocks, rho 0.03 54 and 2132 (32768 cells), 1 115 and 818, 4 242 and 351,
-  // 8 552 and 144; 20000 on 148, rho 1 137 and 1168, 4 288 and 460, 8 506 and
-  // 237; 20000 on 40, rho 8 502 and 774, 16 945 and 662; a million on 148, rho
-  // 1 1384 and 49811, 8 5154 and 11045, 16 8723 and 7469.
-  if (rho < 12.0 && n > rho * (4.0 + 5.0 * rho) * T.nb) {
+  // a time.  A thread alone with its rod's K candidates is a serial chain,
+  // 12 + 2.1 K us (several turns of the threads overlap by a quarter); a cell
+  // that holds rods costs its block some 12 us of barriers and staging, more
+  // when its pairs fill several rounds, and there are a little over n / shared
+  // of them.
+  // Measured, whole builds by rod and by cell, us (some 40 of them the cells
+  // themselves), uniform boxes with rho rods a cell (K = 27 rho): 1000 rods on 8
+  // blocks, rho 0.03 54 and 2132 (32768 cells), 1 115 and 818, 4 242 and 351, 8
+  // 552 and 144; 20000 on 148, rho 1 137 and 1168, 4 288 and 460, 8 506 and 237;
+  // 20000 on 40, rho 8 502 and 774, 16 945 and 662; a million on 148, rho 1 1384
+  // and 49811, 8 5154 and 11045, 16 8723 and 7469.  60 rods in a tube on one
+  // block (few neighbours a rod, and those along one axis): 26 and 133.
+  const double t_rod = (12.0 + 2.1 * K) * fmax(1.0, 0.75 * n / TS);
+  const double t_cell = (13.5 + 4e-5 * K * K) * n / (shared * T.nb);
+  if (t_rod < t_cell) {
     for (int i = tid; i < n; i += TS)
       build_rod_list(i, V.seg, g, V.box, invL, V.cell_of, V.cell_start, V.cell_rods, V.margin, V.skin,
                      V.nbr_cnt, V.nbr, V.maxnb, overflow);
